@@ -269,6 +269,107 @@ def run(state):
         return state["step"]()
 
 
+# --------------------------------------------------------------------------------------------- the same in 64 bits
+
+
+def _nibbles(words, fmt, along_rows):
+    shifts = (0, 16, 4, 20, 8, 24, 12, 28) if fmt == "awq" else (0, 4, 8, 12, 16, 20, 24, 28)
+    parts = [(words >> s) & 15 for s in shifts]
+    if along_rows:
+        return torch.stack(parts, dim=1).reshape(8 * words.shape[0], words.shape[1])
+    return torch.stack(parts, dim=2).reshape(words.shape[0], 8 * words.shape[1])
+
+
+def _w4_values(fmt, qweight, qzeros, scales, g_idx=None):
+    """Checkpoint tensors of one linear -> its weight [K, N], 64 bits."""
+    q = _nibbles(qweight, fmt, fmt != "awq").double()
+    z = _nibbles(qzeros, fmt, False).double() + (1.0 if fmt == "gptq" else 0.0)
+    g = (torch.arange(q.shape[0], device=q.device) // GROUP) if g_idx is None else g_idx.long()
+    return (q - z[g]) * scales.double()[g]
+
+
+def _swiglu(gate_up):
+    gate, up = gate_up.chunk(2, dim=-1)
+    return torch.nn.functional.silu(gate) * up
+
+
+def _fp8_codes(v, amax):
+    """v / (max(amax, 1e-12) / 448) in f32, rounded to e4m3: (the codes' values, the scales), 64 bits."""
+    s = amax.clamp_min(1e-12) / 448.0
+    return (v / s).to(torch.float8_e4m3fn).double(), s.double()
+
+
+def _e2m1(v):
+    a = v.abs()
+    pitch = torch.where(a < 2, 0.5, torch.where(a < 4, 1.0, 2.0))
+    return torch.copysign((torch.round(a / pitch) * pitch).clamp_max(6.0), v).double()
+
+
+def _nvfp4_activation(x):
+    """The static rule: block scales relative to the global one, codes of x / (scale * global), every step in f32."""
+    s2 = x.abs().amax().clamp_min(1e-12) / (6.0 * 448.0)
+    blocks = x.reshape(x.shape[0], -1, 16)
+    sixth = torch.ones((), device=x.device) / 6.0
+    bits = (blocks.abs().amax(dim=-1) * sixth * (1.0 / s2)).clamp_max(448.0).to(torch.float8_e4m3fn).float()
+    codes = _e2m1(blocks / (bits * s2).clamp_min(1e-12)[..., None])
+    return (codes * bits.double()[..., None]).reshape(x.shape) * s2.double()
+
+
+def _nvfp4_weight(w):
+    """The weight rule: block scale = block amax / 6 as e4m3 relative to scale_2, codes of w / f16(scale * scale_2)."""
+    s2 = w.abs().amax().clamp_min(1e-12) / (6.0 * 448.0)
+    blocks = w.reshape(w.shape[0], -1, 16)
+    bits = (blocks.abs().amax(dim=-1) / 6.0 / s2).clamp_max(448.0).to(torch.float8_e4m3fn).float()
+    fused = (bits * s2).half().float()[..., None]
+    codes = _e2m1(torch.where(fused != 0, blocks / fused, torch.zeros_like(blocks)))
+    return (codes * bits.double()[..., None]).reshape(w.shape) * s2.double()
+
+
+def exact(case, seed):
+    """run()'s outputs from the same checkpoint tensors and the same activation codes, everything after them in 64 bits."""
+    with torch.no_grad():
+        m, k, n, kind, dtype = case["rows"], case["k"], case["n"], case["kind"], DTYPE[case["dtype"]]
+        x = torch.randn(m, k, device="cuda", generator=_gen(seed)).to(dtype)
+        outs = []
+        for i in range(case["layers"]):
+            if kind == "w4":
+                outs.append(x.double() @ _w4_values(case["fmt"], *_w4_tensors(_gen(seed, 1 + i), case["fmt"], case["order"], k, n)))
+            elif kind == "mlp":
+                fmt, order = case["fmt"], case["order"]
+                gate, up = (x.double() @ _w4_values(fmt, *_w4_tensors(_gen(seed, 10 * i + j), fmt, order, k, n)) for j in (1, 2))
+                hidden = torch.nn.functional.silu(gate) * up
+                outs.append(hidden @ _w4_values(fmt, *_w4_tensors(_gen(seed, 10 * i + 3), fmt, "none", n, k)))
+            elif kind == "moe":
+                e, topk = case["experts"], case["topk"]
+                logits = torch.randn(m, e, device="cuda", generator=_gen(seed, 1)).double()
+                scores, ids = torch.softmax(logits, dim=-1).topk(topk, dim=-1)
+                scores = scores / scores.sum(dim=-1, keepdim=True)
+                gate_up, down = (_w4_tensors(_gen(seed, 10 * i + 2 + j), "awq", "none", *s, lead=(e,))[:3] for j, s in enumerate([(k, 2 * n), (n, k)]))
+                y = torch.zeros(m, k, dtype=torch.float64, device="cuda")
+                for j in range(e):
+                    rows, slot = (ids == j).nonzero(as_tuple=True)
+                    if rows.numel():
+                        h = _swiglu(x[rows].double() @ _w4_values("awq", *(t[j] for t in gate_up)))
+                        y.index_add_(0, rows, scores[rows, slot, None] * (h @ _w4_values("awq", *(t[j] for t in down))))
+                outs.append(y)
+            else:
+                w = torch.randn(n, k, device="cuda", generator=_gen(seed, 1 + i)) * 0.02
+                xf = x.float()
+                if kind == "fp8":
+                    (xq, xs), (wq, wscale) = (_fp8_codes(v, v.abs().amax(dim=1, keepdim=True)) for v in (xf, w))
+                    outs.append((xq @ wq.T) * xs * wscale.reshape(1, -1))
+                elif kind == "fp8_block":
+                    xb = xf.reshape(m, k // 128, 128)
+                    xq, xs = _fp8_codes(xb, xb.abs().amax(dim=2, keepdim=True))
+                    blocks = w.reshape(n // 128, 128, k // 128, 128)
+                    s = blocks.abs().amax(dim=(1, 3)).clamp_min(1e-12) / 448.0
+                    bits = (blocks / s[:, None, :, None]).to(torch.float8_e4m3fn).double()
+                    outs.append((xq * xs).reshape(m, k) @ (bits * s.double()[:, None, :, None]).reshape(n, k).T)
+                else:
+                    outs.append(_nvfp4_activation(xf) @ _nvfp4_weight(w).T)
+        return outs
+
+
 # -------------------------------------------------------------------------------------------------- bytes and flops
 
 

@@ -20,8 +20,12 @@
 // gather the columns of x into the workspace first.
 #include "tc_common.cuh"
 #include "w4_tile.cuh"
+#include "w4_tmem.cuh"
 
 namespace eq {
+
+int w4_tmem_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
+                         bool promote, int* status, cudaStream_t stream);  // w4_tmem.cu
 
 namespace {
 
@@ -614,40 +618,9 @@ int launch_cfg(const unsigned char* wq, int scale_dtype, const ActT* x, ActT* y,
                       static_cast<int>(K), status, grp, SplitArgs{nullptr, nullptr});
 }
 
-// Up to 128 * HALVES rows: one row tile of 128 * HALVES x 256 with K split over gridDim.z so that about one CTA per SM runs.
-template <typename ActT, int HALVES>
-int launch_split(const unsigned char* wq, int scale_dtype, const ActT* x, ActT* y, int64_t M, int64_t N, int64_t K, int* status,
-                 float* partial, int* counters, cudaStream_t stream) {
-    using Cfg = GemmCfg<HALVES, 256, 16, 2>;
-    CUtensorMap map_x;
-    const CUtensorMapDataType elem = ScaleMul<ActT>::kFmt == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    const int box_rows = HALVES == 1 ? a_box_rows(static_cast<int>(M)) : 128 * Cfg::kBoxHalves;
-    int st = make_tensor_map_2d(&map_x, x, elem, 2, M, K, K * 2, box_rows, kGK, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (st != EQ_OK) return st;
-    const int64_t tiles = ceil_div(N, 256), items = K / 128;
-    int64_t splits = sm_count() / tiles;
-    if (splits > items) splits = items;
-    if (splits > 32) splits = 32;
-    if (splits < 1) splits = 1;
-    const bool cvt = scale_dtype != (ScaleMul<ActT>::kFmt == 0 ? EQ_F16 : EQ_BF16);
-    const GroupArgs none = {nullptr, nullptr, nullptr, nullptr, 0};
-    const SplitArgs sp = {partial, counters};
-    dim3 grid(static_cast<unsigned>(tiles), 1, static_cast<unsigned>(splits));
-    if (splits == 1) {
-        auto kernel = cvt ? w4a16_gemm_tc_kernel<ActT, HALVES, 256, 16, 2, true, kPlain, false> : w4a16_gemm_tc_kernel<ActT, HALVES, 256, 16, 2, false, kPlain, false>;
-        EQ_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmem)));
-        return launch_pdl(kernel, grid, Cfg::kThreads, Cfg::kSmem, stream, true, map_x, wq, y, static_cast<int>(M), static_cast<int>(N),
-                          static_cast<int>(K), status, none, sp);
-    }
-    auto kernel = cvt ? w4a16_gemm_tc_kernel<ActT, HALVES, 256, 16, 2, true, kPlain, true> : w4a16_gemm_tc_kernel<ActT, HALVES, 256, 16, 2, false, kPlain, true>;
-    EQ_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmem)));
-    return launch_pdl(kernel, grid, Cfg::kThreads, Cfg::kSmem, stream, true, map_x, wq, y, static_cast<int>(M), static_cast<int>(N),
-                      static_cast<int>(K), status, none, sp);
-}
-
 template <typename ActT>
 int launch_typed(const unsigned char* wq, int scale_dtype, const int32_t* perm, const ActT* x, ActT* y, int64_t M, int64_t N,
-                 int64_t K, ActT* gathered, int* status, float* partial, int* counters, cudaStream_t stream) {
+                 int64_t K, ActT* gathered, int* status, cudaStream_t stream) {
     if (perm) {
         const int64_t total = M * K;
         gather_cols_kernel<ActT><<<static_cast<unsigned>(ceil_div(total, 256)), 256, 0, stream>>>(x, perm, M, K, gathered);
@@ -655,24 +628,7 @@ int launch_typed(const unsigned char* wq, int scale_dtype, const int32_t* perm, 
         x = gathered;
     }
     const GroupArgs none = {nullptr, nullptr, nullptr, nullptr, 0};
-    if (M <= 128) {
-        // wide matrices fill the SMs with 64-column tiles; narrow ones split K over 256-column tiles instead
-        if (ceil_div(N, 64) >= sm_count())
-            return launch_cfg<ActT, 1, 64, 8, 4, kPlain>(wq, scale_dtype, x, y, M, N, K, status, none, 1, stream);
-        return launch_split<ActT, 1>(wq, scale_dtype, x, y, M, N, K, status, partial, counters, stream);
-    }
-    if (M <= 512 && ceil_div(N, 128) * ceil_div(M, 256) * 2 <= sm_count()) {
-        // a few hundred rows of a narrow matrix would leave most SMs idle on whole-K tiles: run 256-row blocks through the
-        // split-K form instead (each block streams the weight once more, which is still far cheaper; the dequantisation,
-        // not the MMA, bounds these calls, so a 256-row block costs what a 128-row block costs)
-        for (int64_t m0 = 0; m0 < M; m0 += 256) {
-            const int64_t mb = M - m0 < 256 ? M - m0 : 256;
-            const int st = mb > 128 ? launch_split<ActT, 2>(wq, scale_dtype, x + m0 * K, y + m0 * N, mb, N, K, status, partial, counters, stream)
-                                    : launch_split<ActT, 1>(wq, scale_dtype, x + m0 * K, y + m0 * N, mb, N, K, status, partial, counters, stream);
-            if (st != EQ_OK) return st;
-        }
-        return EQ_OK;
-    }
+    if (!w4_tmem_pairs(M, N)) return w4_tmem_dense_launch(wq, scale_dtype, x, y, M, N, K, ScaleMul<ActT>::kFmt == 0 ? EQ_F16 : EQ_BF16, false, false, status, stream);
     if (ceil_div(N, 256) * ceil_div(M, 256) >= sm_count())
         return launch_cfg<ActT, 2, 256, 16, 2, kPlain>(wq, scale_dtype, x, y, M, N, K, status, none, static_cast<unsigned>(ceil_div(M, 256)), stream);
     return launch_cfg<ActT, 2, 128, 16, 3, kPlain>(wq, scale_dtype, x, y, M, N, K, status, none, static_cast<unsigned>(ceil_div(M, 256)), stream);
@@ -681,14 +637,13 @@ int launch_typed(const unsigned char* wq, int scale_dtype, const int32_t* perm, 
 }  // namespace
 
 // gathered: M * K elements of scratch when perm is given.  status: one word, set by a bounded wait that ran out.
-// partial / counters: f32 [min(M, 256)][N] and one int per 256 columns, zero between calls (used by the split-K forms).
 int w4_gemm_tc_launch(const unsigned char* wq, int scale_dtype, const int32_t* perm, const void* x, void* y, int64_t M, int64_t N,
-                      int64_t K, int act_dtype, void* gathered, int* status, float* partial, int* counters, cudaStream_t stream) {
+                      int64_t K, int act_dtype, void* gathered, int* status, cudaStream_t stream) {
     if (act_dtype == EQ_F16)
         return launch_typed<__half>(wq, scale_dtype, perm, static_cast<const __half*>(x), static_cast<__half*>(y), M, N, K,
-                                    static_cast<__half*>(gathered), status, partial, counters, stream);
+                                    static_cast<__half*>(gathered), status, stream);
     return launch_typed<__nv_bfloat16>(wq, scale_dtype, perm, static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), M,
-                                       N, K, static_cast<__nv_bfloat16*>(gathered), status, partial, counters, stream);
+                                       N, K, static_cast<__nv_bfloat16*>(gathered), status, stream);
 }
 
 // Grouped expert GEMM on the tensor path.  x: [R][K] activations in expert order; blocks / n_blocks: device-side list of

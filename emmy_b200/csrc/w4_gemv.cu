@@ -1,10 +1,11 @@
 // W4A16 linear: the entry points and their dispatch.
 //
 //   M == 1         w4a16_gemv1_kernel (w4_gemv1.cu): half-SM CTAs, equal item spans, launches overlap in pairs.
-//   2 <= M <= 24   w4a16_stream_kernel (w4_stream.cu): one fat CTA per SM streams whole column tiles, x staged in shared
-//                  memory (whole, or a K slice per CTA with the slices meeting in the workspace).  From 17 rows on only
-//                  where a slice of x fits; otherwise the next line.
-//   M > 16         w4a16_gemm_tc_kernel (w4_gemm.cu): tcgen05, weights dequantised into shared memory.
+//   2 <= M <= 16   w4a16_stream_kernel (w4_stream.cu): one fat CTA per SM streams whole column tiles, x staged in shared
+//                  memory (whole, or a K slice per CTA with the slices meeting in the workspace).  Weights with a row
+//                  permutation stay with it up to 24 rows where a slice of x fits.
+//   M > 16         w4a16_tmem_kernel (w4_tmem.cu): tcgen05 with the weights expanded into tensor
+//                  memory; larger calls w4a16_gemm_tc_kernel (w4_gemm.cu), which expands them into shared memory.
 //   w4a16_tile_kernel below: M > 16 with an output that is not 16-byte aligned (in 64-row blocks), and decode
 //   shapes whose activations do not fit shared memory (K beyond about 100 k at M == 1).
 //
@@ -21,14 +22,17 @@
 // Warps of a CTA meet in shared memory.  K splits of one tile meet in an f32 workspace with atomic adds; the CTA
 // whose arrival completes the tile converts, stores y and leaves workspace and counter zero.  Nobody waits.
 #include "w4_tile.cuh"
+#include "w4_tmem.cuh"
 
 namespace eq {
 
 int w4_stream_launch(const W4Params& p, int act_dtype, cudaStream_t stream, bool* fits);  // w4_stream.cu
 int w4_gemv1_launch(const unsigned char* wq, int scale_dtype, const int32_t* perm, const void* x, void* y, int64_t N, int64_t K,
                     int act_dtype, uint32_t* xchg, int* status, cudaStream_t stream, bool* fits);  // w4_gemv1.cu
+int w4_tmem_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
+                         bool promote, int* status, cudaStream_t stream);  // w4_tmem.cu
 int w4_gemm_tc_launch(const unsigned char* wq, int scale_dtype, const int32_t* perm, const void* x, void* y, int64_t M, int64_t N,
-                      int64_t K, int act_dtype, void* gathered, int* status, float* partial, int* counters, cudaStream_t stream);  // w4_gemm.cu
+                      int64_t K, int act_dtype, void* gathered, int* status, cudaStream_t stream);  // w4_gemm.cu
 
 template <typename ActT, int MT, bool ONE>
 __global__ void __launch_bounds__(kTileThreads) w4a16_tile_kernel(const W4Params p) {
@@ -154,9 +158,12 @@ extern "C" int eq_w4a16_linear(const void* wq, int scale_dtype, const int32_t* p
     int* counters = reinterpret_cast<int*>(partial + w4_front_rows(M) * N);
 
     const bool streamable = static_cast<long long>(N / 16) * (K / 128) < (1LL << 30);
+    if (M >= kTmemMinRows && M <= kTmemPromoteRows && !perm && aligned(y, 16))
+        return w4_tmem_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, y, M, N, K, act_dtype, false, true, status, stream);
     if (M > 16 && M <= 24 && streamable) {
-        // up to 24 rows still stream the weight once through the mma.sync tile (x staged in shared memory, K sliced where
-        // it does not fit); a shape that does not fit falls through to the tensor path
+        // with a row permutation (or an unaligned output) up to 24 rows still stream the weight through the mma.sync tile
+        // (x gathered and staged in shared memory, K sliced where it does not fit); the tensor path would need a gather
+        // pass first.  A shape that does not fit falls through to it
         W4Params p = w4_params(wq, perm, x, y, partial, counters, K, N, static_cast<int>(M), scale_dtype);
         bool fits = false;
         const int st = w4_stream_launch(p, act_dtype, stream, &fits);
@@ -167,8 +174,7 @@ extern "C" int eq_w4a16_linear(const void* wq, int scale_dtype, const int32_t* p
         // word (a clear would be one more node between this kernel and the one before it, which it overlaps as a
         // programmatic dependent): it stays set until eq_w4a16_status has reported it.
         void* gathered = static_cast<unsigned char*>(workspace) + w4_gather_offset(M, N);
-        const int st = w4_gemm_tc_launch(static_cast<const unsigned char*>(wq), scale_dtype, perm, x, y, M, N, K, act_dtype, gathered, status,
-                                         partial, counters, stream);
+        const int st = w4_gemm_tc_launch(static_cast<const unsigned char*>(wq), scale_dtype, perm, x, y, M, N, K, act_dtype, gathered, status, stream);
         // Everything behind the header is zero between calls, whatever their shapes: a later call of another shape keeps its
         // partial sums or hand-over words where this one kept the gathered copy of x, so that copy is wiped again.
         if (st == EQ_OK && perm) EQ_CUDA_OK(cudaMemsetAsync(gathered, 0, static_cast<size_t>(M) * K * 2, stream));
@@ -203,8 +209,7 @@ extern "C" int eq_w4a16_linear(const void* wq, int scale_dtype, const int32_t* p
 // ---- gate / up + SwiGLU in one call ---------------------------------------------------------------------------
 // h[M, I] = act(silu(x W_gate)) * (x W_up) for a [gate | up] weight (the two projections concatenated along N, as the
 // reference stores them: emmy/compiler/trace/huggingface.py:1663-1669, 2110-2141), with the eager form's two roundings.
-// M > 16: the tensor path's SwiGLU tile (128 gate + 128 up columns per CTA, the activation in the epilogue) over row
-// blocks of the dense matrix; fewer rows: the [gate | up] linear into scratch, then an elementwise pass.
+// M > 16: the tensor path with gate and up tiles side by side in a CTA and the activation in the epilogue; fewer rows: the [gate | up] linear into scratch, then an elementwise pass.
 namespace eq {
 namespace {
 
@@ -292,8 +297,13 @@ extern "C" int eq_w4a16_gate_up_swiglu(const void* wq, int scale_dtype, const in
                workspace_bytes);
     const size_t inner = gu_align(eq_w4a16_workspace_bytes(M, 2 * I, K));
     unsigned char* extra = static_cast<unsigned char*>(workspace) + inner;
+    if (M >= kTmemMinRows && M <= kTmemPromoteRows && !perm && aligned(h, 16))
+        return w4_tmem_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, h, M, 2 * I, K, act_dtype, true, true,
+                                    static_cast<int*>(workspace), stream);
     if (M > 16 && !perm && aligned(h, 16)) {
         int* status = static_cast<int*>(workspace);  // sticky until eq_w4a16_status reports it, as in eq_w4a16_linear
+        if (!w4_tmem_pairs(M, 2 * I))
+            return w4_tmem_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, h, M, 2 * I, K, act_dtype, true, false, status, stream);
         RowBlock* blocks = reinterpret_cast<RowBlock*>(extra);
         const int nb = static_cast<int>((M + 255) / 256);
         int32_t* n_blocks = reinterpret_cast<int32_t*>(blocks + nb);

@@ -1,0 +1,293 @@
+// Arguments of the W4A16 kernel with the weights in tensor memory (w4_tmem.cu).
+#pragma once
+#include "tc_common.cuh"
+#include "w4_tile.cuh"
+
+namespace eq {
+
+// Row counts at which the weights-in-TMEM kernels take over (us, K=4096 N=14336 | K=14336 N=4096 | K=N=4096 | the
+// [gate | up] + down MLP of hidden 4096, intermediate 14336; the other side first).
+// From 17 rows: below, w4_stream.cu stages all rows in shared memory and is the faster one (16 rows: 15.1 against 21.1, MLP
+// 42.8 against 44.5; 20 rows: 25.3 | 12.3 (K=N=4096) | MLP 73.2 against 17.1 | 9.6 | 49.4).  17 to 24 rows keep that
+// kernel's arithmetic, integers in the MMA and scales applied to f32 sums (PROMOTE); above, the weights are scaled before
+// the MMA, which at 28 rows costs 15.8 against 20.0 promoted.
+constexpr int64_t kTmemMinRows = 17, kTmemPromoteRows = 24;
+
+// More than 256 rows whose 256 x 256 tiles occupy at least a quarter of the SMs stay with w4_gemm.cu, the rest run on tiles of
+// 128 channels and at most 128 rows, with K slices where CTAs would idle.
+inline bool w4_tmem_pairs(int64_t M, int64_t N) { return M > 256 && ceil_div(N, 256) * ceil_div(M, 256) * 4 >= sm_count(); }
+
+struct W4TmemArgs {
+    const unsigned char* wq;   // repacked weight (of expert 0)
+    void* y;
+    int M, N, K;               // N: columns of the weight; the SwiGLU form writes N / 2
+    int row_tiles, rows_per_tile, splits, units;  // dense form
+    int scale_dtype;
+    int* status;
+    // grouped form
+    const RowBlock* blocks;
+    const int32_t* n_blocks;
+    const int32_t* y_rows;     // optional: output row m goes to row y_rows[m]
+    const uint64_t* y_ptrs;    // optional: output row m starts at address y_ptrs[m] (0 = drop the row)
+    size_t expert_stride;
+};
+
+// ---- device code shared by w4_tmem.cu and w4_tmem2.cu ----------------------------------------------------------
+namespace tm {
+
+// Bounded wait as tc::mbar_wait, but the thread sleeps in the barrier unit between looks: with dequantisation bound by issue
+// slots, spinning TMA and MMA threads would take theirs.
+__device__ __forceinline__ bool wait_asleep(uint32_t bar, uint32_t parity) {
+    const long long start = clock64();
+    for (;;) {
+        uint32_t ok;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(ok)
+                     : "r"(bar), "r"(parity), "r"(1000000u)
+                     : "memory");
+        if (ok) return true;
+        if (clock64() - start > tc::kWaitCycles) return false;
+    }
+}
+
+// ---- thread-block clusters
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+template <typename ActT>
+struct Mul;
+template <>
+struct Mul<__half> {
+    static constexpr uint32_t kFmt = 0;
+    template <bool CVT>
+    static __device__ __forceinline__ uint32_t pair(uint32_t raw) {
+        if constexpr (CVT) raw = __half_as_ushort(__float2half_rn(__uint_as_float(raw << 16)));
+        return __byte_perm(raw, 0, 0x1010);
+    }
+    static __device__ __forceinline__ uint32_t mul(uint32_t v, uint32_t s) {
+        uint32_t r;
+        asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(s));
+        return r;
+    }
+};
+template <>
+struct Mul<__nv_bfloat16> {
+    static constexpr uint32_t kFmt = 1;
+    template <bool CVT>
+    static __device__ __forceinline__ uint32_t pair(uint32_t raw) {
+        if constexpr (CVT) raw = __bfloat16_as_ushort(__float2bfloat16_rn(__half2float(__ushort_as_half(static_cast<unsigned short>(raw)))));
+        return __byte_perm(raw, 0, 0x1010);
+    }
+    static __device__ __forceinline__ uint32_t mul(uint32_t v, uint32_t s) {
+        uint32_t r;
+        asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(s));
+        return r;
+    }
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t r;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(a) : "memory");
+    return r;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 r;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(a) : "memory");
+    return r;
+}
+
+// 16 lanes x 32 columns: lane 4 g + j of the warp gives rows g and g + 8 of column 4 i + j in registers 2 i, 2 i + 1.
+__device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// D[tmem] (+)= A[tmem] * B[smem]
+__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, bool accumulate) {
+    const uint32_t acc = accumulate ? 1u : 0u;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+template <typename ActT>
+__device__ __forceinline__ uint32_t bits16(float v) {
+    const ActT o = from_float<ActT>(v);
+    return *reinterpret_cast<const uint16_t*>(&o);
+}
+
+// Sixteen accumulator columns (rows c .. c + 15 of a unit) of one warp's 32 channels -> y.  tile_lo: weight tile of lanes
+// 0-15; lanes 16-31 hold the next one, or (SWIGLU) the up tile that belongs to it.
+template <typename ActT, bool SWIGLU, bool GROUPED>
+__device__ __forceinline__ void emit16(const W4TmemArgs& a, const float (&v)[16], int tile_lo, int row0, int rows, int c) {
+    const int lane = threadIdx.x & 31, n_tiles = a.N / 16;
+    if constexpr (SWIGLU) {
+        // lanes 0-15 hold gate, 16-31 up of the same channels: of two rows, the low lanes finish the first
+        const int out_n = a.N / 2;
+        const bool live = tile_lo < n_tiles / 2;
+        ActT* dst = static_cast<ActT*>(a.y) + tile_lo * 16 + (lane & 14);
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+            uint32_t o[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float mine = lane < 16 ? v[i + 2 * h] : v[i + 2 * h + 1];
+                const float theirs = __shfl_xor_sync(0xFFFFFFFFu, lane < 16 ? v[i + 2 * h + 1] : v[i + 2 * h], 16);
+                const float g = to_float(from_float<ActT>(lane < 16 ? mine : theirs));
+                const float u = to_float(from_float<ActT>(lane < 16 ? theirs : mine));
+                const float sg = to_float(from_float<ActT>(g / (1.f + expf(-g))));
+                o[h] = bits16<ActT>(sg * u);
+            }
+            // neighbours swap so that a lane holds two channels of one row
+            const uint32_t p = o[0] | (o[1] << 16), pn = __shfl_xor_sync(0xFFFFFFFFu, p, 1);
+            const uint32_t w = (lane & 1) ? __byte_perm(p, pn, 0x3276) : __byte_perm(p, pn, 0x5410);
+            const int r = c + i + 2 * (lane & 1) + (lane >> 4);
+            if (live && r < rows) *reinterpret_cast<uint32_t*>(dst + static_cast<size_t>(row0 + r) * out_n) = w;
+        }
+    } else {
+        const bool live = tile_lo + (lane >> 4) < n_tiles;
+        const int ch = tile_lo * 16 + (lane & 30);
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+            const uint32_t p = bits16<ActT>(v[i]) | (bits16<ActT>(v[i + 1]) << 16), pn = __shfl_xor_sync(0xFFFFFFFFu, p, 1);
+            const uint32_t w = (lane & 1) ? __byte_perm(p, pn, 0x3276) : __byte_perm(p, pn, 0x5410);
+            const int r = c + i + (lane & 1);
+            if (live && r < rows) {
+                ActT* dst;
+                if (GROUPED && a.y_ptrs)
+                    dst = reinterpret_cast<ActT*>(a.y_ptrs[row0 + r]);  // null: drop the row
+                else
+                    dst = static_cast<ActT*>(a.y) + (GROUPED && a.y_rows ? static_cast<size_t>(a.y_rows[row0 + r]) : static_cast<size_t>(row0 + r)) * a.N;
+                if (!GROUPED || dst) *reinterpret_cast<uint32_t*>(dst + ch) = w;
+            }
+        }
+    }
+}
+
+// A dequant warp's view of one item: two weight tiles of 16 channels, read from the warp's ring slot.
+struct ItemWords {
+    uint32_t wd[2][8];
+    uint2 mt[2];
+};
+// A lane's byte offsets inside a ring slot.  The 16-byte piece of lane 4 g + r of a half tile is put at place
+// (r + g / 2) % 4 of its channel's four, so that the 32 lanes reading word j of piece r of their channels hit 32 banks.
+struct LaneOffsets {
+    uint32_t put, put_meta, get[4], get_meta;
+    __device__ __forceinline__ LaneOffsets() {
+        const int lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+        put = ((lane & ~3) + ((lane + (lane >> 3)) & 3)) * 16;
+        put_meta = 1024 + lane * 16;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) get[r] = (4 * g + ((r + (g >> 1)) & 3)) * 16 + 4 * j;
+        get_meta = 1024 + 8 * g;
+    }
+};
+__device__ __forceinline__ void load_item(uint32_t slot_addr, const LaneOffsets& o, ItemWords& w) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const uint32_t at = slot_addr + o.get[r];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            w.wd[t][2 * r] = lds32(at + t * kItemBytes);
+            w.wd[t][2 * r + 1] = lds32(at + t * kItemBytes + 512);
+        }
+    }
+    w.mt[0] = lds64(slot_addr + o.get_meta);
+    w.mt[1] = lds64(slot_addr + o.get_meta + kItemBytes);
+}
+// One tile's record (1088 bytes) into a ring slot; src: the record + 16 * lane.
+__device__ __forceinline__ void fetch_item(uint32_t slot_addr, const LaneOffsets& o, const unsigned char* src) {
+    cp_async16(slot_addr + o.put, src);
+    cp_async16(slot_addr + o.put + 512, src + 512);
+    if ((threadIdx.x & 31) < 4) cp_async16(slot_addr + o.put_meta, src + 1024);
+}
+// Zero point pair -> constants of the exact dequant (Frag<ActT>::expand), fewer instructions than Frag<ActT>::zero: the
+// zero points are the integers 0..16.
+template <typename ActT>
+__device__ __forceinline__ typename Frag<ActT>::Zero zero_of(uint32_t z_pair);
+template <>
+__device__ __forceinline__ Frag<__half>::Zero zero_of<__half>(uint32_t z_pair) {
+    Frag<__half>::Zero r;
+    asm("add.f16x2 %0, %1, %2;" : "=r"(r.sub) : "r"(z_pair), "r"(0x64006400u));                              // 1024 + z
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r.fma) : "r"(z_pair), "r"(0xBC00BC00u), "r"(0xD400D400u));  // -(64 + z)
+    return r;
+}
+template <>
+__device__ __forceinline__ Frag<__nv_bfloat16>::Zero zero_of<__nv_bfloat16>(uint32_t z_pair) {
+    Frag<__nv_bfloat16>::Zero r;
+    uint32_t t;
+    asm("add.f16x2 %0, %1, %2;" : "=r"(t) : "r"(z_pair), "r"(0x64006400u));  // low mantissa bits of 1024 + z: the integer z
+    r.sub = lop3<0xEA>(t, 0x001F001Fu, 0x43004300u);                           // bf16 128 + z
+    r.fma = 0;
+    return r;
+}
+// Expands the item into 64 columns of TMEM at taddr (lanes of this warp's quarter): q - z, times the scale unless PROMOTE.
+template <typename ActT, bool CVT, bool PROMOTE>
+__device__ __forceinline__ void expand_item(const ItemWords& w, uint32_t taddr) {
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const typename Frag<ActT>::Zero z_lo = zero_of<ActT>(__byte_perm(w.mt[t].y, 0, 0x1010)), z_hi = zero_of<ActT>(__byte_perm(w.mt[t].y, 0, 0x3232));
+        uint32_t s_lo = 0, s_hi = 0;
+        if constexpr (!PROMOTE) {
+            s_lo = Mul<ActT>::template pair<CVT>(w.mt[t].x & 0xFFFFu);
+            s_hi = Mul<ActT>::template pair<CVT>(w.mt[t].x >> 16);
+        }
+        const uint32_t dst = taddr + (static_cast<uint32_t>(16 * t) << 16);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {  // 64 k = 32 columns
+            uint32_t r[16];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {  // k run 32 (2 half + i / 2) + 8 (i & 1), and the one 16 further on
+                uint32_t f[4];
+                Frag<ActT>::expand(w.wd[t][4 * half + i], z_lo, z_hi, f);
+                const int c = 4 * (i >> 1) + (i & 1);
+                if constexpr (PROMOTE) {
+                    r[2 * c] = f[0];
+                    r[2 * c + 1] = f[1];
+                    r[2 * (c + 2)] = f[2];
+                    r[2 * (c + 2) + 1] = f[3];
+                } else {
+                    r[2 * c] = Mul<ActT>::mul(f[0], s_lo);
+                    r[2 * c + 1] = Mul<ActT>::mul(f[1], s_hi);
+                    r[2 * (c + 2)] = Mul<ActT>::mul(f[2], s_lo);
+                    r[2 * (c + 2) + 1] = Mul<ActT>::mul(f[3], s_hi);
+                }
+            }
+            tmem_st_16x128b_x8(dst + 32 * half, r);
+        }
+    }
+}
+
+}  // namespace tm
+}  // namespace eq

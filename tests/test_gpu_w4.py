@@ -431,3 +431,43 @@ def test_gate_up_swiglu_in_one_call(m):
     else:
         with pytest.raises(ops.L.EmmyqError):
             ops.w4a16_gate_up_swiglu(act(x, "bf16"), w, workspace=ws, out=odd)
+
+
+# Rows and widths at which the weights-in-TMEM kernels change form: promoted sums (17-24 rows) against scaled weights, one
+# accumulator width to the next, one-CTA against pair tiles, K slices that meet in a cluster (narrow widths) and whole-K
+# tiles, partial column tiles of 128 and 256, one item of K.
+# Tolerance, against f32 sums over weights rounded once to the activation dtype (unit roundoff u: 2^-8 bf16, 2^-11 f16): the
+# output's rounding u, the scale's rounding to the activation dtype u (the same for a whole group) and the products'
+# rounding on either side, which averages over K: below 4 u of the largest output.
+EDGE_TOL = {"f16": 2.0**-9, "bf16": 2.0**-6}
+
+
+@pytest.mark.parametrize("m", [17, 24, 25, 32, 33, 64, 65, 128, 129, 240, 256, 257, 385])
+@pytest.mark.parametrize("k,n,dtype", [(128, 16, "f16"), (640, 528, "bf16"), (2048, 272, "f16"), (256, 4112, "bf16")])
+def test_rows_and_widths_at_kernel_edges(m, k, n, dtype):
+    from emmy_b200 import ops
+
+    qw, qz, sc, _ = synth.gptq_linear(k, n, seed=m, act_order=False)
+    x = synth.activations(m, k, dtype, seed=m + 1)
+    w = ops.w4_repack(dev(qw), dev(qz), dev(sc), 128, "gptq")
+    ws = torch.zeros(ops.L.load().eq_w4a16_workspace_bytes(m, n, k) + 256, dtype=torch.uint8, device="cuda")
+    y = ops.w4a16_linear(act(x, dtype), w, workspace=ws).float().cpu().numpy()
+    ref = ol.w4a16_linear(x, qw, qz, sc, 128, "gptq", dtype)
+    assert np.abs(y - ref).max() <= EDGE_TOL[dtype] * np.abs(ref).max()
+    assert not ws.any()  # and no bounded wait ran out: the status word is part of it
+
+
+@pytest.mark.parametrize("m", [17, 25, 64, 65, 128, 129, 300])
+@pytest.mark.parametrize("k,inter,dtype", [(128, 16, "f16"), (640, 592, "bf16"), (2048, 144, "f16")])
+def test_gate_up_rows_and_widths_at_kernel_edges(m, k, inter, dtype):
+    from emmy_b200 import ops
+
+    gq, gz, gs, _ = synth.gptq_linear(k, inter, seed=m, act_order=False)
+    uq, uz, us, _ = synth.gptq_linear(k, inter, seed=m + 1, act_order=False)
+    x = synth.activations(m, k, dtype, seed=m + 2)
+    parts = [ops.w4_repack(dev(a), dev(b), dev(c), 128, "gptq") for a, b, c in ((gq, gz, gs), (uq, uz, us))]
+    h = ops.w4a16_gate_up_swiglu(act(x, dtype), ops.w4_concat(parts)).float().cpu().numpy()
+    qw, qz, sc = (np.concatenate(p, axis=1) for p in ((gq, uq), (gz, uz), (gs, us)))
+    ref = ol.w4a16_gate_up_swiglu(x, qw, qz, sc, 128, "gptq", dtype)
+    # two projections, the activation and the product are rounded (and gate enters twice): three times the linear's bound
+    assert np.abs(h - ref).max() <= 3 * EDGE_TOL[dtype] * np.abs(ref).max()

@@ -1,7 +1,8 @@
-// W4A16 linear for prefill-shaped calls (M > 16): y[M,N] = x[M,K] @ W on the tcgen05 tensor cores.
+// Grouped W4A16 GEMM of the expert-parallel MoE layer: 256-row blocks of one expert each, weights dequantised into shared
+// memory, on the tcgen05 tensor cores; and the dense prefill entry, which picks between w4_tmem.cu and w4_tmem2.cu.
 //
-// The int4 weight never exists as a 16-bit matrix in global memory.  A CTA owns a tile of 128 or 256 activation
-// rows by BN output columns and walks K in steps of 64:
+// The int4 weight never exists as a 16-bit matrix in global memory.  A CTA owns a tile of 256 activation rows by BN output
+// columns and walks K in steps of 64:
 //   warp 0        TMA producer: the 64-wide slice of the x rows, 128-byte swizzle, into the stage's A tile
 //   warp 1        MMA issuer: tcgen05.mma kind::f16, 128 x BN x 16 per instruction, f32 accumulators in TMEM (one
 //                 accumulator per 128 activation rows; both read the same B tile)
@@ -24,6 +25,8 @@
 
 namespace eq {
 
+int w4_tmem_pair_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
+                              int* status, cudaStream_t stream);  // w4_tmem2.cu
 int w4_tmem_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
                          bool promote, int* status, cudaStream_t stream);  // w4_tmem.cu
 
@@ -115,15 +118,12 @@ __global__ void gather_cols_kernel(const ActT* __restrict__ x, const int32_t* __
     xg[idx] = x[m * K + perm[k]];
 }
 
-// Rows of the TMA box of the activation tile for single-half plain tiles: the row count rounded up to a swizzle atom.
-__host__ __device__ inline int a_box_rows(int M) { return M >= 121 ? 128 : (M + 7) / 8 * 8; }
-
-// MODE: kPlain: one weight, CTA row tile = blockIdx.y.  kGrouped: blockIdx.y walks a device-side list of row blocks, each
-// a run of rows of ONE expert in an expert-ordered activation matrix; the weight is that expert's slice of a stacked
-// tensor and output rows may be scattered through y_rows.  kGroupedSwiGLU: the same, with the first 128 columns of the
-// CTA's B tile taken from the gate half and the last 128 from the up half of a [gate | up] weight, and the epilogue
-// writing act(silu(gate)) * up (emmy/compiler/trace/huggingface.py:1663-1669) into a matrix of N / 2 columns.
-enum GemmMode { kPlain = 0, kGrouped = 1, kGroupedSwiGLU = 2 };
+// kGrouped: blockIdx.y walks a device-side list of row blocks, each a run of rows of ONE expert in an expert-ordered
+// activation matrix; the weight is that expert's slice of a stacked tensor and output rows may be scattered through y_rows.
+// kGroupedSwiGLU: the same, with the first 128 columns of the CTA's B tile taken from the gate half and the last 128 from the
+// up half of a [gate | up] weight, and the epilogue writing act(silu(gate)) * up
+// (emmy/compiler/trace/huggingface.py:1663-1669) into a matrix of N / 2 columns.
+enum GemmMode { kGrouped = 1, kGroupedSwiGLU = 2 };
 
 struct GroupArgs {
     const RowBlock* blocks;
@@ -133,22 +133,10 @@ struct GroupArgs {
     size_t expert_stride;    // bytes between the experts' repacked weights
 };
 
-// SPLIT (plain mode only): gridDim.z CTAs share one output tile, each contracting a run of whole items of K.  Partial
-// sums meet in an f32 scratch [M][N] by vector reductions; the CTA whose arrival completes the tile converts it, stores y
-// and leaves scratch and counter zero.  Nobody waits.
-struct SplitArgs {
-    float* partial;     // [M][N], zero between calls
-    int* counters;      // one per column tile of this kernel, zero between calls
-};
-
-__device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
-template <typename ActT, int HALVES, int BN, int DW, int AHEAD, bool CVT, int MODE, bool SPLIT = false>
+template <typename ActT, int HALVES, int BN, int DW, int AHEAD, bool CVT, int MODE>
 __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
     w4a16_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const unsigned char* __restrict__ wq, ActT* __restrict__ y,
-                         int M, int N, int K, int* __restrict__ status, const GroupArgs grp, const SplitArgs split) {
+                         int N, int K, int* __restrict__ status, const GroupArgs grp) {
     using Cfg = GemmCfg<HALVES, BN, DW, AHEAD>;
     constexpr int kStages = Cfg::kStages;
     constexpr int kAhead = Cfg::kAhead;
@@ -163,29 +151,14 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
     uint64_t* acc_ready = bars + 3 * kStages;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 1);
 
-    // Plain launches are programmatic dependents (launch_cfg): the next grid may start its prologue and its first weight
-    // loads while this one runs, and this one does the same behind its predecessor.  Weights never depend on the
-    // previous grid; x, y and the split-K scratch may, so the warps that touch them wait below.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * BN;
-    int m0 = blockIdx.y * (128 * HALVES), m_end = M;
-    if constexpr (MODE != kPlain) {
-        if (static_cast<int>(blockIdx.y) >= *grp.n_blocks) return;  // the whole CTA, before any barrier exists
-        const RowBlock rb = grp.blocks[blockIdx.y];
-        m0 = rb.row0;
-        m_end = rb.row0 + rb.rows;
-        wq += static_cast<size_t>(rb.expert) * grp.expert_stride;
-    }
+    if (static_cast<int>(blockIdx.y) >= *grp.n_blocks) return;  // the whole CTA, before any barrier exists
+    const RowBlock rb = grp.blocks[blockIdx.y];
+    const int m0 = rb.row0, m_end = rb.row0 + rb.rows;
+    wq += static_cast<size_t>(rb.expert) * grp.expert_stride;
     const int items = K / 128;
-    // this CTA's run of items (all of K unless SPLIT), in K steps of 64
-    int item_lo = 0, item_hi = items;
-    if constexpr (SPLIT) {
-        item_lo = static_cast<int>(static_cast<long long>(items) * blockIdx.z / gridDim.z);
-        item_hi = static_cast<int>(static_cast<long long>(items) * (blockIdx.z + 1) / gridDim.z);
-    }
-    const int kb_lo = 2 * item_lo;
-    const int k_blocks = 2 * (item_hi - item_lo);
+    const int k_blocks = 2 * items;
     const int live_halves = min(HALVES, (m_end - m0 + 127) / 128);  // 128-row blocks of this tile that hold rows
 
     if (threadIdx.x == 0) {
@@ -210,7 +183,6 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
         // ---- TMA producer of the activation tiles
         if (tc::elect_one()) {
             tc::tma_prefetch_desc(&map_x);
-            asm volatile("griddepcontrol.wait;" ::: "memory");  // x may be the previous grid's output
             int stage = 0;
             uint32_t phase = 0;
             bool first = true;
@@ -223,12 +195,9 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
                 // one copy per TMA box (Cfg::kBoxHalves 128-row halves); halves without rows are not fetched
                 constexpr int kBoxBytes = Cfg::kBoxHalves * 128 * kRowBytes;
                 const int boxes = (live_halves + Cfg::kBoxHalves - 1) / Cfg::kBoxHalves;
-                // single-half plain tiles of fewer than 128 rows use a shorter box (see a_box_rows): rows past it keep
-                // whatever the stage held, and the accumulator rows they feed are never stored
-                const int box_bytes = (HALVES == 1 && MODE == kPlain) ? a_box_rows(M) * kRowBytes : kBoxBytes;
-                tc::mbar_expect_tx(bar, boxes * box_bytes);
+                tc::mbar_expect_tx(bar, boxes * kBoxBytes);
                 for (int bx = 0; bx < boxes; ++bx)
-                    tc::tma_load_2d(a_base + stage * Cfg::kTileA + bx * kBoxBytes, &map_x, (kb_lo + kb) * kGK, m0 + 128 * Cfg::kBoxHalves * bx, bar);
+                    tc::tma_load_2d(a_base + stage * Cfg::kTileA + bx * kBoxBytes, &map_x, kb * kGK, m0 + 128 * Cfg::kBoxHalves * bx, bar);
                 if (++stage == kStages) {
                     stage = 0;
                     phase ^= 1;
@@ -289,14 +258,14 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
             }
             live[nt] = tile < N / 16;
             const unsigned char* rec = wq + static_cast<size_t>(live[nt] ? tile : 0) * items * kItemBytes;
-            wp[nt] = rec + static_cast<size_t>(item_lo) * kItemBytes + h * 512 + (4 * g + jj) * 16;
-            mp[nt] = rec + static_cast<size_t>(item_lo) * kItemBytes + 1024 + g * 8;
+            wp[nt] = rec + h * 512 + (4 * g + jj) * 16;
+            mp[nt] = rec + 1024 + g * 8;
             off_lo[nt] = static_cast<uint32_t>((tile_in_cta * 16 + g) * kRowBytes + (((4 * jj + h) ^ g) << 4));
         }
         // register ring of whole items (two K steps each)
         uint4 w0[kAhead][Cfg::kTilesPerWarp], w1[kAhead][Cfg::kTilesPerWarp];
         uint2 meta[kAhead][Cfg::kTilesPerWarp];
-        const int my_items = item_hi - item_lo;
+        const int my_items = items;
 #pragma unroll
         for (int d = 0; d < kAhead; ++d) {
             if (d < my_items) {
@@ -308,7 +277,6 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
                 }
             }
         }
-        asm volatile("griddepcontrol.wait;" ::: "memory");  // these warps store y / add into the split-K scratch later
         bool broken = false, first = true;
         int stage = 0;
         uint32_t phase = 0;
@@ -456,15 +424,13 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
             bool row_ok = m < m_end;
             size_t out_row = static_cast<size_t>(m);
             ActT* out_base = y;
-            if constexpr (MODE != kPlain) {
-                if (row_ok && grp.y_ptrs) {
-                    // the row's own destination: results go straight to the rank that owns the token
-                    out_base = reinterpret_cast<ActT*>(grp.y_ptrs[m]);
-                    out_row = 0;
-                    row_ok = out_base != nullptr;
-                } else if (row_ok && grp.y_rows) {
-                    out_row = static_cast<size_t>(grp.y_rows[m]);
-                }
+            if (row_ok && grp.y_ptrs) {
+                // the row's own destination: results go straight to the rank that owns the token
+                out_base = reinterpret_cast<ActT*>(grp.y_ptrs[m]);
+                out_row = 0;
+                row_ok = out_base != nullptr;
+            } else if (row_ok && grp.y_rows) {
+                out_row = static_cast<size_t>(grp.y_rows[m]);
             }
             const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * BN;
             if constexpr (MODE == kGroupedSwiGLU) {
@@ -501,25 +467,6 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
                         }
                     }
                 }
-            } else if constexpr (SPLIT) {
-                {
-                    uint32_t r[32];
-                    tc::tmem_ld_32x32(t_row + c, r);
-                    tc::tmem_ld_wait();
-                    if (row_ok && n0 + c < N) {
-                        float* dst = split.partial + static_cast<size_t>(m) * N + n0 + c;
-                        if (n0 + c + 32 <= N) {
-#pragma unroll
-                            for (int v = 0; v < 8; ++v)
-                                red_add_v4(dst + 4 * v, __uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]), __uint_as_float(r[4 * v + 2]),
-                                           __uint_as_float(r[4 * v + 3]));
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                                if (n0 + c + i < N) atomicAdd(dst + i, __uint_as_float(r[i]));
-                        }
-                    }
-                }
             } else {
                 {
                     uint32_t r[32];
@@ -547,33 +494,6 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
                 }
             }
         }
-        if constexpr (SPLIT) {
-            // the epilogue warps of this CTA meet, one of them counts the CTA in; the last CTA of the tile finishes it
-            __shared__ int s_last;
-            __threadfence();
-            asm volatile("bar.sync 1, %0;" ::"n"(Cfg::kDequantWarps * 32) : "memory");
-            if (dw == 0 && lane == 0) s_last = atomicAdd(split.counters + blockIdx.x, 1) == static_cast<int>(gridDim.z) - 1;
-            asm volatile("bar.sync 1, %0;" ::"n"(Cfg::kDequantWarps * 32) : "memory");
-            if (s_last) {
-                __threadfence();
-                const int rows = min(m_end - m0, 128 * HALVES);
-                const int cols = min(BN, N - n0);  // multiples of 16
-                for (int idx = (dw * 32 + lane) * 4; idx < rows * cols; idx += Cfg::kDequantWarps * 32 * 4) {
-                    const int rr = idx / cols, cc = idx - rr * cols;
-                    float4* src = reinterpret_cast<float4*>(split.partial + static_cast<size_t>(m0 + rr) * N + n0 + cc);
-                    const float4 v = __ldcg(src);
-                    __stcg(src, make_float4(0.f, 0.f, 0.f, 0.f));
-                    const ActT o0 = from_float<ActT>(v.x), o1 = from_float<ActT>(v.y), o2 = from_float<ActT>(v.z), o3 = from_float<ActT>(v.w);
-                    uint2 pk;
-                    pk.x = static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(&o0)) | (static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(&o1)) << 16);
-                    pk.y = static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(&o2)) | (static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(&o3)) << 16);
-                    *reinterpret_cast<uint2*>(y + static_cast<size_t>(m0 + rr) * N + n0 + cc) = pk;
-                }
-                if (dw == 0 && lane == 0) split.counters[blockIdx.x] = 0;
-            }
-        }
-        if (lane == 0 && dw == 0) {
-        }
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -583,39 +503,22 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
     }
 }
 
-// Launch, as a programmatic dependent of the stream's previous kernel when asked (plain linears; the grouped modes read a
-// block list the previous kernel wrote before anything else and stay ordinary launches).
-template <typename Kernel, typename... Args>
-int launch_pdl(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t stream, bool dependent, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(static_cast<unsigned>(threads));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = dependent ? 1 : 0;
-    EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, args...));
-    return EQ_OK;
-}
-
 template <typename ActT, int HALVES, int BN, int DW, int AHEAD, int MODE>
 int launch_cfg(const unsigned char* wq, int scale_dtype, const ActT* x, ActT* y, int64_t M, int64_t N, int64_t K, int* status,
                const GroupArgs& grp, unsigned grid_y, cudaStream_t stream) {
     using Cfg = GemmCfg<HALVES, BN, DW, AHEAD>;
     CUtensorMap map_x;
     const CUtensorMapDataType elem = ScaleMul<ActT>::kFmt == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    const int box_rows = (HALVES == 1 && MODE == kPlain) ? a_box_rows(static_cast<int>(M)) : 128 * Cfg::kBoxHalves;
+    const int box_rows = 128 * Cfg::kBoxHalves;
     int st = make_tensor_map_2d(&map_x, x, elem, 2, M, K, K * 2, box_rows, kGK, CU_TENSOR_MAP_SWIZZLE_128B);
     if (st != EQ_OK) return st;
     const bool cvt = scale_dtype != (ScaleMul<ActT>::kFmt == 0 ? EQ_F16 : EQ_BF16);
     auto kernel = cvt ? w4a16_gemm_tc_kernel<ActT, HALVES, BN, DW, AHEAD, true, MODE> : w4a16_gemm_tc_kernel<ActT, HALVES, BN, DW, AHEAD, false, MODE>;
     EQ_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmem)));
     dim3 grid(static_cast<unsigned>(ceil_div(N, BN)), grid_y);
-    return launch_pdl(kernel, grid, Cfg::kThreads, Cfg::kSmem, stream, MODE == kPlain, map_x, wq, y, static_cast<int>(M), static_cast<int>(N),
-                      static_cast<int>(K), status, grp, SplitArgs{nullptr, nullptr});
+    kernel<<<grid, Cfg::kThreads, Cfg::kSmem, stream>>>(map_x, wq, y, static_cast<int>(N), static_cast<int>(K), status, grp);
+    EQ_LAUNCH_OK("w4a16_gemm_tc_kernel");
+    return EQ_OK;
 }
 
 template <typename ActT>
@@ -627,11 +530,9 @@ int launch_typed(const unsigned char* wq, int scale_dtype, const int32_t* perm, 
         EQ_LAUNCH_OK("gather_cols_kernel");
         x = gathered;
     }
-    const GroupArgs none = {nullptr, nullptr, nullptr, nullptr, 0};
-    if (!w4_tmem_pairs(M, N)) return w4_tmem_dense_launch(wq, scale_dtype, x, y, M, N, K, ScaleMul<ActT>::kFmt == 0 ? EQ_F16 : EQ_BF16, false, false, status, stream);
-    if (ceil_div(N, 256) * ceil_div(M, 256) >= sm_count())
-        return launch_cfg<ActT, 2, 256, 16, 2, kPlain>(wq, scale_dtype, x, y, M, N, K, status, none, static_cast<unsigned>(ceil_div(M, 256)), stream);
-    return launch_cfg<ActT, 2, 128, 16, 3, kPlain>(wq, scale_dtype, x, y, M, N, K, status, none, static_cast<unsigned>(ceil_div(M, 256)), stream);
+    const int act = ScaleMul<ActT>::kFmt == 0 ? EQ_F16 : EQ_BF16;
+    if (!w4_tmem_pairs(M, N)) return w4_tmem_dense_launch(wq, scale_dtype, x, y, M, N, K, act, false, false, status, stream);
+    return w4_tmem_pair_dense_launch(wq, scale_dtype, x, y, M, N, K, act, false, status, stream);
 }
 
 }  // namespace

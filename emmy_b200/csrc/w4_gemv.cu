@@ -4,8 +4,8 @@
 //   2 <= M <= 16   w4a16_stream_kernel (w4_stream.cu): one fat CTA per SM streams whole column tiles, x staged in shared
 //                  memory (whole, or a K slice per CTA with the slices meeting in the workspace).  Weights with a row
 //                  permutation stay with it up to 24 rows where a slice of x fits.
-//   M > 16         w4a16_tmem_kernel (w4_tmem.cu): tcgen05 with the weights expanded into tensor
-//                  memory; larger calls w4a16_gemm_tc_kernel (w4_gemm.cu), which expands them into shared memory.
+//   M > 16         w4a16_tmem_kernel (w4_tmem.cu) and, for larger calls, w4a16_tmem_pair_kernel (w4_tmem2.cu): tcgen05 with
+//                  the weights expanded into tensor memory.
 //   w4a16_tile_kernel below: M > 16 with an output that is not 16-byte aligned (in 64-row blocks), and decode
 //   shapes whose activations do not fit shared memory (K beyond about 100 k at M == 1).
 //
@@ -29,6 +29,8 @@ namespace eq {
 int w4_stream_launch(const W4Params& p, int act_dtype, cudaStream_t stream, bool* fits);  // w4_stream.cu
 int w4_gemv1_launch(const unsigned char* wq, int scale_dtype, const int32_t* perm, const void* x, void* y, int64_t N, int64_t K,
                     int act_dtype, uint32_t* xchg, int* status, cudaStream_t stream, bool* fits);  // w4_gemv1.cu
+int w4_tmem_pair_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
+                              int* status, cudaStream_t stream);  // w4_tmem2.cu
 int w4_tmem_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
                          bool promote, int* status, cudaStream_t stream);  // w4_tmem.cu
 int w4_gemm_tc_launch(const unsigned char* wq, int scale_dtype, const int32_t* perm, const void* x, void* y, int64_t M, int64_t N,
@@ -213,17 +215,6 @@ extern "C" int eq_w4a16_linear(const void* wq, int scale_dtype, const int32_t* p
 namespace eq {
 namespace {
 
-__global__ void dense_row_blocks_kernel(RowBlock* __restrict__ blocks, int32_t* __restrict__ n_blocks, int M) {
-    const int nb = (M + 255) / 256;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-        blocks[b].expert = 0;
-        blocks[b].row0 = b * 256;
-        blocks[b].rows = min(256, M - b * 256);
-        blocks[b].pad = 0;
-    }
-    if (threadIdx.x == 0) *n_blocks = nb;
-}
-
 // h[r][i] = act(silu(gu[r][i])) * gu[r][I + i], eight columns per thread (I is a multiple of 16).  A programmatic
 // dependent of the linear that wrote gu, and a primary of the kernel after it: that one is resident, with its weights on
 // the way, while this one runs.
@@ -269,20 +260,15 @@ int launch_swiglu_rows(const void* gu, int64_t M, int64_t I, void* h, cudaStream
 }
 
 size_t gu_align(size_t v) { return (v + 255) / 256 * 256; }
-size_t gu_blocks_bytes(int64_t M) { return gu_align((static_cast<size_t>((M + 255) / 256) + 1) * sizeof(RowBlock)); }
 
 }  // namespace
-
-int w4_gemm_tc_grouped_launch(const unsigned char* wq, size_t expert_stride, int scale_dtype, const void* x, void* y, int64_t R, int64_t N,
-                              int64_t K, int act_dtype, const RowBlock* blocks, const int32_t* n_blocks, int max_blocks,
-                              const int32_t* y_rows, const uint64_t* y_ptrs, bool swiglu, int* status, cudaStream_t stream);  // w4_gemm.cu
 
 }  // namespace eq
 
 extern "C" size_t eq_w4a16_gate_up_workspace_bytes(int64_t M, int64_t I, int64_t K) {
     if (M <= 0 || I <= 0 || K <= 0) return 0;
-    // the linear's own workspace, then the row-block list (M > 16) or the [M, 2 I] scratch (M <= 16)
-    return gu_align(eq_w4a16_workspace_bytes(M, 2 * I, K)) + (M > 16 ? gu_blocks_bytes(M) : gu_align(static_cast<size_t>(M) * 2 * I * 2));
+    // the linear's own workspace, then the [M, 2 I] scratch (M <= 16)
+    return gu_align(eq_w4a16_workspace_bytes(M, 2 * I, K)) + (M > 16 ? 0 : gu_align(static_cast<size_t>(M) * 2 * I * 2));
 }
 
 extern "C" int eq_w4a16_gate_up_swiglu(const void* wq, int scale_dtype, const int32_t* perm, int64_t K, int64_t I, int64_t G, const void* x,
@@ -304,13 +290,7 @@ extern "C" int eq_w4a16_gate_up_swiglu(const void* wq, int scale_dtype, const in
         int* status = static_cast<int*>(workspace);  // sticky until eq_w4a16_status reports it, as in eq_w4a16_linear
         if (!w4_tmem_pairs(M, 2 * I))
             return w4_tmem_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, h, M, 2 * I, K, act_dtype, true, false, status, stream);
-        RowBlock* blocks = reinterpret_cast<RowBlock*>(extra);
-        const int nb = static_cast<int>((M + 255) / 256);
-        int32_t* n_blocks = reinterpret_cast<int32_t*>(blocks + nb);
-        dense_row_blocks_kernel<<<1, 256, 0, stream>>>(blocks, n_blocks, static_cast<int>(M));
-        EQ_LAUNCH_OK("dense_row_blocks_kernel");
-        return w4_gemm_tc_grouped_launch(static_cast<const unsigned char*>(wq), 0, scale_dtype, x, h, M, 2 * I, K, act_dtype, blocks, n_blocks, nb, nullptr,
-                                         nullptr, true, status, stream);
+        return w4_tmem_pair_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, h, M, 2 * I, K, act_dtype, true, status, stream);
     }
     // few rows, scattered act-order groups or an unaligned output: the [gate | up] linear, then the activation
     EQ_REQUIRE(M <= 16, EQ_ERR_UNSUPPORTED, "eq_w4a16_gate_up_swiglu: M > 16 needs a 16-byte aligned output and a weight without a row permutation");

@@ -13,8 +13,10 @@ namespace eq {
 // the MMA, which at 28 rows costs 15.8 against 20.0 promoted.
 constexpr int64_t kTmemMinRows = 17, kTmemPromoteRows = 24;
 
-// More than 256 rows whose 256 x 256 tiles occupy at least a quarter of the SMs stay with w4_gemm.cu, the rest run on tiles of
-// 128 channels and at most 128 rows, with K slices where CTAs would idle.
+// More than 256 rows whose 256 x 256 tiles occupy at least half of the CTA pairs run on pairs (w4_tmem2.cu), the rest on
+// one-CTA tiles of at most 128 rows with K slices where CTAs would idle.  Measured, one-CTA against pairs: MLP 256 rows
+// 94.9 : 101.3, 300 rows 158 : 134, 512 rows 182 : 158, 4096 rows 1266 : 1076; K=N=4096, 512 rows (32 tiles) 23.2 : 28.0;
+// K=4096 N=1792, 2048 rows (56 tiles) 33.5 : 28.8.
 inline bool w4_tmem_pairs(int64_t M, int64_t N) { return M > 256 && ceil_div(N, 256) * ceil_div(M, 256) * 4 >= sm_count(); }
 
 struct W4TmemArgs {

@@ -14,11 +14,13 @@
 //                         rows of ONE expert, its weights are that expert's slice of the stacked repacked tensor.
 //                         Rows are gathered (first GEMM) / scattered (second GEMM) through index arrays, nothing is
 //                         copied.  Body: the W4A16 tile code of w4_tile.cuh.
-//                         With many rows per expert the two GEMMs run on the tensor path instead (w4_gemm.cu): rows are
-//                         first copied into expert order (moe_gather_rows_kernel) so that TMA can read them, row
-//                         blocks are 256 rows, and SwiGLU is fused into the first GEMM's epilogue.
-//   streaming tier        up to eight rows per expert on average (and more tokens than the decode tier takes): the plan's
-//                         row blocks hold at most eight rows and both grouped linears run through moe_stream.cu, which
+//                         With three rows per expert and more the two GEMMs run on the tensor path instead (w4_tmem.cu):
+//                         rows are first copied into expert order (moe_gather_rows_kernel) so that TMA can read them, row
+//                         blocks are 16 rows up to eight rows per expert and 128 above, and SwiGLU is fused into the first
+//                         GEMM's epilogue.  (The expert-parallel layer has 256-row blocks on w4_gemm.cu, whose epilogue
+//                         stores whole lines to peers.)
+//   streaming tier        fewer rows per expert (and more tokens than the decode tier takes): the plan's row blocks hold
+//                         at most eight rows and both grouped linears run through moe_stream.cu, which
 //                         streams every touched expert's weights once per block; SwiGLU is a kernel of its own between.
 //   moe_swiglu_kernel     h = silu(gate) * up with the roundings of the eager form
 //                         (emmy/compiler/trace/huggingface.py:1663-1669).
@@ -27,6 +29,7 @@
 #include <type_traits>
 
 #include "w4_tile.cuh"
+#include "w4_tmem.cuh"
 
 namespace eq {
 
@@ -41,6 +44,10 @@ int moe_stream_launch(const unsigned char* wq, size_t expert_stride, int scale_d
 int w4_gemm_tc_grouped_launch(const unsigned char* wq, size_t expert_stride, int scale_dtype, const void* x, void* y, int64_t R, int64_t N,
                               int64_t K, int act_dtype, const RowBlock* blocks, const int32_t* n_blocks, int max_blocks,
                               const int32_t* y_rows, const uint64_t* y_ptrs, bool swiglu, int* status, cudaStream_t stream);  // w4_gemm.cu
+
+int w4_tmem_grouped_launch(const unsigned char* wq, size_t expert_stride, int scale_dtype, const void* x, void* y, int64_t R, int64_t N, int64_t K,
+                           int act_dtype, const RowBlock* blocks, const int32_t* n_blocks, int block_rows, const int32_t* y_rows, const uint64_t* y_ptrs,
+                           bool swiglu, int* status, cudaStream_t stream);  // w4_tmem.cu
 
 constexpr int kMaxTopK = 16;
 constexpr int kBadExpertId = 16;  // status code of a row whose expert id is out of range (1..4 are the tensor path's waits)
@@ -367,13 +374,18 @@ struct MoeWorkspace {
     size_t bytes;
 };
 
-// Rows per expert at which the grouped GEMMs move to the tensor path (256-row blocks).
-// Up to eight rows per expert on average the layer is a weight stream with a little math attached: row blocks of eight
-// rows through the streaming tier (moe_stream.cu; the tile code serves shapes it cannot hold).  Above that the tensor
-// path with 256-row blocks.
+// Up to eight rows per expert on average the layer is a weight stream with a little math attached, and the scales are
+// applied to f32 sums: row blocks of eight rows through the streaming tier (moe_stream.cu; the tile code serves shapes it
+// cannot hold) or of sixteen through the tensor path.  Above, scaled weights in 128-row blocks: two CTAs an SM overlap each
+// other's epilogues and a ragged last block wastes little (T = 256 / 1024 / 4096 of the Qwen3-30B-A3B layer: 144 / 194 / 490
+// us; the 256-row tiles of w4_gemm.cu 300 / 323 / 557, 256-row blocks on CTA pairs 184 / 236 / 502).
 static bool stream_rows(int64_t R, int64_t E) { return R <= 8 * E; }
 static bool tensor_path(int64_t R, int64_t E) { return !stream_rows(R, E); }
-static int block_rows_for(int64_t R, int64_t E) { return tensor_path(R, E) ? 256 : 8; }
+static int block_rows_for(int64_t R, int64_t E) { return tensor_path(R, E) ? 128 : 8; }
+// From three rows per expert on the weights-in-TMEM kernel with 16-row blocks beats the streaming tier (Qwen3-30B-A3B layer,
+// 48 / 64 / 128 tokens = 3 / 4 / 8 rows an expert: 134 / 135 / 138 us against 141 / 157 / 220; at 1.25 and 2 rows the two are
+// even, 109 : 111 and 128 : 128, and the streaming tier needs no copy of the rows).
+static bool tmem_rows(int64_t R, int64_t E) { return R >= 3 * E; }
 
 static MoeWorkspace carve(void* base, int64_t T, int64_t E, int64_t topk, int64_t H, int64_t I) {
     MoeWorkspace w;
@@ -421,7 +433,9 @@ template <typename ActT>
 static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const void* wq_down, int scale_dtype, int64_t E, int64_t H,
                            int64_t I, const void* x, const int32_t* src_row, int src_div, const int32_t* eid, int64_t R, void* out,
                            const uint64_t* row_ptr, cudaStream_t stream) {
-    const int br = block_rows_for(R, E);
+    // few rows per expert: 16-row blocks of the weights-in-TMEM kernel where TMA can read the rows
+    const bool tensor = tensor_path(R, E), tmem = tensor || (tmem_rows(R, E) && aligned(x, 16) && aligned(out, 16));
+    const int br = tmem && !tensor ? 16 : block_rows_for(R, E);
     if (R <= kSmallPlanRows) {
         moe_plan_small_kernel<<<1, 1024, 3 * E * sizeof(int32_t), stream>>>(eid, src_row, src_div, static_cast<int>(R), static_cast<int>(E), br, w.offsets,
                                                                             w.blocks, w.n_blocks, w.max_blocks, w.src_of, w.dst_of, row_ptr, w.dst_ptr,
@@ -438,7 +452,7 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
                                                                                       w.cursor, w.src_of, w.dst_of, row_ptr, w.dst_ptr, src_div);
         EQ_LAUNCH_OK("moe_scatter_kernel");
     }
-    if (tensor_path(R, E)) {
+    if (tmem) {
         // rows into expert order (the region of the second GEMM's output in the workspace is free until then)
         const int act = sizeof(ActT) == 2 && std::is_same<ActT, __half>::value ? EQ_F16 : EQ_BF16;
         const int row_vec = static_cast<int>(H * 2 / 16);
@@ -447,13 +461,11 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
         moe_gather_rows_kernel<<<static_cast<unsigned>(gather_ctas < 32LL * sm_count() ? gather_ctas : 32LL * sm_count()), 256, 0, stream>>>(
             static_cast<const uint4*>(x), w.src_of, w.offsets + E, row_vec, reinterpret_cast<uint4*>(w.out));
         EQ_LAUNCH_OK("moe_gather_rows_kernel");
-        int st = w4_gemm_tc_grouped_launch(static_cast<const unsigned char*>(wq_gate_up), static_cast<size_t>(2 * I / 16) * (H / 128) * kItemBytes,
-                                           scale_dtype, w.out, w.h, R, 2 * I, H, act, w.blocks, w.n_blocks, w.max_blocks, nullptr, nullptr, true,
-                                           w.status, stream);
+        int st = w4_tmem_grouped_launch(static_cast<const unsigned char*>(wq_gate_up), static_cast<size_t>(2 * I / 16) * (H / 128) * kItemBytes, scale_dtype,
+                                        w.out, w.h, R, 2 * I, H, act, w.blocks, w.n_blocks, br, nullptr, nullptr, true, w.status, stream);
         if (st != EQ_OK) return st;
-        return w4_gemm_tc_grouped_launch(static_cast<const unsigned char*>(wq_down), static_cast<size_t>(H / 16) * (I / 128) * kItemBytes,
-                                         scale_dtype, w.h, out, R, H, I, act, w.blocks, w.n_blocks, w.max_blocks, w.dst_of,
-                                         row_ptr ? w.dst_ptr : nullptr, false, w.status, stream);
+        return w4_tmem_grouped_launch(static_cast<const unsigned char*>(wq_down), static_cast<size_t>(H / 16) * (I / 128) * kItemBytes, scale_dtype, w.h,
+                                      out, R, H, I, act, w.blocks, w.n_blocks, br, w.dst_of, row_ptr ? w.dst_ptr : nullptr, false, w.status, stream);
     }
     if (moe_stream_fits(w.max_blocks, 2 * I) && moe_stream_fits(w.max_blocks, H)) {
         const int act = std::is_same<ActT, __half>::value ? EQ_F16 : EQ_BF16;

@@ -79,6 +79,29 @@ def test_moe_layer_matches_oracle(t):
     assert float((got - ref).abs().max()) <= TOL * float(ref.abs().max())
 
 
+# Rows per expert at which the grouped kernels change form: 16-row blocks filled, overfilled and mostly empty, and the larger
+# blocks of the tensor tier (128 and 256 rows an expert and one more); widths that leave partial column tiles.
+@pytest.mark.parametrize("t,e,k", [(17, 16, 4), (40, 20, 4), (64, 32, 4), (66, 4, 1), (256, 4, 2), (258, 4, 2), (516, 4, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_moe_layer_at_row_block_edges(t, e, k, dtype):
+    from emmy_b200 import ops_moe as om
+
+    h, inter = 384, 128
+    ex = make_experts(e, h, inter, seed=300)
+    w = om.moe_repack(tuple(dev(a) for a in ex["gate_up"]), tuple(dev(a) for a in ex["down"]))
+    wgu, wdn = omoe.dequant_expert_weights(ex, dtype)
+    x = torch.from_numpy(synth.activations(t, h, "bf16" if dtype == torch.bfloat16 else "f16", seed=t)).to(dtype)
+    # every expert gets the same number of rows, but the first one more of expert 1's
+    logits = torch.zeros(t, e)
+    for j in range(k):
+        logits[torch.arange(t), (torch.arange(t) * k + j) % e] = 2.0 + 0.1 * j
+    logits[0, 1 % e] = 5.0
+    y = om.moe_forward(x.cuda(), logits.cuda(), w, k).float().cpu()
+    ref = omoe.moe_layer(x, logits, wgu, wdn, k).float()
+    assert torch.isfinite(y).all()
+    assert float((y - ref).abs().max()) <= TOL * float(ref.abs().max())
+
+
 def test_moe_layer_qwen3_shapes_decode():
     """128 experts, top-8, hidden 2048, intermediate 768, T = 1: the decode-shaped case at full width."""
     from emmy_b200 import ops_moe as om

@@ -146,6 +146,11 @@ def w4_unpack_repacked(w: W4Weight) -> torch.Tensor:
     return out
 
 
+def _scratch(need: int, device) -> torch.Tensor:
+    """Scratch of one call that reads nothing it has not written (the kernels' own writes cover it): no zero fill."""
+    return torch.empty(max(need, 256), dtype=torch.uint8, device=device)
+
+
 _workspaces: dict = {}
 
 
@@ -187,7 +192,8 @@ def w4a16_gate_up_swiglu(x: torch.Tensor, w: W4Weight, workspace: torch.Tensor |
     inter = w.n // 2
     h = out if out is not None else torch.empty((m, inter), dtype=x.dtype, device=x.device)
     need = L.load().eq_w4a16_gate_up_workspace_bytes(m, inter, k)
-    ws = workspace if workspace is not None else torch.zeros(max(need, 256), dtype=torch.uint8, device=x.device)
+    # up to 16 rows take kernels that meet in a workspace which is zero between calls; more rows read nothing of it
+    ws = workspace if workspace is not None else torch.zeros(max(need, 256), dtype=torch.uint8, device=x.device) if m <= 16 else _scratch(need, x.device)
     L.check(L.load().eq_w4a16_gate_up_swiglu(_ptr(w.wq), _DTYPE[w.scale_dtype], _ptr(w.perm), w.k, inter, w.group, _ptr(x), m, _DTYPE[x.dtype],
                                              _ptr(h), _ptr(ws), ws.numel(), _stream()))
     return h
@@ -243,7 +249,7 @@ def fp8_linear(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor
     if weight.shape[1] != k:
         raise ValueError(f"x has {k} features, the weight takes {weight.shape[1]}")
     y = out if out is not None else torch.empty((m, n), dtype=x.dtype, device=x.device)
-    ws = workspace if workspace is not None else fp8_workspace(m, k, x.device)
+    ws = workspace if workspace is not None else _scratch(L.load().eq_fp8_workspace_bytes(m, k), x.device)
     if norm_weight is not None:
         if input_scale is not None or norm_weight.dtype != x.dtype or norm_weight.numel() != k:
             raise ValueError("fp8_linear: norm_weight is [K] in x's dtype and excludes a static input_scale")
@@ -291,7 +297,7 @@ def fp8_block_linear(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.
         raise ValueError(f"block-scaled FP8: x {tuple(x.shape)}, weight {tuple(weight.shape)}, scale {tuple(weight_scale.shape)} do not fit")
     y = out if out is not None else torch.empty((m, n), dtype=x.dtype, device=x.device)
     need = L.load().eq_fp8_block_workspace_bytes(m, k)
-    ws = workspace if workspace is not None else torch.empty(max(need, 256), dtype=torch.uint8, device=x.device)
+    ws = workspace if workspace is not None else _scratch(need, x.device)
     L.check(L.load().eq_fp8_block_linear(_ptr(weight), _ptr(weight_scale), n, k, _ptr(x), m, _DTYPE[x.dtype], _ptr(y), _ptr(ws), ws.numel(), _stream()))
     return y
 

@@ -7,7 +7,7 @@ import ctypes as C
 import torch
 
 from . import lib as L
-from .ops import _DTYPE, _FMT, _need_cuda, _ptr, _stream
+from .ops import _DTYPE, _FMT, _need_cuda, _ptr, _scratch, _stream
 
 
 class MoEWeights:
@@ -69,7 +69,8 @@ def moe_experts(x, expert_ids, w: MoEWeights, src_row=None, workspace=None, out=
     _need_cuda(x, expert_ids, src_row)
     r = expert_ids.numel()
     y = out if out is not None else torch.empty((r, w.hidden), dtype=x.dtype, device=x.device)
-    ws = workspace if workspace is not None else moe_workspace(r, w, 1, x.device)
+    # (the grouped kernels write all they read)
+    ws = workspace if workspace is not None else _scratch(L.load().eq_moe_workspace_bytes(r, w.experts, 1, w.hidden, w.inter), x.device)
     L.check(
         L.load().eq_moe_experts_w4a16(
             _ptr(w.gate_up), _ptr(w.down), _DTYPE[w.scale_dtype], w.experts, w.hidden, w.inter, w.group, _ptr(x), _ptr(src_row),
@@ -92,7 +93,12 @@ def moe_forward(x, router_logits, w: MoEWeights, topk: int, workspace=None, out=
     _need_cuda(x, router_logits)
     t = x.shape[0]
     y = out if out is not None else torch.empty((t, w.hidden), dtype=x.dtype, device=x.device)
-    ws = workspace if workspace is not None else moe_workspace(t, w, topk, x.device)
+    if workspace is not None:
+        ws = workspace
+    elif t <= 16:  # the decode tier counts arrivals in words that are zero between calls
+        ws = moe_workspace(t, w, topk, x.device)
+    else:
+        ws = _scratch(L.load().eq_moe_workspace_bytes(t, w.experts, topk, w.hidden, w.inter), x.device)
     L.check(
         L.load().eq_moe_w4a16(
             _ptr(w.gate_up), _ptr(w.down), _DTYPE[w.scale_dtype], w.experts, topk, w.hidden, w.inter, w.group, _ptr(x),

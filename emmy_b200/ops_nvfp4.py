@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from . import lib as L
-from .ops import _DTYPE, _need_cuda, _ptr, _stream
+from .ops import _DTYPE, _need_cuda, _ptr, _scratch, _stream
 
 
 def nvfp4_global_scale(x: torch.Tensor) -> torch.Tensor:
@@ -78,7 +78,7 @@ def nvfp4_linear(x, weight, weight_scale_tiled, weight_scale_2, input_scale, wor
     if weight.shape[1] * 2 != k:
         raise ValueError(f"x has {k} features, the weight takes {weight.shape[1] * 2}")
     y = out if out is not None else torch.empty((m, n), dtype=x.dtype, device=x.device)
-    ws = workspace if workspace is not None else nvfp4_workspace(m, k, x.device)
+    ws = workspace if workspace is not None else _scratch(L.load().eq_nvfp4_workspace_bytes(m, k), x.device)
     if norm_weight is not None:
         if norm_weight.dtype != x.dtype or norm_weight.numel() != k:
             raise ValueError("nvfp4_linear: norm_weight is [K] in x's dtype")

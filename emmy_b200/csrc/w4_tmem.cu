@@ -375,10 +375,10 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
     if constexpr (SPLIT) {
         // The K slices of a tile are the CTAs of one cluster (one unit each): every CTA adds up and stores its share of the
         // rows from all partial tiles, in the slices' order.
-        cluster_sync();
+        tc::cluster_sync();
         int col, row0, rows, item0, n_items, expert;
         locate(blockIdx.x, col, row0, rows, item0, n_items, expert);
-        const int rank = static_cast<int>(cluster_rank());
+        const int rank = static_cast<int>(tc::cluster_rank());
         const int r_lo = rows * rank / a.splits, r_hi = rows * (rank + 1) / a.splits;
         const uint32_t part_addr = tc::smem_u32(part);
         constexpr int kPerRow = SWIGLU ? 16 : 32;  // threads of a row: four channels each
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
             float s[4] = {0.f, 0.f, 0.f, 0.f}, up[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
             for (int z = 0; z < a.splits; ++z) {
-                const uint32_t src = map_to_rank(part_addr, z) + static_cast<uint32_t>(r * 128 + at) * 4;
+                const uint32_t src = tc::map_to_rank(part_addr, z) + static_cast<uint32_t>(r * 128 + at) * 4;
                 const float4 v = ld_cluster_v4(src);
                 s[0] += v.x, s[1] += v.y, s[2] += v.z, s[3] += v.w;
                 if constexpr (SWIGLU) {
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                     make_uint2(bits16<ActT>(s[0]) | (bits16<ActT>(s[1]) << 16), bits16<ActT>(s[2]) | (bits16<ActT>(s[3]) << 16));
         }
         __syncwarp();
-        cluster_sync();  // nobody leaves while its partial tile may still be read
+        tc::cluster_sync();  // nobody leaves while its partial tile may still be read
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -458,8 +458,10 @@ int launch_dense(W4TmemArgs a, const void* x, int scale_dtype, cudaStream_t stre
     if (a.rows_per_tile > NB) a.rows_per_tile = NB;
     a.row_tiles = static_cast<int>(ceil_div(a.M, a.rows_per_tile));
     const int tiles = col_tiles * a.row_tiles, slots = 2 * sm_count();
-    // K slices (a cluster's CTAs, eight at most) where the tiles leave CTA slots idle; at least two items a slice
-    int splits = slots / tiles;
+    // K slices (a cluster's CTAs, eight at most) where the tiles leave CTA slots idle; at least two items a slice.  A cluster
+    // lives in one GPC, so not every slot can be filled: with 288 of the 296 asked for (K=14336 N=4096, 300 rows, clusters of
+    // three) a second wave ran and the call took 72 us.
+    int splits = (slots - slots / 8) / tiles;
     if (splits > items / 2) splits = items / 2;
     if (splits > 8) splits = 8;
     if (splits < 1) splits = 1;

@@ -15,8 +15,8 @@ constexpr int64_t kTmemMinRows = 17, kTmemPromoteRows = 24;
 
 // More than 256 rows whose 256 x 256 tiles occupy at least half of the CTA pairs run on pairs (w4_tmem2.cu), the rest on
 // one-CTA tiles of at most 128 rows with K slices where CTAs would idle.  Measured, one-CTA against pairs: MLP 256 rows
-// 94.9 : 101.3, 300 rows 158 : 134, 512 rows 182 : 158, 4096 rows 1266 : 1076; K=N=4096, 512 rows (32 tiles) 23.2 : 28.0;
-// K=4096 N=1792, 2048 rows (56 tiles) 33.5 : 28.8.
+// 94.9 : 101.3, 300 rows (both linears) 158 : 134, 1024 rows 317 : 277, 4096 rows 1266 : 1076; K=N=4096, 512 rows (32 tiles)
+// 21.2 : 28.0, K=14336 N=4096, 300 rows (32 tiles) 48 against 50; K=4096 N=1792, 2048 rows (56 tiles) 33.5 : 28.8.
 inline bool w4_tmem_pairs(int64_t M, int64_t N) { return M > 256 && ceil_div(N, 256) * ceil_div(M, 256) * 4 >= sm_count(); }
 
 struct W4TmemArgs {
@@ -52,21 +52,7 @@ __device__ __forceinline__ bool wait_asleep(uint32_t bar, uint32_t parity) {
     }
 }
 
-// ---- thread-block clusters
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+// ---- distributed shared memory
 __device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");

@@ -39,16 +39,6 @@ constexpr int64_t kExpandCycles = 480, kUnitCycles = 3500;  // of an SM: one ite
 static_assert(kNB + 64 * kStagesA <= 512, "accumulator and A stages fill TMEM");
 static_assert(kSmem <= 227 * 1024, "one CTA per SM");
 
-// Arrival on a barrier of either CTA.  What it hands over is TMEM contents, ordered by the tcgen05 fences on both sides; a
-// release at cluster scope would also wait for the weight copies this warp has in flight (measured: the largest stall).
-__device__ __forceinline__ void arrive_pair(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
-// The barrier may be the peer CTA's (a shared::cluster address); the data goes to this CTA's shared memory.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst), "l"(map),
-        "r"(bar), "r"(c0), "r"(c1)
-        : "memory");
-}
 __device__ __forceinline__ void mma_f16_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, bool accumulate) {
     const uint32_t acc = accumulate ? 1u : 0u;
     asm volatile(
@@ -57,12 +47,6 @@ __device__ __forceinline__ void mma_f16_ts_pair(uint32_t tmem_d, uint32_t tmem_a
         "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc)
         : "memory");
 }
-// The barrier at this offset of BOTH CTAs completes once the MMAs issued so far have.
-__device__ __forceinline__ void commit_pair(uint32_t bar) {
-    const uint16_t both = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(both) : "memory");
-}
-
 template <typename ActT, bool CVT, bool SWIGLU>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     w4a16_tmem_pair_kernel(const __grid_constant__ CUtensorMap map_x, const W4TmemArgs a) {
@@ -77,7 +61,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                    acc_full = empty_b + 8 * kStagesB, acc_empty = acc_full + 8;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_rank();
+    const uint32_t rank = tc::cluster_rank();
     const int cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
     const int items = a.K / 128, n_tiles = a.N / 16;  // SWIGLU: a CTA's channels are four gate and four up tiles
     const int units = a.units;
@@ -104,17 +88,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         tc::mbar_fence_init();
     }
     if (warp == kWarps - 1) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        tc::tmem_alloc_pair(tc::smem_u32(tmem_slot), kTmemCols);
     }
     tc::fence_before_sync();
     __syncthreads();
-    cluster_sync();  // the peer's barriers exist from here on
+    tc::cluster_sync();  // the peer's barriers exist from here on
     tc::fence_after_sync();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // with the TMEM columns in hand (w4_tmem.cu)
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_a = tmem_base + kNB;
-    const uint32_t lead_full_a = map_to_rank(full_a, 0), lead_full_b = map_to_rank(full_b, 0), lead_acc_empty = map_to_rank(acc_empty, 0);
+    const uint32_t lead_full_a = tc::map_to_rank(full_a, 0), lead_full_b = tc::map_to_rank(full_b, 0), lead_acc_empty = tc::map_to_rank(acc_empty, 0);
 
     if (warp < kDW) {
         const int q = warp & 3, wg = warp >> 2;
@@ -187,7 +170,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 tmem_st_wait();
                 tc::fence_before_sync();
                 __syncwarp();
-                if (lane == 0) arrive_pair(my_full);
+                if (lane == 0) tc::arrive_pair(my_full);
             }
             next -= items;
             // ---- epilogue: group wg takes the 16-row chunks wg, wg + 4, ...
@@ -215,7 +198,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
             tc::fence_before_sync();
             __syncwarp();
-            if (lane == 0) arrive_pair(lead_acc_empty);
+            if (lane == 0) tc::arrive_pair(lead_acc_empty);
         }
     } else if (warp == kWarps - 2) {
         if (tc::elect_one()) {
@@ -240,7 +223,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     const uint32_t dst = tiles_b + stage * kTileB;
                     for (int piece = 0; piece < 2; ++piece)
                         for (int bx = 0; bx < boxes; ++bx)
-                            tma_load_2d_pair(dst + piece * (kHalfRows * 128) + bx * (kBoxRows * 128), &map_x, it * 128 + piece * kGK, first + bx * kBoxRows,
+                            tc::tma_load_2d_pair(dst + piece * (kHalfRows * 128) + bx * (kBoxRows * 128), &map_x, it * 128 + piece * kGK, first + bx * kBoxRows,
                                              lead_full_b + 8 * stage);
                 }
             }
@@ -266,20 +249,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     for (int ks = 0; ks < 8; ++ks)
                         mma_f16_ts_pair(tmem_base, tmem_a + 64 * sa + 8 * ks, tc::smem_desc_k_sw128(b_addr + (ks >> 2) * (kHalfRows * 128) + (ks & 3) * 32), idesc,
                                         ks > 0 || it > 0);
-                    commit_pair(empty_a + 8 * sa);
-                    commit_pair(empty_b + 8 * sb);
+                    tc::commit_pair(empty_a + 8 * sa);
+                    tc::commit_pair(empty_b + 8 * sb);
                 }
                 if (broken) atomicExch(a.status, 2);
-                commit_pair(acc_full);
+                tc::commit_pair(acc_full);
             }
         }
     }
     __syncwarp();
     tc::fence_before_sync();
     __syncthreads();
-    cluster_sync();  // neither CTA leaves while the other may still signal it or read its rows
+    tc::cluster_sync();  // neither CTA leaves while the other may still signal it or read its rows
     tc::fence_after_sync();
-    if (warp == kWarps - 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+    if (warp == kWarps - 1) tc::tmem_dealloc_pair(tmem_base, kTmemCols);
 }
 
 template <typename ActT, bool SWIGLU>

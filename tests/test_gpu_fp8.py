@@ -165,3 +165,26 @@ def test_rmsnorm_inside_the_quantize(m):
     got = y.float().cpu().numpy()
     assert np.isfinite(got).all()
     assert np.abs(got - ref).max() <= 2e-2 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("m", [17, 128, 129, 256, 257, 300, 400])
+@pytest.mark.parametrize("n,k,dtype", [(128, 128, "bf16"), (384, 640, "f16"), (512, 1024, "bf16")])
+def test_block_scaled_at_tile_edges(m, n, k, dtype):
+    """Block-scaled FP8 where the kernel changes form (128-row tiles up to 128 rows, 256-row tiles of a CTA pair above) and
+    where tiles are partial (a last pair with one CTA's rows only, half a column tile, one K block).  Against the same codes
+    and scales in 64 bits: the output's rounding (2^-8 bf16, 2^-11 f16, relative) and the f32 sums over K (2^-24 K)."""
+    from emmy_b200 import ops
+    from oracle import activations as oact
+
+    rng = np.random.default_rng(m + n)
+    w = rng.standard_normal((n // 128, 128, k // 128, 128)).astype(np.float32) * 0.02
+    s = (np.abs(w).max(axis=(1, 3)) / 448).astype(np.float32)
+    bits = fm.e4m3_encode(w / s[:, None, :, None])
+    x = synth.activations(m, k, dtype, seed=m)
+    xq, xs = oact.fp8_dynamic_per_group(x)
+    ref = (fm.e4m3_decode(xq).astype(np.float64) * np.repeat(xs, 128, axis=1)) @ (
+        fm.e4m3_decode(bits).astype(np.float64) * s[:, None, :, None]).reshape(n, k).T
+    xd = dev(x).bfloat16() if dtype == "bf16" else dev(x).half()
+    y = ops.fp8_block_linear(xd, dev(bits.reshape(n, k)), dev(s)).float().cpu().numpy()
+    u = 2.0**-8 if dtype == "bf16" else 2.0**-11
+    assert (np.abs(y - ref) <= u * np.abs(ref) + 2.0**-24 * k * np.abs(ref).max()).all()

@@ -295,7 +295,7 @@ def wl_w4(device, rank, fmt, k, n, m):
         for w in ws:
             ops.w4a16_linear(x, w, workspace=wsp, out=y)
 
-    kernel = GEMV_KERNEL if m == 1 else ("w4a16_stream_kernel" if m <= 24 else "w4a16_gemm_tc_kernel<__half>")
+    kernel = GEMV_KERNEL if m == 1 else ("w4a16_stream_kernel" if m <= 16 else "w4a16_tmem_pair_kernel" if m > 256 else "w4a16_tmem_kernel")
     return dict(step=step, calls=copies, kernels_per_call=1, alg_bytes=algorithmic_bytes(k, n, m, fmt == "gptq"), flops=2.0 * m * k * n, peak_mult=1.0,
                 h2d=[(x, x_host)], d2h=[(y_host, y)], status=lambda: ops.w4a16_status(wsp, m, n), kernel=kernel,
                 dtype="int4 weights, f16 activations, f32 accumulate")
@@ -478,7 +478,7 @@ def wl_moe(device, rank, world, t, exchange="peer"):
         hit = int(torch.unique(om.moe_route(logits, topk)[0]).numel())  # distinct experts this batch touches
     else:
         hit = local_e  # every local expert is hit by the ranks' tokens at these sizes
-    tier = "moe_decode_kernel (two phases)" if (world == 1 and t <= 16) else "moe_stream_kernel (grouped)" if t * topk <= 8 * e else "w4a16_gemm_tc_kernel (grouped)"
+    tier = "moe_decode_kernel (two phases)" if (world == 1 and t <= 16) else "w4a16_gemm_tc_kernel (grouped)" if world > 1 and t * topk > 8 * e else "moe_stream_kernel (grouped)" if world > 1 or t * topk < 3 * e else "w4a16_tmem_kernel (grouped)"
     return dict(step=step, calls=layers, kernels_per_call=2 if t <= 16 else 6 if t * topk <= 8 * e else 8, alg_bytes=hit * MOE_EXPERT_BYTES + t * (2 * hidden * 2 + e * 4),
                 flops=float(t) * topk * (2.0 * hidden * 2 * inter + 2.0 * inter * hidden), peak_mult=1.0,
                 h2d=[(x, x_host)], d2h=[(y_host, y)], status=status, capture=capture, parity=parity if world > 1 else None,

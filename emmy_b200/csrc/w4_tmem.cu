@@ -213,10 +213,16 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                 prefetch();  // refills the slot just read
                 slot += 2 * kItemBytes;
                 if (slot == my_ring + D * 2 * kItemBytes) slot = my_ring;
-                if (!first && !__all_sync(0xFFFFFFFFu, wait_asleep(empty + 8 * stage, phase))) {
-                    if (lane == 0) atomicExch(a.status, 4);
-                    broken = true;
-                    break;
+                if (!first) {
+                    if (!GROUPED && !waited) {
+                        asm volatile("griddepcontrol.wait;" ::: "memory");  // bounded waits count from the moment x exists
+                        waited = true;
+                    }
+                    if (!__all_sync(0xFFFFFFFFu, wait_asleep(empty + 8 * stage, phase))) {
+                        if (lane == 0) atomicExch(a.status, 4);
+                        broken = true;
+                        break;
+                    }
                 }
                 tc::fence_after_sync();
                 if constexpr (PROMOTE) {
@@ -270,7 +276,8 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
     } else if (PROMOTE && warp < kDW + 4) {
         // ---- promotion: sums[r] += scale * accumulator, then the epilogue
         int seq = 0;
-        bool broken = false, waited = false;
+        bool broken = false;
+        if constexpr (!GROUPED) asm volatile("griddepcontrol.wait;" ::: "memory");  // as the dequant warps: waits, and y in use until then
         const uint32_t t_row = tmem_base + (static_cast<uint32_t>(32 * q) << 16);
         for (int u = blockIdx.x; u < units && !broken; u += gridDim.x) {
             int col, row0, rows, item0, n_items, expert;
@@ -298,10 +305,6 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(acc_empty + 8 * b);
-            }
-            if (!GROUPED && !waited) {
-                asm volatile("griddepcontrol.wait;" ::: "memory");
-                waited = true;
             }
 #pragma unroll
             for (int c = 0; c < NB; c += 16) {
@@ -340,6 +343,7 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
         }
     } else {
         if (tc::elect_one()) {
+            if constexpr (!GROUPED) asm volatile("griddepcontrol.wait;" ::: "memory");  // as the dequant warps
             int seq = 0, n_unit = 0;
             bool broken = false;
             for (int u = blockIdx.x; u < units && !broken; u += gridDim.x, ++n_unit) {

@@ -158,10 +158,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 prefetch();  // refills the slot just read
                 slot += 2 * kItemBytes;
                 if (slot == my_ring + kDepth * 2 * kItemBytes) slot = my_ring;
-                if (!first && !__all_sync(0xFFFFFFFFu, wait_asleep(my_empty, phase))) {
-                    if (lane == 0) atomicExch(a.status, 4);
-                    broken = true;
-                    break;
+                if (!first) {
+                    if (!waited) {
+                        asm volatile("griddepcontrol.wait;" ::: "memory");  // bounded waits count from the moment x exists
+                        waited = true;
+                    }
+                    if (!__all_sync(0xFFFFFFFFu, wait_asleep(my_empty, phase))) {
+                        if (lane == 0) atomicExch(a.status, 4);
+                        broken = true;
+                        break;
+                    }
                 }
                 first = false;
                 phase ^= 1;
@@ -230,6 +236,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
     } else if (rank == 0) {
         if (tc::elect_one()) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");  // as the dequant warps
             int seq = 0, n_unit = 0;
             bool broken = false;
             for (int u = cluster; u < units && !broken; u += clusters, ++n_unit) {

@@ -471,3 +471,35 @@ def test_gate_up_rows_and_widths_at_kernel_edges(m, k, inter, dtype):
     ref = ol.w4a16_gate_up_swiglu(x, qw, qz, sc, 128, "gptq", dtype)
     # two projections, the activation and the product are rounded (and gate enters twice): three times the linear's bound
     assert np.abs(h - ref).max() <= 3 * EDGE_TOL[dtype] * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("m,n", [(20, 256), (64, 256), (300, 9488)])
+def test_linear_behind_a_kernel_that_takes_a_second(m, n):
+    """The tensor-path kernels are resident while the kernel before them still runs, and that kernel may take longer than
+    their own bounded waits allow (about 0.2 s): those count only from its end.  Here it is the peer-memory sum, whose peer
+    never answers: it gives up after about a second and says so in its own state."""
+    import ctypes as C
+
+    from emmy_b200 import ops
+
+    k, lib, dt = 1024, ops.L.load(), torch.float16
+    qw, qz, sc = synth.awq_linear(k, n, seed=m)
+    w = ops.w4_repack(dev(qw), dev(qz), dev(sc), 128, "awq")
+    x = act(synth.activations(m, k, "f16", seed=m), "f16")
+    ws = torch.zeros(lib.eq_w4a16_workspace_bytes(m, n, k) + 256, dtype=torch.uint8, device="cuda")
+    want, y = ops.w4a16_linear(x, w, workspace=ws).clone(), torch.zeros(m, n, dtype=dt, device="cuda")
+    cap = 2048
+    recv = [torch.zeros(lib.eq_peer_allreduce_recv_bytes(2, cap), dtype=torch.uint8, device="cuda") for _ in range(2)]
+    flags = [torch.zeros(lib.eq_peer_allreduce_flag_bytes(2, cap), dtype=torch.uint8, device="cuda") for _ in range(2)]
+    peers = ops.L.ArPeers()
+    peers.world, peers.rank, peers.cap, peers.max_blocks = 2, 0, cap, 1
+    for r in range(2):
+        peers.recv[r], peers.flags[r] = recv[r].data_ptr(), flags[r].data_ptr()
+    part, total = torch.ones(cap, dtype=dt, device="cuda"), torch.empty(cap, dtype=dt, device="cuda")
+    state = torch.zeros(256, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    ops.L.check(lib.eq_peer_allreduce(C.byref(peers), ops._ptr(part), cap, ops.L.EQ_F16, ops._ptr(total), ops._ptr(state), ops._stream()))
+    ops.w4a16_linear(x, w, workspace=ws, out=y)
+    ops.w4a16_status(ws, m, n)
+    assert int(state[:4].view(torch.int32)) == 70  # it did run into its limit
+    assert torch.equal(y, want)

@@ -98,7 +98,8 @@ __global__ void __launch_bounds__(BlkCfg<BN>::kThreads, 1)
         if (tc::elect_one()) {
             tc::tma_prefetch_desc(&map_a);
             tc::tma_prefetch_desc(&map_b);
-            for (int kb = 0; kb < k_blocks; ++kb) {
+            int kb = 0;
+            for (; kb < k_blocks; ++kb) {
                 const int s = kb % kStages;
                 if (kb >= kStages && !tc::mbar_wait(tc::smem_u32(empty + s), ((kb / kStages) - 1) & 1)) {
                     atomicExch(status, 1);
@@ -116,11 +117,16 @@ __global__ void __launch_bounds__(BlkCfg<BN>::kThreads, 1)
                     tc::tma_load_2d(tc::smem_u32(tiles_b + s * kTileB), &map_b, kb * kBK, n0, bar);
                 }
             }
+            // where a wait ran out nobody else has waited for these: no CTA ends with a copy under way into its shared memory
+            // (a pair's even CTA waits for both)
+            if (rank == 0)
+                for (int i = kb < kStages ? 0 : kb - kStages; i < kb; ++i) tc::mbar_wait(tc::smem_u32(full + i % kStages), (i / kStages) & 1);
         }
     } else if (warp == 1) {
         if (rank == 0 && tc::elect_one()) {
             constexpr uint32_t idesc = tc::instr_desc(0, 0, kPair ? 2 * kBM : kBM, kBN);
-            for (int kb = 0; kb < k_blocks; ++kb) {
+            int kb = 0;
+            for (; kb < k_blocks; ++kb) {
                 const int s = kb % kStages, buf = kb % kBufs, use = kb / kBufs;
                 // the accumulator's previous block has been read out
                 if (use > 0 && !tc::mbar_wait(tc::smem_u32(acc_free + buf), (use - 1) & 1)) {
@@ -149,6 +155,8 @@ __global__ void __launch_bounds__(BlkCfg<BN>::kThreads, 1)
                     tc::mma_commit(tc::smem_u32(acc_full + buf));
                 }
             }
+            // nor does TMEM go back with an MMA under way
+            if (kb > 0) tc::mbar_wait(tc::smem_u32(acc_full + (kb - 1) % kBufs), ((kb - 1) / kBufs) & 1);
         }
     } else {
         const int quarter = warp & 3;         // TMEM lanes 32 quarter .. + 31

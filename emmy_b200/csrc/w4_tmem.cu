@@ -273,6 +273,7 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                 if (lane == 0) tc::mbar_arrive(acc_empty);
             }
         }
+        cp_wait<0>();  // (left with copies under way only where a wait ran out)
     } else if (PROMOTE && warp < kDW + 4) {
         // ---- promotion: sums[r] += scale * accumulator, then the epilogue
         int seq = 0;
@@ -340,6 +341,8 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                             tc::tma_load_2d(dst + half * (NB * 128) + bx * (Cfg::kBoxRows * 128), &map_x, (item0 + it) * 128 + half * kGK, row0 + bx * Cfg::kBoxRows, bar);
                 }
             }
+            // where a wait ran out nobody else has waited for these: the CTA does not end with a copy under way into its shared memory
+            for (int i = seq < S ? 0 : seq - S; i < seq; ++i) wait_asleep(full_b + 8 * (i % S), (i / S) & 1);
         }
     } else {
         if (tc::elect_one()) {
@@ -370,8 +373,13 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                     tc::mma_commit(empty + 8 * stage);
                     if (PROMOTE) tc::mma_commit(acc_full + 8 * b);
                 }
-                if (broken) atomicExch(a.status, 2);
                 if (!PROMOTE) tc::mma_commit(acc_full);
+                if (broken) {
+                    atomicExch(a.status, 2);
+                    // the columns are freed below: not with an MMA under way
+                    if (!PROMOTE) wait_asleep(acc_full, n_unit & 1);
+                    if (PROMOTE && seq > 0) wait_asleep(acc_full + 8 * ((seq - 1) & 1), ((seq - 1) >> 1) & 1);
+                }
             }
         }
     }

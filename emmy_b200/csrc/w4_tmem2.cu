@@ -206,6 +206,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             __syncwarp();
             if (lane == 0) tc::arrive_pair(lead_acc_empty);
         }
+        cp_wait<0>();  // (left with copies under way only where a wait ran out)
     } else if (warp == kWarps - 2) {
         if (tc::elect_one()) {
             tc::tma_prefetch_desc(&map_x);
@@ -233,6 +234,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                                              lead_full_b + 8 * stage);
                 }
             }
+            // where a wait ran out nobody else has waited for these: the pair does not end with a copy under way into either CTA's
+            // rows (the even CTA's barriers count both)
+            if (rank == 0)
+                for (int i = seq < kStagesB ? 0 : seq - kStagesB; i < seq; ++i) wait_asleep(full_b + 8 * (i % kStagesB), (i / kStagesB) & 1);
         }
     } else if (rank == 0) {
         if (tc::elect_one()) {
@@ -259,8 +264,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     tc::commit_pair(empty_a + 8 * sa);
                     tc::commit_pair(empty_b + 8 * sb);
                 }
-                if (broken) atomicExch(a.status, 2);
                 tc::commit_pair(acc_full);
+                if (broken) {
+                    atomicExch(a.status, 2);
+                    wait_asleep(acc_full, n_unit & 1);  // the columns are freed below: not with an MMA under way
+                }
             }
         }
     }

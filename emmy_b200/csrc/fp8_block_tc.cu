@@ -10,9 +10,8 @@
 // core works on the next block.  (The reference spells the same arithmetic as a per-group activation round trip in front
 // of a block-dequantized weight, emmy/compiler/loader/quant.py:1655-1717.)
 //
-//   warp 0      TMA producer: 128 rows x 128 bytes of A and 128 channels x 128 bytes of B, six 32 KB stages
-//   warp 1      MMA issuer: per K block 4 x tcgen05.mma (256 x 256 x 32 over a CTA pair, issued by its even CTA; 128 x 128 x
-//               32 up to 128 rows), commit -> stage free, commit -> accumulator full
+//   warp 0      TMA producer: A tile 128 rows x 128 bytes, B tile 256 channels x 128 bytes, four 48 KB stages
+//   warp 1      MMA issuer: per K block 4 x tcgen05.mma 128 x 256 x 32, commit -> stage free, commit -> accumulator full
 //   warps 2..9  promotion and store: quartet q owns columns [128 q, 128 q + 128) = one weight scale block; a thread owns
 //               one row and keeps its 128 sums in registers; after reading a block's accumulator it hands it back
 // Every wait is bounded and reports through the status word.
@@ -25,19 +24,19 @@ namespace {
 constexpr int kBM = 128, kBK = 128;
 constexpr int kTileA = kBM * kBK;
 
-// BN = 256: two weight scale blocks per CTA, eight promotion warps, six 32 KB stages, all of TMEM.  BN = 128 (calls of
+// BN = 256: two weight scale blocks per CTA, eight promotion warps, four 48 KB stages, all of TMEM.  BN = 128 (calls of
 // at most 128 rows, where the grid is one row of CTAs): twice as many CTAs stream the weight, six 32 KB stages.
 //
-// BN = 256 runs on CTA pairs (cta_group::2, one MMA of 256 rows x 256 columns over both CTAs): each CTA brings its own 128
-// rows and half of the weight tile, 32 KB a K block instead of a lone CTA's 48 (8.8 TB/s through L2 at K=5120 N=17408 M=2048).
-// With the block's factor loaded ahead and the accumulator read in overlapped pieces: M=300 61.0 -> 58.8 us, M=2048 237 -> 228,
-// M=8192 875 -> 850.  A K block still takes about 1100 cycles against 256 of MMA: the promotion bounds the kernel (128 adds
-// and 16 KB of TMEM reads per warp and block).
+// The promotion bounds the kernel: a K block takes about 950 cycles against 512 of MMA (128 x 256 x 128 products at 8192 a
+// clock), for 128 adds and 16 KB of TMEM reads per warp and block.  So a block's factor is loaded one block ahead, off the
+// path behind the wait: K=5120 N=17408, 300 rows 62.8 -> 56.0 us, 2048 rows 237 -> 210, 8192 rows 878 -> 797.
+// Measured on top of that and dropped: reading the accumulator in pieces of 16 columns, one under way while the other is
+// added (it spills; 2048 rows 226), and CTA pairs (cta_group::2, half of the weight tile per CTA: 2048 rows 227 with those
+// pieces, and an odd number of row tiles leaves half a pair idle: K=5120 N=12288, 300 rows, one wave 37.0, two waves 57.9).
 template <int BN>
 struct BlkCfg {
-    static constexpr bool kPair = BN == 256;
-    static constexpr int kTileB = (kPair ? BN / 2 : BN) * kBK;
-    static constexpr int kStages = 6;
+    static constexpr int kTileB = BN * kBK;
+    static constexpr int kStages = BN == 256 ? 4 : 6;
     static constexpr int kQuartets = BN / 128;
     static constexpr int kThreads = 64 + 128 * kQuartets;
     static constexpr size_t kSmem = static_cast<size_t>(kStages) * (kTileA + kTileB) + 1024 + 256;
@@ -63,10 +62,8 @@ __global__ void __launch_bounds__(BlkCfg<BN>::kThreads, 1)
     uint64_t* acc_full = bars + 2 * kStages;  // [kBufs] MMA -> promotion warps
     uint64_t* acc_free = acc_full + kBufs;    // [kBufs] promotion warps -> MMA (one arrival per warp)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + kBufs);
-    constexpr bool kPair = Cfg::kPair;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = kPair ? tc::cluster_rank() : 0;
     // row tiles run fastest: the CTAs that share a weight tile are co-resident and the weight comes from DRAM once
     const int n0 = blockIdx.y * kBN, m0 = blockIdx.x * kBM;
     const int k_blocks = K / kBK;
@@ -78,19 +75,13 @@ __global__ void __launch_bounds__(BlkCfg<BN>::kThreads, 1)
         }
         for (int b = 0; b < kBufs; ++b) {
             tc::mbar_init(tc::smem_u32(acc_full + b), 1);
-            tc::mbar_init(tc::smem_u32(acc_free + b), 4 * Cfg::kQuartets * (kPair ? 2 : 1));
+            tc::mbar_init(tc::smem_u32(acc_free + b), 4 * Cfg::kQuartets);
         }
         tc::mbar_fence_init();
     }
-    if (warp == 1) {
-        if constexpr (kPair)
-            tc::tmem_alloc_pair(tc::smem_u32(tmem_slot), kTmemCols);
-        else
-            tc::tmem_alloc(tc::smem_u32(tmem_slot), kTmemCols);
-    }
+    if (warp == 1) tc::tmem_alloc(tc::smem_u32(tmem_slot), kTmemCols);
     tc::fence_before_sync();
     __syncthreads();
-    if constexpr (kPair) tc::cluster_sync();  // the peer's barriers exist from here on
     tc::fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
@@ -106,25 +97,16 @@ __global__ void __launch_bounds__(BlkCfg<BN>::kThreads, 1)
                     break;
                 }
                 const uint32_t bar = tc::smem_u32(full + s);
-                if constexpr (kPair) {  // both CTAs' copies complete on the even CTA's barrier
-                    if (rank == 0) tc::mbar_expect_tx(bar, 2 * (kTileA + kTileB));
-                    const uint32_t lead = tc::map_to_rank(bar, 0);
-                    tc::tma_load_2d_pair(tc::smem_u32(tiles_a + s * kTileA), &map_a, kb * kBK, m0, lead);
-                    tc::tma_load_2d_pair(tc::smem_u32(tiles_b + s * kTileB), &map_b, kb * kBK, n0 + static_cast<int>(rank) * (kBN / 2), lead);
-                } else {
-                    tc::mbar_expect_tx(bar, kTileA + kTileB);
-                    tc::tma_load_2d(tc::smem_u32(tiles_a + s * kTileA), &map_a, kb * kBK, m0, bar);
-                    tc::tma_load_2d(tc::smem_u32(tiles_b + s * kTileB), &map_b, kb * kBK, n0, bar);
-                }
+                tc::mbar_expect_tx(bar, kTileA + kTileB);
+                tc::tma_load_2d(tc::smem_u32(tiles_a + s * kTileA), &map_a, kb * kBK, m0, bar);
+                tc::tma_load_2d(tc::smem_u32(tiles_b + s * kTileB), &map_b, kb * kBK, n0, bar);
             }
-            // where a wait ran out nobody else has waited for these: no CTA ends with a copy under way into its shared memory
-            // (a pair's even CTA waits for both)
-            if (rank == 0)
-                for (int i = kb < kStages ? 0 : kb - kStages; i < kb; ++i) tc::mbar_wait(tc::smem_u32(full + i % kStages), (i / kStages) & 1);
+            // where a wait ran out nobody else has waited for these: the CTA does not end with a copy under way into its shared memory
+            for (int i = kb < kStages ? 0 : kb - kStages; i < kb; ++i) tc::mbar_wait(tc::smem_u32(full + i % kStages), (i / kStages) & 1);
         }
     } else if (warp == 1) {
-        if (rank == 0 && tc::elect_one()) {
-            constexpr uint32_t idesc = tc::instr_desc(0, 0, kPair ? 2 * kBM : kBM, kBN);
+        if (tc::elect_one()) {
+            constexpr uint32_t idesc = tc::instr_desc(0, 0, kBM, kBN);
             int kb = 0;
             for (; kb < k_blocks; ++kb) {
                 const int s = kb % kStages, buf = kb % kBufs, use = kb / kBufs;
@@ -140,20 +122,11 @@ __global__ void __launch_bounds__(BlkCfg<BN>::kThreads, 1)
                 tc::fence_after_sync();
                 const uint32_t a_addr = tc::smem_u32(tiles_a + s * kTileA), b_addr = tc::smem_u32(tiles_b + s * kTileB);
 #pragma unroll
-                for (int ks = 0; ks < kBK / 32; ++ks) {  // every K block starts a fresh sum
-                    const uint64_t da = tc::smem_desc_k_sw128(a_addr + ks * 32), db = tc::smem_desc_k_sw128(b_addr + ks * 32);
-                    if constexpr (kPair)
-                        tc::mma_f8f6f4_pair(tmem_base + buf * kBN, da, db, idesc, ks > 0);
-                    else
-                        tc::mma_f8f6f4(tmem_base + buf * kBN, da, db, idesc, ks > 0);
-                }
-                if constexpr (kPair) {
-                    tc::commit_pair(tc::smem_u32(empty + s));
-                    tc::commit_pair(tc::smem_u32(acc_full + buf));
-                } else {
-                    tc::mma_commit(tc::smem_u32(empty + s));
-                    tc::mma_commit(tc::smem_u32(acc_full + buf));
-                }
+                for (int ks = 0; ks < kBK / 32; ++ks)
+                    tc::mma_f8f6f4(tmem_base + buf * kBN, tc::smem_desc_k_sw128(a_addr + ks * 32), tc::smem_desc_k_sw128(b_addr + ks * 32), idesc,
+                                   ks > 0);  // every K block starts a fresh sum
+                tc::mma_commit(tc::smem_u32(empty + s));
+                tc::mma_commit(tc::smem_u32(acc_full + buf));
             }
             // nor does TMEM go back with an MMA under way
             if (kb > 0) tc::mbar_wait(tc::smem_u32(acc_full + (kb - 1) % kBufs), ((kb - 1) / kBufs) & 1);
@@ -185,24 +158,18 @@ __global__ void __launch_bounds__(BlkCfg<BN>::kThreads, 1)
             }
             tc::fence_after_sync();
             const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * kBN + q * 128;
-            uint32_t r[2][16];  // one piece is read while the other is added
-            tc::tmem_ld_32x16(t_row, r[0]);
 #pragma unroll
-            for (int c = 0; c < 128; c += 16) {
+            for (int c = 0; c < 128; c += 32) {
+                uint32_t r[32];
+                tc::tmem_ld_32x32(t_row + c, r);
                 tc::tmem_ld_wait();
-                if (c + 16 < 128) tc::tmem_ld_32x16(t_row + c + 16, r[(c / 16 + 1) & 1]);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) sum[c + i] = fmaf(__uint_as_float(r[(c / 16) & 1][i]), f, sum[c + i]);
+                for (int i = 0; i < 32; ++i) sum[c + i] = fmaf(__uint_as_float(r[i]), f, sum[c + i]);
             }
             // this warp is done with the accumulator
             tc::fence_before_sync();
             __syncwarp();
-            if (lane == 0) {
-                if constexpr (kPair)
-                    tc::arrive_pair(tc::map_to_rank(tc::smem_u32(acc_free + buf), 0));
-                else
-                    tc::mbar_arrive(tc::smem_u32(acc_free + buf));
-            }
+            if (lane == 0) tc::mbar_arrive(tc::smem_u32(acc_free + buf));
         }
         if (ok && m < M && cols_live) {
             OutT* dst = y + static_cast<size_t>(m) * N + n0 + q * 128;
@@ -221,13 +188,9 @@ __global__ void __launch_bounds__(BlkCfg<BN>::kThreads, 1)
     __syncwarp();
     tc::fence_before_sync();
     __syncthreads();
-    if constexpr (kPair) tc::cluster_sync();  // neither CTA leaves while the other may still signal it or read its tiles
     if (warp == 1) {
         tc::fence_after_sync();
-        if constexpr (kPair)
-            tc::tmem_dealloc_pair(tmem_base, kTmemCols);
-        else
-            tc::tmem_dealloc(tmem_base, kTmemCols);
+        tc::tmem_dealloc(tmem_base, kTmemCols);
     }
 }
 
@@ -400,23 +363,13 @@ int launch(const uint8_t* qx, const float* sx, const uint8_t* w, const float* sw
     CUtensorMap map_a, map_b;
     int st = make_tensor_map_2d(&map_a, qx, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K, K, kBM, kBK, CU_TENSOR_MAP_SWIZZLE_128B);
     if (st != EQ_OK) return st;
-    st = make_tensor_map_2d(&map_b, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, Cfg::kTileB / kBK, kBK, CU_TENSOR_MAP_SWIZZLE_128B);
+    st = make_tensor_map_2d(&map_b, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, BN, kBK, CU_TENSOR_MAP_SWIZZLE_128B);
     if (st != EQ_OK) return st;
     auto kernel = fp8_block_tc_kernel<OutT, BN>;
     EQ_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmem)));
-    constexpr unsigned kCluster = Cfg::kPair ? 2 : 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(ceil_div(M, kBM * kCluster)) * kCluster, static_cast<unsigned>(ceil_div(N, BN)));
-    cfg.blockDim = dim3(Cfg::kThreads);
-    cfg.dynamicSmemBytes = Cfg::kSmem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kCluster;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = Cfg::kPair ? 1 : 0;
-    EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, sx, sw, y, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), status));
+    dim3 grid(static_cast<unsigned>(ceil_div(M, kBM)), static_cast<unsigned>(ceil_div(N, BN)));
+    kernel<<<grid, Cfg::kThreads, Cfg::kSmem, stream>>>(map_a, map_b, sx, sw, y, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), status);
+    EQ_LAUNCH_OK("fp8_block_tc_kernel");
     return EQ_OK;
 }
 

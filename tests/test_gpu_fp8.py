@@ -170,8 +170,8 @@ def test_rmsnorm_inside_the_quantize(m):
 @pytest.mark.parametrize("m", [17, 128, 129, 256, 257, 300, 400])
 @pytest.mark.parametrize("n,k,dtype", [(128, 128, "bf16"), (384, 640, "f16"), (512, 1024, "bf16")])
 def test_block_scaled_at_tile_edges(m, n, k, dtype):
-    """Block-scaled FP8 where the kernel changes form (128-row tiles up to 128 rows, 256-row tiles of a CTA pair above) and
-    where tiles are partial (a last pair with one CTA's rows only, half a column tile, one K block).  Against the same codes
+    """Block-scaled FP8 where the kernel changes form (128-column tiles up to 128 rows, 256-column tiles above) and where
+    tiles are partial (a last row tile of one row, an odd number of row tiles, half a column tile, one K block).  Against the same codes
     and scales in 64 bits: the output's rounding (2^-8 bf16, 2^-11 f16, relative) and the f32 sums over K (2^-24 K)."""
     from emmy_b200 import ops
     from oracle import activations as oact

@@ -295,7 +295,7 @@ def wl_w4(device, rank, fmt, k, n, m):
         for w in ws:
             ops.w4a16_linear(x, w, workspace=wsp, out=y)
 
-    kernel = GEMV_KERNEL if m == 1 else ("w4a16_stream_kernel" if m <= 16 else "w4a16_tmem_pair_kernel" if m > 256 else "w4a16_tmem_kernel")
+    kernel = GEMV_KERNEL if m == 1 else ops.L.load().eq_w4a16_kernel(m, n, k, 0).decode()
     return dict(step=step, calls=copies, kernels_per_call=1, alg_bytes=algorithmic_bytes(k, n, m, fmt == "gptq"), flops=2.0 * m * k * n, peak_mult=1.0,
                 h2d=[(x, x_host)], d2h=[(y_host, y)], status=lambda: ops.w4a16_status(wsp, m, n), kernel=kernel,
                 dtype="int4 weights, f16 activations, f32 accumulate")

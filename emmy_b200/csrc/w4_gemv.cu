@@ -160,9 +160,10 @@ extern "C" int eq_w4a16_linear(const void* wq, int scale_dtype, const int32_t* p
     int* counters = reinterpret_cast<int*>(partial + w4_front_rows(M) * N);
 
     const bool streamable = static_cast<long long>(N / 16) * (K / 128) < (1LL << 30);
-    if (M >= kTmemMinRows && M <= kTmemPromoteRows && !perm && aligned(y, 16))
+    const W4Route route = w4_route(M, N, perm != nullptr);
+    if (M > 16 && route == W4Route::kPromoted && aligned(y, 16))
         return w4_tmem_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, y, M, N, K, act_dtype, false, true, status, stream);
-    if (M > 16 && M <= 24 && streamable) {
+    if (M > 16 && M <= kTmemPromoteRows && streamable) {
         // with a row permutation (or an unaligned output) up to 24 rows still stream the weight through the mma.sync tile
         // (x gathered and staged in shared memory, K sliced where it does not fit); the tensor path would need a gather
         // pass first.  A shape that does not fit falls through to it
@@ -206,6 +207,16 @@ extern "C" int eq_w4a16_linear(const void* wq, int scale_dtype, const int32_t* p
         if (st != EQ_OK) return st;
     }
     return EQ_OK;
+}
+
+extern "C" const char* eq_w4a16_kernel(int64_t M, int64_t N, int64_t K, int has_perm) {
+    if (M <= 1) return "w4a16_gemv1_kernel";
+    if (M <= 16) return "w4a16_stream_kernel";
+    switch (w4_route(M, N, has_perm != 0)) {
+        case W4Route::kStream: return "w4a16_stream_kernel";
+        case W4Route::kPairs: return "w4a16_tmem_pair_kernel";
+        default: return "w4a16_tmem_kernel";
+    }
 }
 
 // ---- gate / up + SwiGLU in one call ---------------------------------------------------------------------------
@@ -283,13 +294,12 @@ extern "C" int eq_w4a16_gate_up_swiglu(const void* wq, int scale_dtype, const in
                workspace_bytes);
     const size_t inner = gu_align(eq_w4a16_workspace_bytes(M, 2 * I, K));
     unsigned char* extra = static_cast<unsigned char*>(workspace) + inner;
-    if (M >= kTmemMinRows && M <= kTmemPromoteRows && !perm && aligned(h, 16))
-        return w4_tmem_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, h, M, 2 * I, K, act_dtype, true, true,
-                                    static_cast<int*>(workspace), stream);
     if (M > 16 && !perm && aligned(h, 16)) {
         int* status = static_cast<int*>(workspace);  // sticky until eq_w4a16_status reports it, as in eq_w4a16_linear
-        if (!w4_tmem_pairs(M, 2 * I))
-            return w4_tmem_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, h, M, 2 * I, K, act_dtype, true, false, status, stream);
+        const W4Route route = w4_route(M, 2 * I, false);
+        if (route != W4Route::kPairs)
+            return w4_tmem_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, h, M, 2 * I, K, act_dtype, true, route == W4Route::kPromoted,
+                                        status, stream);
         return w4_tmem_pair_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, h, M, 2 * I, K, act_dtype, true, status, stream);
     }
     // few rows, scattered act-order groups or an unaligned output: the [gate | up] linear, then the activation

@@ -11,13 +11,21 @@ namespace eq {
 // 42.8 against 44.5; 20 rows: 25.3 | 12.3 (K=N=4096) | MLP 73.2 against 17.1 | 9.6 | 49.4).  17 to 24 rows keep that
 // kernel's arithmetic, integers in the MMA and scales applied to f32 sums (PROMOTE); above, the weights are scaled before
 // the MMA, which at 28 rows costs 15.8 against 20.0 promoted.
-constexpr int64_t kTmemMinRows = 17, kTmemPromoteRows = 24;
+constexpr int64_t kTmemPromoteRows = 24;
 
 // More than 256 rows whose 256 x 256 tiles occupy at least half of the CTA pairs run on pairs (w4_tmem2.cu), the rest on
 // one-CTA tiles of at most 128 rows with K slices where CTAs would idle.  Measured, one-CTA against pairs: MLP 256 rows
 // 94.9 : 101.3, 300 rows (both linears) 158 : 134, 1024 rows 317 : 277, 4096 rows 1266 : 1076; K=N=4096, 512 rows (32 tiles)
 // 21.2 : 28.0, K=14336 N=4096, 300 rows (32 tiles) 48 against 50; K=4096 N=1792, 2048 rows (56 tiles) 33.5 : 28.8.
 inline bool w4_tmem_pairs(int64_t M, int64_t N) { return M > 256 && ceil_div(N, 256) * ceil_div(M, 256) * 4 >= sm_count(); }
+
+// The kernel of a call of more than 16 rows with a 16-byte aligned output.  perm: the weight carries a row permutation (the
+// stream kernel gathers x while it stages it, the tensor path needs a pass of its own).  swiglu: N is the width of [gate | up].
+enum class W4Route { kStream, kPromoted, kScaled, kPairs };
+inline W4Route w4_route(int64_t M, int64_t N, bool perm) {
+    if (M <= kTmemPromoteRows) return perm ? W4Route::kStream : W4Route::kPromoted;
+    return w4_tmem_pairs(M, N) ? W4Route::kPairs : W4Route::kScaled;
+}
 
 struct W4TmemArgs {
     const unsigned char* wq;   // repacked weight (of expert 0)

@@ -98,6 +98,7 @@ def load() -> C.CDLL:
         "eq_w4_unpack_repacked": (i, [p, i64, i64, p, p]),
         "eq_w4a16_workspace_bytes": (sz, [i64, i64, i64]),
         "eq_w4a16_linear": (i, [p, i, p, i64, i64, i64, p, i64, i, p, p, sz, p]),
+        "eq_w4a16_kernel": (C.c_char_p, [i64, i64, i64, i]),
         "eq_w4a16_status": (i, [p, i64, i64, p]),
         "eq_w4a16_gate_up_workspace_bytes": (sz, [i64, i64, i64]),
         "eq_w4a16_gate_up_swiglu": (i, [p, i, p, i64, i64, i64, p, i64, i, p, p, sz, p]),

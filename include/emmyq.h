@@ -140,6 +140,9 @@ size_t eq_w4a16_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int eq_w4a16_linear(const void* wq, int scale_dtype, const int32_t* perm, int64_t K, int64_t N, int64_t G,
                     const void* x, int64_t M, int act_dtype, void* y, void* workspace, size_t workspace_bytes,
                     void* stream);
+/* Name of the kernel that eq_w4a16_linear runs for these extents on the current device, with a 16-byte aligned output and
+ * activations that fit (for labels and tests; above 16 rows eq_w4a16_gate_up_swiglu goes by the same with N = 2 I). */
+const char* eq_w4a16_kernel(int64_t M, int64_t N, int64_t K, int has_perm);
 /* The device-side waits (the tensor-path kernel's pipeline barriers, the GEMV's wait for a neighbour's sixteen words)
  * are bounded; one that runs out sets the status word at the start of the workspace and the affected outputs are
  * undefined.  The linear itself never clears the word: it stays set over later calls until this call, which

@@ -88,3 +88,14 @@ def test_ops_refuse_cpu_tensors():
 
     with pytest.raises(RuntimeError, match="no CPU path"):
         ops.unpack_int4(torch.zeros(2, 2, dtype=torch.int32), "awq")
+
+
+def test_kernel_names_by_extent(eq):
+    """The dispatch of the W4A16 linear, as it stands on 148 SMs (what a machine without a GPU assumes)."""
+    name = lambda m, n, k=4096, perm=0: eq.eq_w4a16_kernel(m, n, k, perm).decode()
+    assert name(1, 4096) == "w4a16_gemv1_kernel"
+    assert name(16, 4096) == "w4a16_stream_kernel"
+    assert name(20, 4096) == "w4a16_tmem_kernel" and name(20, 4096, perm=1) == "w4a16_stream_kernel"
+    assert name(25, 4096, perm=1) == "w4a16_tmem_kernel"
+    assert name(257, 28672) == name(257, 28672, perm=1) == "w4a16_tmem_pair_kernel"
+    assert name(4096, 16) == "w4a16_tmem_kernel"  # too narrow to occupy the pairs

@@ -433,9 +433,9 @@ def test_gate_up_swiglu_in_one_call(m):
             ops.w4a16_gate_up_swiglu(act(x, "bf16"), w, workspace=ws, out=odd)
 
 
-# Rows and widths at which the weights-in-TMEM kernels change form: promoted sums (17-24 rows) against scaled weights, one
-# accumulator width to the next, one-CTA against pair tiles, K slices that meet in a cluster (narrow widths) and whole-K
-# tiles, partial column tiles of 128 and 256, one item of K.
+# Rows and widths at which the one-CTA weights-in-TMEM kernel changes form: promoted sums (17-24 rows) against scaled
+# weights, one accumulator width to the next, K slices that meet in a cluster (narrow widths) and whole-K tiles, partial
+# column tiles of 128, one item of K.
 # Tolerance, against f32 sums over weights rounded once to the activation dtype (unit roundoff u: 2^-8 bf16, 2^-11 f16): the
 # output's rounding u, the scale's rounding to the activation dtype u (the same for a whole group) and the products'
 # rounding on either side, which averages over K: below 4 u of the largest output.
@@ -471,6 +471,62 @@ def test_gate_up_rows_and_widths_at_kernel_edges(m, k, inter, dtype):
     ref = ol.w4a16_gate_up_swiglu(x, qw, qz, sc, 128, "gptq", dtype)
     # two projections, the activation and the product are rounded (and gate enters twice): three times the linear's bound
     assert np.abs(h - ref).max() <= 3 * EDGE_TOL[dtype] * np.abs(ref).max()
+
+
+# CTA pairs: a last column tile of 256 with 16 channels (the even CTA's) or 144 (16 of them the odd one's), one item of K (three
+# of the four dequant groups have none) and five, a last row tile of a few rows, scales in the other 16-bit type.
+def _awq(k, n, dtype, cvt, seed):
+    scale = {"f16": "bf16", "bf16": "f16"}[dtype] if cvt else dtype
+    qw, qz, sc = synth.awq_linear(k, n, seed=seed, scale_dtype=np.float16 if scale == "f16" else np.float32)
+    return (qw, qz, sc), (dev(qw), dev(qz), dev(sc) if scale == "f16" else dev(sc).bfloat16())
+
+
+@pytest.mark.parametrize("m", [257, 300, 385, 513])
+@pytest.mark.parametrize("k,n,dtype,cvt", [(128, 9488, "f16", True), (640, 9616, "bf16", False), (640, 9488, "bf16", True)])
+def test_pair_tiles(m, k, n, dtype, cvt):
+    from emmy_b200 import ops
+
+    assert ops.L.load().eq_w4a16_kernel(m, n, k, 0) == b"w4a16_tmem_pair_kernel"
+    host, device = _awq(k, n, dtype, cvt, seed=m)
+    x = synth.activations(m, k, dtype, seed=m + 1)
+    ws = torch.zeros(ops.L.load().eq_w4a16_workspace_bytes(m, n, k) + 256, dtype=torch.uint8, device="cuda")
+    y = ops.w4a16_linear(act(x, dtype), ops.w4_repack(*device, 128, "awq"), workspace=ws).float().cpu().numpy()
+    ref = ol.w4a16_linear(x, *host, 128, "awq", dtype)
+    assert np.abs(y - ref).max() <= EDGE_TOL[dtype] * np.abs(ref).max()
+    assert not ws.any()
+
+
+@pytest.mark.parametrize("m", [257, 300, 513])
+@pytest.mark.parametrize("k,inter,dtype,cvt", [(128, 4752, "f16", False), (640, 4816, "bf16", True), (640, 4752, "f16", True)])
+def test_gate_up_pair_tiles(m, k, inter, dtype, cvt):
+    from emmy_b200 import ops
+
+    assert ops.L.load().eq_w4a16_kernel(m, 2 * inter, k, 0) == b"w4a16_tmem_pair_kernel"
+    parts = [_awq(k, inter, dtype, cvt, seed=m + i) for i in range(2)]
+    x = synth.activations(m, k, dtype, seed=m + 2)
+    ws = torch.zeros(ops.L.load().eq_w4a16_gate_up_workspace_bytes(m, inter, k) + 256, dtype=torch.uint8, device="cuda")
+    w = ops.w4_concat([ops.w4_repack(*p[1], 128, "awq") for p in parts])
+    h = ops.w4a16_gate_up_swiglu(act(x, dtype), w, workspace=ws).float().cpu().numpy()
+    ref = ol.w4a16_gate_up_swiglu(x, *(np.concatenate(p, axis=1) for p in zip(parts[0][0], parts[1][0])), 128, "awq", dtype)
+    assert np.abs(h - ref).max() <= 3 * EDGE_TOL[dtype] * np.abs(ref).max()
+    assert not ws.any()
+
+
+@pytest.mark.parametrize("m", [257, 400])
+def test_pair_tiles_scattered_act_order(m):
+    from emmy_b200 import ops
+
+    k, n = 256, 9488
+    qw, qz, sc, _ = synth.gptq_linear(k, n, seed=8)
+    gi = np.random.default_rng(3).permutation(np.arange(k) // 128).astype(np.int32)
+    w = ops.w4_repack(dev(qw), dev(qz), dev(sc), 128, "gptq", g_idx=dev(gi))
+    assert w.perm is not None and ops.L.load().eq_w4a16_kernel(m, n, k, 1) == b"w4a16_tmem_pair_kernel"
+    x = synth.activations(m, k, "bf16", seed=m)
+    ws = torch.zeros(ops.L.load().eq_w4a16_workspace_bytes(m, n, k) + 256, dtype=torch.uint8, device="cuda")
+    y = ops.w4a16_linear(act(x, "bf16"), w, workspace=ws).float().cpu().numpy()
+    ref = ol.w4a16_linear(x, qw, qz, sc, 128, "gptq", "bf16", gi)
+    assert np.abs(y - ref).max() <= EDGE_TOL["bf16"] * np.abs(ref).max()
+    assert not ws.any()
 
 
 @pytest.mark.parametrize("m,n", [(20, 256), (64, 256), (300, 9488)])

@@ -2,8 +2,8 @@
 //
 //   M == 1         w4a16_gemv1_kernel (w4_gemv1.cu): half-SM CTAs, equal item spans, launches overlap in pairs.
 //   2 <= M <= 16   w4a16_stream_kernel (w4_stream.cu): one fat CTA per SM streams whole column tiles, x staged in shared
-//                  memory (whole, or a K slice per CTA with the slices meeting in the workspace).  Weights with a row
-//                  permutation stay with it up to 24 rows where a slice of x fits.
+//                  memory (whole, or a K slice per CTA with the slices meeting in the workspace).  Small matrices, and
+//                  weights with a row permutation, stay with it up to 24 rows where a slice of x fits.
 //   M > 16         w4a16_tmem_kernel (w4_tmem.cu) and, for larger calls, w4a16_tmem_pair_kernel (w4_tmem2.cu): tcgen05 with
 //                  the weights expanded into tensor memory.
 //   w4a16_tile_kernel below: M > 16 with an output that is not 16-byte aligned (in 64-row blocks), and decode
@@ -160,17 +160,19 @@ extern "C" int eq_w4a16_linear(const void* wq, int scale_dtype, const int32_t* p
     int* counters = reinterpret_cast<int*>(partial + w4_front_rows(M) * N);
 
     const bool streamable = static_cast<long long>(N / 16) * (K / 128) < (1LL << 30);
-    const W4Route route = w4_route(M, N, perm != nullptr);
+    const W4Route route = w4_route(M, N, K, perm != nullptr, false);
     if (M > 16 && route == W4Route::kPromoted && aligned(y, 16))
         return w4_tmem_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, y, M, N, K, act_dtype, false, true, status, stream);
     if (M > 16 && M <= kTmemPromoteRows && streamable) {
-        // with a row permutation (or an unaligned output) up to 24 rows still stream the weight through the mma.sync tile
-        // (x gathered and staged in shared memory, K sliced where it does not fit); the tensor path would need a gather
-        // pass first.  A shape that does not fit falls through to it
+        // small matrices, and weights with a row permutation (the tensor path would need a gather pass first) or an
+        // unaligned output, still stream the weight through the mma.sync tile (x staged in shared memory, gathered on the
+        // way, K sliced where it does not fit).  A shape that does not fit falls through to the tensor path
         W4Params p = w4_params(wq, perm, x, y, partial, counters, K, N, static_cast<int>(M), scale_dtype);
         bool fits = false;
         const int st = w4_stream_launch(p, act_dtype, stream, &fits);
         if (st != EQ_OK || fits) return st;
+        if (!perm && aligned(y, 16))
+            return w4_tmem_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, y, M, N, K, act_dtype, false, true, status, stream);
     }
     if (M > 16 && aligned(y, 16)) {
         // prefill-shaped: the tcgen05 kernel; its bounded waits report through the status word.  No call clears the
@@ -212,7 +214,7 @@ extern "C" int eq_w4a16_linear(const void* wq, int scale_dtype, const int32_t* p
 extern "C" const char* eq_w4a16_kernel(int64_t M, int64_t N, int64_t K, int has_perm) {
     if (M <= 1) return "w4a16_gemv1_kernel";
     if (M <= 16) return "w4a16_stream_kernel";
-    switch (w4_route(M, N, has_perm != 0)) {
+    switch (w4_route(M, N, K, has_perm != 0, false)) {
         case W4Route::kStream: return "w4a16_stream_kernel";
         case W4Route::kPairs: return "w4a16_tmem_pair_kernel";
         default: return "w4a16_tmem_kernel";
@@ -296,7 +298,7 @@ extern "C" int eq_w4a16_gate_up_swiglu(const void* wq, int scale_dtype, const in
     unsigned char* extra = static_cast<unsigned char*>(workspace) + inner;
     if (M > 16 && !perm && aligned(h, 16)) {
         int* status = static_cast<int*>(workspace);  // sticky until eq_w4a16_status reports it, as in eq_w4a16_linear
-        const W4Route route = w4_route(M, 2 * I, false);
+        const W4Route route = w4_route(M, 2 * I, K, false, true);
         if (route != W4Route::kPairs)
             return w4_tmem_dense_launch(static_cast<const unsigned char*>(wq), scale_dtype, x, h, M, 2 * I, K, act_dtype, true, route == W4Route::kPromoted,
                                         status, stream);

@@ -13,6 +13,21 @@ namespace eq {
 // the MMA, which at 28 rows costs 15.8 against 20.0 promoted.
 constexpr int64_t kTmemPromoteRows = 24;
 
+// 17 to 24 rows of a small matrix stay with w4_stream.cu: with little of K per slice the tensor path's prologue, hand-overs
+// and cluster meeting are not hidden, and one wave of the stream's column tiles (16 channels a CTA) takes no longer for a
+// wider matrix.  So the limits on K are: short whatever the width (K=512 N=4096, 17 rows: 3.8 us streamed against 4.9);
+// about 1280 for one or one and a half waves (1280 x 2048: 4.3 | 5.2, 24 rows 4.8 | 5.3; 1280 x 512: even; 1792 x 2048, 24
+// rows: 6.0 | 5.7); above that a limit on K x rows, the staged x, and on K x N x rows (1792 x 4096, 17 rows 6.1 | 7.2, 24 rows
+// 6.7 | 7.4; 2560 x 4096, 17 rows 7.3 | 7.9, 24 rows even; 3072 x 4096: 8.3 | 8.1; 1792 x 8192, 24 rows even).  A long K with a
+// handful of column tiles leaves the tensor path fewer CTAs than the stream's K slices (14336 x 256: 7.3 | 9.1; 5120 x 256:
+// 5.2 | 5.5; 5120 x 512: 6.3 | 5.7).
+inline bool w4_few_rows_stream(int64_t M, int64_t N, int64_t K) {
+    if (K <= 768) return N <= 8192;
+    if (K >= 5120) return K >= 20 * N;
+    if (N <= 3072) return N >= 1024 && K <= 1280;
+    return N <= 8192 && K * M <= 43520 && K * N * M <= int64_t(1) << 28;
+}
+
 // More than 256 rows whose 256 x 256 tiles occupy at least half of the CTA pairs run on pairs (w4_tmem2.cu), the rest on
 // one-CTA tiles of at most 128 rows with K slices where CTAs would idle.  Measured, one-CTA against pairs: MLP 256 rows
 // 94.9 : 101.3, 300 rows (both linears) 158 : 134, 1024 rows 317 : 277, 4096 rows 1266 : 1076; K=N=4096, 512 rows (32 tiles)
@@ -22,8 +37,8 @@ inline bool w4_tmem_pairs(int64_t M, int64_t N) { return M > 256 && ceil_div(N, 
 // The kernel of a call of more than 16 rows with a 16-byte aligned output.  perm: the weight carries a row permutation (the
 // stream kernel gathers x while it stages it, the tensor path needs a pass of its own).  swiglu: N is the width of [gate | up].
 enum class W4Route { kStream, kPromoted, kScaled, kPairs };
-inline W4Route w4_route(int64_t M, int64_t N, bool perm) {
-    if (M <= kTmemPromoteRows) return perm ? W4Route::kStream : W4Route::kPromoted;
+inline W4Route w4_route(int64_t M, int64_t N, int64_t K, bool perm, bool swiglu) {
+    if (M <= kTmemPromoteRows) return perm || (!swiglu && w4_few_rows_stream(M, N, K)) ? W4Route::kStream : W4Route::kPromoted;
     return w4_tmem_pairs(M, N) ? W4Route::kPairs : W4Route::kScaled;
 }
 

@@ -134,14 +134,14 @@ size_t eq_w4a16_workspace_bytes(int64_t M, int64_t N, int64_t K);
  * (emmy/compiler/loader/quant.py:1235-1435) and evaluates eagerly as dequantize + F.linear
  * (emmy/compiler/trace/huggingface.py:2877-2920).  perm is NULL unless eq_w4_repack asked for it.
  * Needs K % 128 == 0, N % 16 == 0, G % 128 == 0 (or G = -1); x and wq 16-byte aligned.
- * M <= 16 (24 with a row permutation) runs the bandwidth kernels (any K: shapes whose activations do not fit shared
+ * M <= 16 (24 with a row permutation or a small matrix) runs the bandwidth kernels (any K: shapes whose activations do not fit shared
  * memory run a split-K form through the workspace, and from 17 rows on such shapes take the next path); above that the
  * tcgen05 kernels, which expand the weights into tensor memory. */
 int eq_w4a16_linear(const void* wq, int scale_dtype, const int32_t* perm, int64_t K, int64_t N, int64_t G,
                     const void* x, int64_t M, int act_dtype, void* y, void* workspace, size_t workspace_bytes,
                     void* stream);
 /* Name of the kernel that eq_w4a16_linear runs for these extents on the current device, with a 16-byte aligned output and
- * activations that fit (for labels and tests; above 16 rows eq_w4a16_gate_up_swiglu goes by the same with N = 2 I). */
+ * activations that fit (for labels and tests; above 24 rows eq_w4a16_gate_up_swiglu goes by the same with N = 2 I). */
 const char* eq_w4a16_kernel(int64_t M, int64_t N, int64_t K, int has_perm);
 /* The device-side waits (the tensor-path kernel's pipeline barriers, the GEMV's wait for a neighbour's sixteen words)
  * are bounded; one that runs out sets the status word at the start of the workspace and the affected outputs are

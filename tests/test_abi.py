@@ -98,4 +98,9 @@ def test_kernel_names_by_extent(eq):
     assert name(20, 4096) == "w4a16_tmem_kernel" and name(20, 4096, perm=1) == "w4a16_stream_kernel"
     assert name(25, 4096, perm=1) == "w4a16_tmem_kernel"
     assert name(257, 28672) == name(257, 28672, perm=1) == "w4a16_tmem_pair_kernel"
+    # 17 to 24 rows of small matrices
+    for m, n, k, kernel in [(17, 4096, 512, "stream"), (24, 8192, 768, "stream"), (17, 9488, 768, "tmem"), (17, 2048, 1280, "stream"), (17, 512, 1280, "tmem"),
+                            (24, 2048, 1792, "tmem"), (17, 4096, 2560, "stream"), (24, 4096, 2560, "tmem"), (24, 4096, 1792, "stream"), (17, 4096, 3072, "tmem"),
+                            (20, 256, 14336, "stream"), (20, 512, 5120, "tmem"), (25, 4096, 512, "tmem")]:
+        assert name(m, n, k) == f"w4a16_{kernel}_kernel", (m, n, k)
     assert name(4096, 16) == "w4a16_tmem_kernel"  # too narrow to occupy the pairs

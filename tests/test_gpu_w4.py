@@ -473,6 +473,25 @@ def test_gate_up_rows_and_widths_at_kernel_edges(m, k, inter, dtype):
     assert np.abs(h - ref).max() <= 3 * EDGE_TOL[dtype] * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("m", [17, 24])
+@pytest.mark.parametrize("k,n,dtype", [(128, 9488, "f16"), (640, 8208, "bf16"), (768, 528, "bf16"), (1280, 1040, "f16"), (1408, 1040, "bf16"), (5120, 256, "f16"),
+                                       (1792, 4112, "f16"), (2560, 4112, "bf16"), (128, 16, "bf16")])
+def test_few_rows_on_both_sides_of_the_small_matrix_rule(m, k, n, dtype):
+    """17 to 24 rows: the mma.sync stream and the promoted tensor form take neighbouring sizes; both keep integers in the MMA
+    and scales on f32 sums, so the bound is the output's rounding and the oracle's rounded weights (EDGE_TOL)."""
+    from emmy_b200 import ops
+
+    qw, qz, sc = synth.awq_linear(k, n, seed=m)
+    x = synth.activations(m, k, dtype, seed=m + 1)
+    ws = torch.zeros(ops.L.load().eq_w4a16_workspace_bytes(m, n, k) + 256, dtype=torch.uint8, device="cuda")
+    w = ops.w4_repack(dev(qw), dev(qz), dev(sc), 128, "awq")
+    for _ in range(2):
+        y = ops.w4a16_linear(act(x, dtype), w, workspace=ws)
+    ref = ol.w4a16_linear(x, qw, qz, sc, 128, "awq", dtype)
+    assert np.abs(y.float().cpu().numpy() - ref).max() <= EDGE_TOL[dtype] * np.abs(ref).max()
+    assert not ws.any()
+
+
 # CTA pairs: a last column tile of 256 with 16 channels (the even CTA's) or 144 (16 of them the odd one's), one item of K (three
 # of the four dequant groups have none) and five, a last row tile of a few rows, scales in the other 16-bit type.
 def _awq(k, n, dtype, cvt, seed):

@@ -473,9 +473,14 @@ int launch_dense(W4TmemArgs a, const void* x, int scale_dtype, cudaStream_t stre
     // K slices (a cluster's CTAs, eight at most) where the tiles leave CTA slots idle; at least two items a slice.  A cluster
     // lives in one GPC, so not every slot can be filled: with 288 of the 296 asked for (K=14336 N=4096, 300 rows, clusters of
     // three) a second wave ran and the call took 72 us.
+    // A meeting costs about what three items do, so a short K is not cut, nor one into two slices only (promoted: 9 items)
+    // (plain linears; us, cut against whole.  32 rows: 512 x 14336 6.7 : 4.2, 1024 x 14336 8.1 : 6.7, 1536 x 14336 10.4 : 9.3;
+    // 128 rows: 512 x 14336 9.6 : 7.2; 20 rows: 512 x 14336 6.4 : 4.7, 1280 x 14336 even).  The SwiGLU epilogue gains from being
+    // shared out: K=768, 20 rows, cutting is 4 to 39 % faster.
     int splits = (slots - slots / 8) / tiles;
     if (splits > items / 2) splits = items / 2;
     if (splits > 8) splits = 8;
+    if (!SWIGLU && (items <= 6 || (splits == 2 && items < (PROMOTE ? 9 : 14)))) splits = 1;
     if (splits < 1) splits = 1;
     a.splits = splits;
     a.units = tiles * splits;
@@ -489,7 +494,9 @@ int dense_typed(const W4TmemArgs& a, const void* x, int scale_dtype, bool swiglu
         if (a.M <= 16) return swiglu ? launch_dense<ActT, 16, true, true>(a, x, scale_dtype, stream) : launch_dense<ActT, 16, true, false>(a, x, scale_dtype, stream);
         return swiglu ? launch_dense<ActT, 32, true, true>(a, x, scale_dtype, stream) : launch_dense<ActT, 32, true, false>(a, x, scale_dtype, stream);
     }
-    if (a.M <= 64) return swiglu ? launch_dense<ActT, 64, false, true>(a, x, scale_dtype, stream) : launch_dense<ActT, 64, false, false>(a, x, scale_dtype, stream);
+    // 65 to 128 rows of a short K, where the epilogue is the larger part, run as two row tiles of 64 on twice as many CTAs (128
+    // rows: 512 x 4096 5.8 -> 4.3 us, 512 x 14336 7.4 -> 5.8, 896 x 11136 9.2 -> 6.7; at K=1024 the second expansion costs more)
+    if (a.M <= 64 || (!swiglu && a.M <= 128 && a.K <= 896)) return swiglu ? launch_dense<ActT, 64, false, true>(a, x, scale_dtype, stream) : launch_dense<ActT, 64, false, false>(a, x, scale_dtype, stream);
     return swiglu ? launch_dense<ActT, 128, false, true>(a, x, scale_dtype, stream) : launch_dense<ActT, 128, false, false>(a, x, scale_dtype, stream);
 }
 

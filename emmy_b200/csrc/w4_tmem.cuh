@@ -22,7 +22,7 @@ constexpr int64_t kTmemPromoteRows = 24;
 // handful of column tiles leaves the tensor path fewer CTAs than the stream's K slices (14336 x 256: 7.3 | 9.1; 5120 x 256:
 // 5.2 | 5.5; 5120 x 512: 6.3 | 5.7).
 inline bool w4_few_rows_stream(int64_t M, int64_t N, int64_t K) {
-    if (K <= 768) return N <= 8192;
+    if (K <= 896) return N <= 8192;
     if (K >= 5120) return K >= 20 * N;
     if (N <= 3072) return N >= 1024 && K <= 1280;
     return N <= 8192 && K * M <= 43520 && K * N * M <= int64_t(1) << 28;

@@ -492,6 +492,21 @@ def test_few_rows_on_both_sides_of_the_small_matrix_rule(m, k, n, dtype):
     assert not ws.any()
 
 
+@pytest.mark.parametrize("m", [25, 64, 65, 128, 129])
+@pytest.mark.parametrize("k,n,dtype", [(768, 9488, "f16"), (896, 272, "bf16"), (1024, 272, "f16"), (1024, 11152, "bf16"), (1792, 11152, "f16")])
+def test_short_k(m, k, n, dtype):
+    """Where K is cut into slices and where not, and 65 to 128 rows as two tiles of 64 (a last one of one row) or one of 128."""
+    from emmy_b200 import ops
+
+    qw, qz, sc = synth.awq_linear(k, n, seed=m)
+    x = synth.activations(m, k, dtype, seed=m + 1)
+    ws = torch.zeros(ops.L.load().eq_w4a16_workspace_bytes(m, n, k) + 256, dtype=torch.uint8, device="cuda")
+    y = ops.w4a16_linear(act(x, dtype), ops.w4_repack(dev(qw), dev(qz), dev(sc), 128, "awq"), workspace=ws).float().cpu().numpy()
+    ref = ol.w4a16_linear(x, qw, qz, sc, 128, "awq", dtype)
+    assert np.abs(y - ref).max() <= EDGE_TOL[dtype] * np.abs(ref).max()
+    assert not ws.any()
+
+
 # CTA pairs: a last column tile of 256 with 16 channels (the even CTA's) or 144 (16 of them the odd one's), one item of K (three
 # of the four dequant groups have none) and five, a last row tile of a few rows, scales in the other 16-bit type.
 def _awq(k, n, dtype, cvt, seed):

@@ -531,7 +531,7 @@ int launch_typed(const unsigned char* wq, int scale_dtype, const int32_t* perm, 
         x = gathered;
     }
     const int act = ScaleMul<ActT>::kFmt == 0 ? EQ_F16 : EQ_BF16;
-    if (!w4_tmem_pairs(M, N)) return w4_tmem_dense_launch(wq, scale_dtype, x, y, M, N, K, act, false, false, status, stream);
+    if (!w4_tmem_pairs(M, N, K)) return w4_tmem_dense_launch(wq, scale_dtype, x, y, M, N, K, act, false, false, status, stream);
     return w4_tmem_pair_dense_launch(wq, scale_dtype, x, y, M, N, K, act, false, status, stream);
 }
 

@@ -28,18 +28,23 @@ inline bool w4_few_rows_stream(int64_t M, int64_t N, int64_t K) {
     return N <= 8192 && K * M <= 43520 && K * N * M <= int64_t(1) << 28;
 }
 
-// More than 256 rows whose 256 x 256 tiles occupy at least half of the CTA pairs run on pairs (w4_tmem2.cu), the rest on
-// one-CTA tiles of at most 128 rows with K slices where CTAs would idle.  Measured, one-CTA against pairs: MLP 256 rows
-// 94.9 : 101.3, 300 rows (both linears) 158 : 134, 1024 rows 317 : 277, 4096 rows 1266 : 1076; K=N=4096, 512 rows (32 tiles)
-// 21.2 : 28.0, K=14336 N=4096, 300 rows (32 tiles) 48 against 50; K=4096 N=1792, 2048 rows (56 tiles) 33.5 : 28.8.
-inline bool w4_tmem_pairs(int64_t M, int64_t N) { return M > 256 && ceil_div(N, 256) * ceil_div(M, 256) * 4 >= sm_count(); }
+// More than 256 rows (128 from K=2048 on, where a pair's longer prologue and epilogue are hidden) whose 256 x 256 tiles occupy
+// at least half of the CTA pairs run on pairs (w4_tmem2.cu), the rest on one-CTA tiles of at most 128 rows with K slices where
+// CTAs would idle.  Measured, us, one-CTA against pairs: MLP of hidden 4096, intermediate 14336, both linears forced: 300 rows
+// 158 : 134, 1024 rows 317 : 277, 4096 rows 1266 : 1076; K=N=4096, 512 rows (32 tiles) 21.2 : 28.0, K=14336 N=4096, 300 rows
+// (32 tiles) 48 : 50; K=4096 N=1792, 2048 rows (56 tiles) 33.5 : 28.8.  [gate | up] of hidden 5120, intermediate 17408: 160
+// rows 66 : 50, 256 rows 80 : 68; linears of 136 to 256 rows, pairs over one-CTA: K=4096 N=14336 0.78 to 0.91, K=2048 N=9472
+// 1.00 to 0.93, K=1024 N=9472 1.14 to 1.10.
+inline bool w4_tmem_pairs(int64_t M, int64_t N, int64_t K) {
+    return M > (K >= 2048 ? 128 : 256) && ceil_div(N, 256) * ceil_div(M, 256) * 4 >= sm_count();
+}
 
 // The kernel of a call of more than 16 rows with a 16-byte aligned output.  perm: the weight carries a row permutation (the
 // stream kernel gathers x while it stages it, the tensor path needs a pass of its own).  swiglu: N is the width of [gate | up].
 enum class W4Route { kStream, kPromoted, kScaled, kPairs };
 inline W4Route w4_route(int64_t M, int64_t N, int64_t K, bool perm, bool swiglu) {
     if (M <= kTmemPromoteRows) return perm || (!swiglu && w4_few_rows_stream(M, N, K)) ? W4Route::kStream : W4Route::kPromoted;
-    return w4_tmem_pairs(M, N) ? W4Route::kPairs : W4Route::kScaled;
+    return w4_tmem_pairs(M, N, K) ? W4Route::kPairs : W4Route::kScaled;
 }
 
 struct W4TmemArgs {

@@ -1,4 +1,4 @@
-// W4A16 linear for prefill: the weights-in-TMEM form of w4_tmem.cu on CTA pairs (tcgen05 cta_group::2).
+// W4A16 linear for prefill (w4_tmem_pairs: when): the weights-in-TMEM form of w4_tmem.cu on CTA pairs (tcgen05 cta_group::2).
 //
 // A pair owns 256 output channels (128 TMEM lanes in each CTA) by up to NB activation rows.  Each CTA expands its own
 // channels' int4 into its own TMEM (A operand) and fetches HALF of the activation rows; the pair's MMA (256 x rows x 16,

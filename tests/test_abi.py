@@ -97,6 +97,7 @@ def test_kernel_names_by_extent(eq):
     assert name(16, 4096) == "w4a16_stream_kernel"
     assert name(20, 4096) == "w4a16_tmem_kernel" and name(20, 4096, perm=1) == "w4a16_stream_kernel"
     assert name(25, 4096, perm=1) == "w4a16_tmem_kernel"
+    assert name(128, 28672) == name(256, 28672, k=1920) == "w4a16_tmem_kernel" and name(129, 28672, k=2048) == "w4a16_tmem_pair_kernel"
     assert name(257, 28672) == name(257, 28672, perm=1) == "w4a16_tmem_pair_kernel"
     # 17 to 24 rows of small matrices
     for m, n, k, kernel in [(17, 4096, 512, "stream"), (24, 8192, 768, "stream"), (17, 9488, 768, "tmem"), (17, 2048, 1280, "stream"), (17, 512, 1280, "tmem"),

@@ -515,8 +515,8 @@ def _awq(k, n, dtype, cvt, seed):
     return (qw, qz, sc), (dev(qw), dev(qz), dev(sc) if scale == "f16" else dev(sc).bfloat16())
 
 
-@pytest.mark.parametrize("m", [257, 300, 385, 513])
-@pytest.mark.parametrize("k,n,dtype,cvt", [(128, 9488, "f16", True), (640, 9616, "bf16", False), (640, 9488, "bf16", True)])
+@pytest.mark.parametrize("m,k,n,dtype,cvt", [(m, *shape) for shape in [(128, 9488, "f16", True), (640, 9616, "bf16", False), (640, 9488, "bf16", True)] for m in (257, 300, 385, 513)]
+                         + [(129, 2048, 9488, "f16", False), (200, 2048, 9616, "bf16", True), (256, 2176, 9488, "f16", False)])
 def test_pair_tiles(m, k, n, dtype, cvt):
     from emmy_b200 import ops
 
@@ -530,8 +530,8 @@ def test_pair_tiles(m, k, n, dtype, cvt):
     assert not ws.any()
 
 
-@pytest.mark.parametrize("m", [257, 300, 513])
-@pytest.mark.parametrize("k,inter,dtype,cvt", [(128, 4752, "f16", False), (640, 4816, "bf16", True), (640, 4752, "f16", True)])
+@pytest.mark.parametrize("m,k,inter,dtype,cvt", [(m, *shape) for shape in [(128, 4752, "f16", False), (640, 4816, "bf16", True), (640, 4752, "f16", True)] for m in (257, 300, 513)]
+                         + [(129, 2048, 4752, "bf16", False), (240, 2048, 4816, "f16", False)])
 def test_gate_up_pair_tiles(m, k, inter, dtype, cvt):
     from emmy_b200 import ops
 

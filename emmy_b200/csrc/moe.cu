@@ -14,11 +14,12 @@
 //                         rows of ONE expert, its weights are that expert's slice of the stacked repacked tensor.
 //                         Rows are gathered (first GEMM) / scattered (second GEMM) through index arrays, nothing is
 //                         copied.  Body: the W4A16 tile code of w4_tile.cuh.
-//                         With three rows per expert and more the two GEMMs run on the tensor path instead (w4_tmem.cu):
-//                         rows are first copied into expert order (moe_gather_rows_kernel) so that TMA can read them, row
-//                         blocks are 16 rows up to eight rows per expert and 128 above, and SwiGLU is fused into the first
-//                         GEMM's epilogue.  (The expert-parallel layer has 256-row blocks on w4_gemm.cu, whose epilogue
-//                         stores whole lines to peers.)
+//                         With three rows per expert and more (later where experts are few and small:
+//                         tmem_rows_per_expert) the two GEMMs run on the tensor path instead (w4_tmem.cu): rows are first
+//                         copied into expert order (moe_gather_rows_kernel) so that TMA can read them, row blocks are 16
+//                         rows up to eight rows per expert and 128 above, and SwiGLU is fused into the first GEMM's
+//                         epilogue.  (The expert-parallel layer has 256-row blocks on w4_gemm.cu, whose epilogue stores
+//                         whole lines to peers.)
 //   streaming tier        fewer rows per expert (and more tokens than the decode tier takes): the plan's row blocks hold
 //                         at most eight rows and both grouped linears run through moe_stream.cu, which
 //                         streams every touched expert's weights once per block; SwiGLU is a kernel of its own between.
@@ -26,6 +27,7 @@
 //                         (emmy/compiler/trace/huggingface.py:1663-1669).
 //   moe_combine_kernel    out[t] = dtype(sum_j f32(score_j) * f32(expert_j(x_t))), picks in ascending expert order,
 //                         products and sum in f32, one rounding (gen_runner.py:235-287).
+#include <cmath>
 #include <type_traits>
 
 #include "w4_tile.cuh"
@@ -397,10 +399,17 @@ struct MoeWorkspace {
 static bool stream_rows(int64_t R, int64_t E) { return R <= 8 * E; }
 static bool tensor_path(int64_t R, int64_t E) { return !stream_rows(R, E); }
 static int block_rows_for(int64_t R, int64_t E) { return tensor_path(R, E) ? 128 : 8; }
-// From three rows per expert on the weights-in-TMEM kernel with 16-row blocks beats the streaming tier (Qwen3-30B-A3B layer,
-// 48 / 64 / 128 tokens = 3 / 4 / 8 rows an expert: 134 / 135 / 138 us against 141 / 157 / 220 under one and the same plan; at
-// 1.25 and 2 rows the two are even, 109 : 111 and 128 : 128, and the streaming tier needs no copy of the rows).
-static bool tmem_rows(int64_t R, int64_t E) { return R >= 3 * E; }
+// Rows per expert from which the weights-in-TMEM kernel with 16-row blocks beats the streaming tier.  Its units are (expert,
+// 128-column tile), a CTA each.  With many units for each CTA slot (two an SM) it pays from three rows on (128 experts, hidden
+// 2048, intermediate 768, tensor over streaming: 0.92 at 3 rows, 0.88 at 4, 0.61 at 8; at 1.25 and 2 rows the two are even and
+// the streaming tier needs no copy of the rows).  With few it pays later, since a CTA walks one long K while the streaming tier
+// spreads the columns over all SMs.  Units of the two GEMMs, 296 slots, ratios: 512 and 512 (32 experts, 2048, 1024) 1.05 at
+// 3 rows, 0.99 at 4; 448 and 256 (8, 4096, 3584) 1.04 at 5, 0.95 at 6; 192 and 256 (16, 2048, 768) 1.10 at 6, 1.00 at 7; 64 and
+// 128 (8, 2048, 512) 1.03 at 8.
+static int64_t tmem_rows_per_expert(int64_t E, int64_t H, int64_t I) {
+    const double units = std::sqrt(static_cast<double>(E * 2 * I / 128) * static_cast<double>(E * H / 128)) / (2 * sm_count());
+    return units >= 2.5 ? 3 : units >= 1.33 ? 4 : units >= 0.78 ? 6 : units >= 0.33 ? 7 : 9;
+}
 
 static MoeWorkspace carve(void* base, int64_t T, int64_t E, int64_t topk, int64_t H, int64_t I) {
     MoeWorkspace w;
@@ -449,7 +458,8 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
                            int64_t I, const void* x, const int32_t* src_row, int src_div, const int32_t* eid, int64_t R, void* out,
                            const uint64_t* row_ptr, cudaStream_t stream) {
     // few rows per expert: 16-row blocks of the weights-in-TMEM kernel where TMA can read the rows
-    const bool tensor = tensor_path(R, E), tmem = tensor || (tmem_rows(R, E) && aligned(x, 16) && aligned(out, 16));
+    const bool tensor = tensor_path(R, E), streamable = moe_stream_fits(w.max_blocks, 2 * I) && moe_stream_fits(w.max_blocks, H);
+    const bool tmem = tensor || (R >= (streamable ? tmem_rows_per_expert(E, H, I) : 3) * E && aligned(x, 16) && aligned(out, 16));
     const int br = tmem && !tensor ? 16 : block_rows_for(R, E);
     if (R <= kSmallPlanRows) {
         moe_plan_small_kernel<<<1, 1024, 3 * E * sizeof(int32_t), stream>>>(eid, src_row, src_div, static_cast<int>(R), static_cast<int>(E), br, w.offsets,
@@ -482,7 +492,7 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
         return w4_tmem_grouped_launch(static_cast<const unsigned char*>(wq_down), static_cast<size_t>(H / 16) * (I / 128) * kItemBytes, scale_dtype, w.h,
                                       out, R, H, I, act, w.blocks, w.n_blocks, br, w.dst_of, row_ptr ? w.dst_ptr : nullptr, false, w.status, stream);
     }
-    if (moe_stream_fits(w.max_blocks, 2 * I) && moe_stream_fits(w.max_blocks, H)) {
+    if (streamable) {
         const int act = std::is_same<ActT, __half>::value ? EQ_F16 : EQ_BF16;
         int st = moe_stream_launch(static_cast<const unsigned char*>(wq_gate_up), static_cast<size_t>(2 * I / 16) * (H / 128) * kItemBytes, scale_dtype,
                                    x, w.h1, w.src_of, nullptr, nullptr, w.blocks, w.n_blocks, w.max_blocks, H, 2 * I, act, stream);

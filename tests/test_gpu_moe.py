@@ -102,6 +102,33 @@ def test_moe_layer_at_row_block_edges(t, e, k, dtype):
     assert float((y - ref).abs().max()) <= TOL * float(ref.abs().max())
 
 
+# Both sides of the rule that hands few rows per expert to the tensor path (many experts from three rows on, fewer from four,
+# six, seven, very few not before more than eight), with rows spread so that experts get none, one, sixteen, seventeen and more than two blocks of sixteen.
+@pytest.mark.parametrize("e,inter,rows", [(376, 128, 2), (376, 128, 3), (200, 128, 3), (200, 128, 4), (120, 128, 5), (120, 128, 6), (56, 128, 6), (56, 128, 7), (40, 128, 8)])
+def test_moe_layer_at_the_few_rows_rule(e, inter, rows):
+    from emmy_b200 import ops_moe as om
+
+    h, k, dtype = 256, 2, torch.bfloat16
+    t = rows * e // k
+    base = make_experts(4, h, inter, seed=310)
+    idx = np.arange(e) % 4
+    ex = {key: tuple(a[idx] for a in base[key]) for key in ("gate_up", "down")}
+    w = om.moe_repack(tuple(dev(a) for a in ex["gate_up"]), tuple(dev(a) for a in ex["down"]))
+    wgu, wdn = omoe.dequant_expert_weights(base, dtype)
+    x = torch.from_numpy(synth.activations(t, h, "bf16", seed=t)).to(dtype)
+    first = torch.cat([torch.full((n,), j) for j, n in enumerate((1, 16, 17, 33))])
+    first = torch.cat([first, 4 + torch.arange(t - len(first)) % (e // 2 - 4)])  # the second half of the experts: second picks
+    second = e // 2 + torch.arange(t) % (e // 2 - 3)
+    logits = torch.zeros(t, e)
+    logits[torch.arange(t), first], logits[torch.arange(t), second] = 5.0, 4.5
+    ws = om.moe_workspace(t, w, k, torch.device("cuda"))
+    y = om.moe_forward(x.cuda(), logits.cuda(), w, k, workspace=ws).float().cpu()
+    om.moe_status(ws, t, w, k)
+    scores, ids = omoe.route_softmax_topk(logits, k)
+    ref = omoe.combine_routed(x, scores, ids, lambda ee, r: omoe.expert_ffn(x[r], wgu[ee % 4], wdn[ee % 4])).float()
+    assert float((y - ref).abs().max()) <= TOL * float(ref.abs().max())
+
+
 def test_moe_layer_qwen3_shapes_decode():
     """128 experts, top-8, hidden 2048, intermediate 768, T = 1: the decode-shaped case at full width."""
     from emmy_b200 import ops_moe as om

@@ -129,6 +129,45 @@ def test_moe_layer_at_the_few_rows_rule(e, inter, rows):
     assert float((y - ref).abs().max()) <= TOL * float(ref.abs().max())
 
 
+# The expert-parallel layer with a world of one: every step of it on one GPU (counts, layout, dispatch, grouped FFN with
+# results stored through per-row addresses, combine).  More than eight rows per expert run 256-row blocks (here experts of 1,
+# 128, 129, 256, 257 and several hundred rows), fewer the streaming tier; twice, so that flags and counters carry over.
+@pytest.mark.parametrize("t,e", [(900, 16), (37, 16)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_expert_parallel_layer_of_one_rank(t, e, dtype):
+    import ctypes as C
+
+    from emmy_b200 import ops_moe as om
+    from emmy_b200.ops import _DTYPE, _ptr, _stream
+
+    h, inter, k, lib = 384, 384, 2, om.L.load()
+    ex = make_experts(e, h, inter, seed=320)
+    w = om.moe_repack(tuple(dev(a) for a in ex["gate_up"]), tuple(dev(a) for a in ex["down"]))
+    wgu, wdn = omoe.dequant_expert_weights(ex, dtype)
+    x = torch.from_numpy(synth.activations(t, h, "bf16" if dtype == torch.bfloat16 else "f16", seed=t)).to(dtype)
+    first = torch.cat([torch.full((n,), j) for j, n in enumerate((1, 128, 129, 256, 257))])[:t]
+    first = torch.cat([first, torch.full((t - len(first),), 5)])
+    logits = torch.zeros(t, e)
+    logits[torch.arange(t), first], logits[torch.arange(t), 6 + torch.arange(t) % (e - 7)] = 5.0, 4.5
+    scores, ids = omoe.route_softmax_topk(logits, k)
+    ref = omoe.combine_routed(x, scores, ids, lambda ee, r: omoe.expert_ffn(x[r], wgu[ee], wdn[ee])).float()
+    did, dsc = om.moe_route(logits.cuda(), k)
+    cap = t * k
+    buf = lambda n: torch.zeros(n, dtype=torch.uint8, device="cuda")
+    bufs = {"recv_x": buf(cap * h * 2), "recv_meta": buf(cap * 8), "recv_count": buf(e * 4), "back": buf(cap * h * 2), "flags": buf(12)}
+    peers = om.L.EpPeers()
+    peers.world, peers.rank, peers.cap = 1, 0, cap
+    for name, b in bufs.items():
+        getattr(peers, name)[0] = b.data_ptr()
+    ws = buf(lib.eq_ep_moe_workspace_bytes(1, cap, e, h, inter))
+    dx, y = x.cuda(), torch.zeros(t, h, dtype=dtype, device="cuda")
+    for _ in range(2):
+        om.L.check(lib.eq_ep_moe_w4a16(_ptr(w.gate_up), _ptr(w.down), _DTYPE[w.scale_dtype], e, k, h, inter, 128, _ptr(dx), _ptr(did), _ptr(dsc), t, _DTYPE[dtype],
+                                       _ptr(y), C.byref(peers), 0, _ptr(ws), ws.numel(), _stream()))
+        om.L.check(lib.eq_ep_moe_status(_ptr(ws), 1, cap, e, h, inter, _stream()))
+    assert float((y.float().cpu() - ref).abs().max()) <= TOL * float(ref.abs().max())
+
+
 def test_moe_layer_qwen3_shapes_decode():
     """128 experts, top-8, hidden 2048, intermediate 768, T = 1: the decode-shaped case at full width."""
     from emmy_b200 import ops_moe as om

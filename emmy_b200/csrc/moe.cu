@@ -45,11 +45,7 @@ int moe_stream_launch(const unsigned char* wq, size_t expert_stride, int scale_d
                       int64_t N, int act_dtype, cudaStream_t stream);
 int w4_gemm_tc_grouped_launch(const unsigned char* wq, size_t expert_stride, int scale_dtype, const void* x, void* y, int64_t R, int64_t N,
                               int64_t K, int act_dtype, const RowBlock* blocks, const int32_t* n_blocks, int max_blocks,
-                              const int32_t* y_rows, const uint64_t* y_ptrs, bool swiglu, int* status, cudaStream_t stream);  // w4_gemm.cu
-
-int w4_tmem_grouped_launch(const unsigned char* wq, size_t expert_stride, int scale_dtype, const void* x, void* y, int64_t R, int64_t N, int64_t K,
-                           int act_dtype, const RowBlock* blocks, const int32_t* n_blocks, int block_rows, const int32_t* y_rows, const uint64_t* y_ptrs,
-                           bool swiglu, int* status, cudaStream_t stream);  // w4_tmem.cu
+                              const uint64_t* y_ptrs, bool swiglu, int* status, cudaStream_t stream);  // w4_gemm.cu
 
 constexpr int kMaxTopK = 16;
 constexpr int kBadExpertId = 16;  // status code of a row whose expert id is out of range (1..4 are the tensor path's waits)
@@ -197,11 +193,9 @@ __global__ void moe_plan_kernel(const int32_t* __restrict__ counts, int E, int b
 }
 
 // pos_of[r]: position of row r in expert order; src_of[pos]: the activation row that feeds position pos; dst_of[pos] = r.
-// row_ptr (optional): the address output row r goes to; dst_ptr[pos] carries it into expert order.
 __global__ void moe_scatter_kernel(const int32_t* __restrict__ eid, const int32_t* __restrict__ src_row, int R, int E,
                                    const int32_t* __restrict__ offsets, int32_t* __restrict__ cursor, int32_t* __restrict__ src_of,
-                                   int32_t* __restrict__ dst_of, const uint64_t* __restrict__ row_ptr, uint64_t* __restrict__ dst_ptr,
-                                   int src_div) {
+                                   int32_t* __restrict__ dst_of, int src_div) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= R) return;
     const int e = eid[r];
@@ -209,15 +203,13 @@ __global__ void moe_scatter_kernel(const int32_t* __restrict__ eid, const int32_
     const int pos = offsets[e] + atomicAdd(cursor + e, 1);
     src_of[pos] = src_row ? src_row[r] : (src_div > 0 ? r / src_div : r);
     dst_of[pos] = r;
-    if (row_ptr) dst_ptr[pos] = row_ptr[r];
 }
 
 // The three kernels above in one CTA, for row counts where the launches cost more than the work.
 constexpr int kSmallPlanRows = 8192;
 __global__ void moe_plan_small_kernel(const int32_t* __restrict__ eid, const int32_t* __restrict__ src_row, int src_div, int R, int E, int block_rows,
                                       int32_t* __restrict__ offsets, RowBlock* __restrict__ blocks, int32_t* __restrict__ n_blocks, int max_blocks,
-                                      int32_t* __restrict__ src_of, int32_t* __restrict__ dst_of, const uint64_t* __restrict__ row_ptr,
-                                      uint64_t* __restrict__ dst_ptr, int32_t* __restrict__ status) {
+                                      int32_t* __restrict__ src_of, int32_t* __restrict__ dst_of, int32_t* __restrict__ status) {
     extern __shared__ int32_t sh[];  // counts -> cursors [E], offsets [E], block offsets [E]
     int32_t* cnt = sh;
     int32_t* off = sh + E;
@@ -264,7 +256,6 @@ __global__ void moe_plan_small_kernel(const int32_t* __restrict__ eid, const int
         const int pos = off[e] + atomicAdd(cnt + e, 1);
         src_of[pos] = src_row ? src_row[r] : (src_div > 0 ? r / src_div : r);
         dst_of[pos] = r;
-        if (row_ptr) dst_ptr[pos] = row_ptr[r];
     }
 }
 
@@ -288,15 +279,14 @@ struct GroupedParams {
     void* y;                      // outputs (rows addressed through y_rows, or contiguous in expert order)
     const int32_t* x_rows;        // optional [R] gather index in expert order
     const int32_t* y_rows;        // optional [R] scatter index in expert order
-    const uint64_t* y_ptrs;       // optional [R] destination address of each row in expert order (overrides y / y_rows)
     const RowBlock* blocks;
     const int32_t* n_blocks;
     int K, N, scale_dtype;
 };
 
-template <typename ActT, int MT, bool ONE>
+template <typename ActT>
 __global__ void __launch_bounds__(kTileThreads) moe_expert_gemm_kernel(const GroupedParams gp) {
-    __shared__ float red[kTileWarps][MT * 8][16];
+    __shared__ float red[kTileWarps][8][16];
     __shared__ int last_flag;
     if (static_cast<int>(blockIdx.y) >= *gp.n_blocks) return;
     const RowBlock rb = gp.blocks[blockIdx.y];
@@ -318,7 +308,6 @@ __global__ void __launch_bounds__(kTileThreads) moe_expert_gemm_kernel(const Gro
         p.x = static_cast<const ActT*>(gp.x) + static_cast<size_t>(rb.row0) * gp.K;
         p.x_rows = nullptr;
     }
-    p.y_ptrs = gp.y_ptrs ? gp.y_ptrs + rb.row0 : nullptr;
     if (gp.y_rows) {
         p.y = gp.y;
         p.y_rows = gp.y_rows + rb.row0;
@@ -326,7 +315,7 @@ __global__ void __launch_bounds__(kTileThreads) moe_expert_gemm_kernel(const Gro
         p.y = static_cast<ActT*>(gp.y) + static_cast<size_t>(rb.row0) * gp.N;
         p.y_rows = nullptr;
     }
-    w4_tile<ActT, MT, ONE>(p, blockIdx.x, 0, red, &last_flag);
+    w4_tile<ActT, 1, false>(p, blockIdx.x, 0, red, &last_flag);
 }
 
 // h[r][i] = act( silu(gate[r][i]) ) * up[r][i], gate = gu[r][i], up = gu[r][I + i]; silu in f32, rounded to the
@@ -384,7 +373,6 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 struct MoeWorkspace {
     int32_t *counts, *offsets, *cursor, *n_blocks, *status, *src_of, *dst_of, *ids, *src_row;
     float* scores;
-    uint64_t* dst_ptr;
     RowBlock* blocks;
     unsigned char *h1, *h, *out;
     int max_blocks;
@@ -433,7 +421,6 @@ static MoeWorkspace carve(void* base, int64_t T, int64_t E, int64_t topk, int64_
     w.ids = reinterpret_cast<int32_t*>(take(R * 4));
     w.src_row = reinterpret_cast<int32_t*>(take(R * 4));
     w.scores = reinterpret_cast<float*>(take(R * 4));
-    w.dst_ptr = reinterpret_cast<uint64_t*>(take(R * 8));
     w.h1 = take(R * 2 * I * 2);
     w.h = take(R * I * 2);
     w.out = take(R * H * 2);
@@ -442,11 +429,9 @@ static MoeWorkspace carve(void* base, int64_t T, int64_t E, int64_t topk, int64_
 }
 
 template <typename ActT>
-static int launch_grouped(const GroupedParams& gp, int block_rows, int max_blocks, cudaStream_t stream) {
+static int launch_grouped(const GroupedParams& gp, int max_blocks, cudaStream_t stream) {  // row blocks of at most eight rows
     dim3 grid(static_cast<unsigned>(gp.N / 16), static_cast<unsigned>(max_blocks));
-    if (block_rows <= 8) moe_expert_gemm_kernel<ActT, 1, false><<<grid, kTileThreads, 0, stream>>>(gp);
-    else if (block_rows <= 16) moe_expert_gemm_kernel<ActT, 2, false><<<grid, kTileThreads, 0, stream>>>(gp);
-    else moe_expert_gemm_kernel<ActT, 8, false><<<grid, kTileThreads, 0, stream>>>(gp);
+    moe_expert_gemm_kernel<ActT><<<grid, kTileThreads, 0, stream>>>(gp);
     EQ_LAUNCH_OK("moe_expert_gemm_kernel");
     return EQ_OK;
 }
@@ -456,15 +441,14 @@ static int launch_grouped(const GroupedParams& gp, int block_rows, int max_block
 template <typename ActT>
 static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const void* wq_down, int scale_dtype, int64_t E, int64_t H,
                            int64_t I, const void* x, const int32_t* src_row, int src_div, const int32_t* eid, int64_t R, void* out,
-                           const uint64_t* row_ptr, cudaStream_t stream) {
+                           cudaStream_t stream) {
     // few rows per expert: 16-row blocks of the weights-in-TMEM kernel where TMA can read the rows
     const bool tensor = tensor_path(R, E), streamable = moe_stream_fits(w.max_blocks, 2 * I) && moe_stream_fits(w.max_blocks, H);
     const bool tmem = tensor || (R >= (streamable ? tmem_rows_per_expert(E, H, I) : 3) * E && aligned(x, 16) && aligned(out, 16));
     const int br = tmem && !tensor ? 16 : block_rows_for(R, E);
     if (R <= kSmallPlanRows) {
         moe_plan_small_kernel<<<1, 1024, 3 * E * sizeof(int32_t), stream>>>(eid, src_row, src_div, static_cast<int>(R), static_cast<int>(E), br, w.offsets,
-                                                                            w.blocks, w.n_blocks, w.max_blocks, w.src_of, w.dst_of, row_ptr, w.dst_ptr,
-                                                                            w.status);
+                                                                            w.blocks, w.n_blocks, w.max_blocks, w.src_of, w.dst_of, w.status);
         EQ_LAUNCH_OK("moe_plan_small_kernel");
     } else {
         EQ_CUDA_OK(cudaMemsetAsync(w.counts, 0, E * 4, stream));
@@ -474,7 +458,7 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
                                                                      w.max_blocks);
         EQ_LAUNCH_OK("moe_plan_kernel");
         moe_scatter_kernel<<<static_cast<unsigned>(ceil_div(R, 256)), 256, 0, stream>>>(eid, src_row, static_cast<int>(R), static_cast<int>(E), w.offsets,
-                                                                                      w.cursor, w.src_of, w.dst_of, row_ptr, w.dst_ptr, src_div);
+                                                                                      w.cursor, w.src_of, w.dst_of, src_div);
         EQ_LAUNCH_OK("moe_scatter_kernel");
     }
     if (tmem) {
@@ -487,10 +471,10 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
             static_cast<const uint4*>(x), w.src_of, w.offsets + E, row_vec, reinterpret_cast<uint4*>(w.out));
         EQ_LAUNCH_OK("moe_gather_rows_kernel");
         int st = w4_tmem_grouped_launch(static_cast<const unsigned char*>(wq_gate_up), static_cast<size_t>(2 * I / 16) * (H / 128) * kItemBytes, scale_dtype,
-                                        w.out, w.h, R, 2 * I, H, act, w.blocks, w.n_blocks, br, nullptr, nullptr, true, w.status, stream);
+                                        w.out, w.h, R, 2 * I, H, act, w.blocks, w.n_blocks, br, nullptr, true, w.status, stream);
         if (st != EQ_OK) return st;
         return w4_tmem_grouped_launch(static_cast<const unsigned char*>(wq_down), static_cast<size_t>(H / 16) * (I / 128) * kItemBytes, scale_dtype, w.h,
-                                      out, R, H, I, act, w.blocks, w.n_blocks, br, w.dst_of, row_ptr ? w.dst_ptr : nullptr, false, w.status, stream);
+                                      out, R, H, I, act, w.blocks, w.n_blocks, br, w.dst_of, false, w.status, stream);
     }
     if (streamable) {
         const int act = std::is_same<ActT, __half>::value ? EQ_F16 : EQ_BF16;
@@ -501,7 +485,7 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
                                                                                               static_cast<int>(I), reinterpret_cast<ActT*>(w.h));
         EQ_LAUNCH_OK("moe_swiglu_kernel");
         return moe_stream_launch(static_cast<const unsigned char*>(wq_down), static_cast<size_t>(H / 16) * (I / 128) * kItemBytes, scale_dtype, w.h,
-                                 out, nullptr, w.dst_of, row_ptr ? w.dst_ptr : nullptr, w.blocks, w.n_blocks, w.max_blocks, I, H, act, stream);
+                                 out, nullptr, w.dst_of, nullptr, w.blocks, w.n_blocks, w.max_blocks, I, H, act, stream);
     }
     GroupedParams g1;
     g1.wq = static_cast<const unsigned char*>(wq_gate_up);
@@ -510,13 +494,12 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
     g1.y = w.h1;
     g1.x_rows = w.src_of;
     g1.y_rows = nullptr;
-    g1.y_ptrs = nullptr;
     g1.blocks = w.blocks;
     g1.n_blocks = w.n_blocks;
     g1.K = static_cast<int>(H);
     g1.N = static_cast<int>(2 * I);
     g1.scale_dtype = scale_dtype;
-    int st = launch_grouped<ActT>(g1, br, w.max_blocks, stream);
+    int st = launch_grouped<ActT>(g1, w.max_blocks, stream);
     if (st != EQ_OK) return st;
     moe_swiglu_kernel<ActT><<<static_cast<unsigned>(ceil_div(R * I, 256)), 256, 0, stream>>>(reinterpret_cast<const ActT*>(w.h1), w.offsets + E,
                                                                                           static_cast<int>(I), reinterpret_cast<ActT*>(w.h));
@@ -528,10 +511,9 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
     g2.y = out;
     g2.x_rows = nullptr;
     g2.y_rows = w.dst_of;
-    g2.y_ptrs = row_ptr ? w.dst_ptr : nullptr;
     g2.K = static_cast<int>(I);
     g2.N = static_cast<int>(H);
-    return launch_grouped<ActT>(g2, br, w.max_blocks, stream);
+    return launch_grouped<ActT>(g2, w.max_blocks, stream);
 }
 
 
@@ -803,8 +785,8 @@ extern "C" int eq_moe_experts_w4a16(const void* wq_gate_up, const void* wq_down,
     MoeWorkspace w = carve(workspace, R, E, 1, H, I);
     EQ_CUDA_OK(cudaMemsetAsync(w.status, 0, 4, stream));
     if (act_dtype == EQ_F16)
-        return experts_forward<__half>(w, wq_gate_up, wq_down, scale_dtype, E, H, I, x, src_row, 0, expert_ids, R, out, nullptr, stream);
-    return experts_forward<__nv_bfloat16>(w, wq_gate_up, wq_down, scale_dtype, E, H, I, x, src_row, 0, expert_ids, R, out, nullptr, stream);
+        return experts_forward<__half>(w, wq_gate_up, wq_down, scale_dtype, E, H, I, x, src_row, 0, expert_ids, R, out, stream);
+    return experts_forward<__nv_bfloat16>(w, wq_gate_up, wq_down, scale_dtype, E, H, I, x, src_row, 0, expert_ids, R, out, stream);
 }
 
 extern "C" int eq_moe_combine(const void* out_rows, const float* scores, int64_t T, int64_t topk, int64_t H, int act_dtype, void* y, void* stream_) {
@@ -854,9 +836,9 @@ extern "C" int eq_moe_w4a16(const void* wq_gate_up, const void* wq_down, int sca
     st = eq_moe_route(router_logits, T, E, topk, 1, w.ids, w.scores, stream_);
     if (st != EQ_OK) return st;
     if (act_dtype == EQ_F16)
-        st = experts_forward<__half>(w, wq_gate_up, wq_down, scale_dtype, E, H, I, x, nullptr, static_cast<int>(topk), w.ids, R, w.out, nullptr, stream);
+        st = experts_forward<__half>(w, wq_gate_up, wq_down, scale_dtype, E, H, I, x, nullptr, static_cast<int>(topk), w.ids, R, w.out, stream);
     else
-        st = experts_forward<__nv_bfloat16>(w, wq_gate_up, wq_down, scale_dtype, E, H, I, x, nullptr, static_cast<int>(topk), w.ids, R, w.out, nullptr, stream);
+        st = experts_forward<__nv_bfloat16>(w, wq_gate_up, wq_down, scale_dtype, E, H, I, x, nullptr, static_cast<int>(topk), w.ids, R, w.out, stream);
     if (st != EQ_OK) return st;
     return eq_moe_combine(w.out, w.scores, T, topk, H, act_dtype, y, stream_);
 }
@@ -957,10 +939,10 @@ extern "C" int eq_ep_moe_w4a16(const void* wq_gate_up, const void* wq_down, int 
     } else {
         EQ_REQUIRE(aligned(peers->recv_x[me], 16), EQ_ERR_BAD_ALIGN, "eq_ep_moe_w4a16: the receive buffer must be 16-byte aligned");
         st = w4_gemm_tc_grouped_launch(gu, stride_gu, scale_dtype, peers->recv_x[me], w.moe.h, R, 2 * I, H, act_dtype, w.blocks, w.moe.n_blocks,
-                                       w.max_blocks, nullptr, nullptr, true, w.moe.status, stream);
+                                       w.max_blocks, nullptr, true, w.moe.status, stream);
         if (st != EQ_OK) return st;
         st = w4_gemm_tc_grouped_launch(dn, stride_dn, scale_dtype, w.moe.h, nullptr, R, H, I, act_dtype, w.blocks, w.moe.n_blocks, w.max_blocks,
-                                       nullptr, w.row_ptr, false, w.moe.status, stream);
+                                       w.row_ptr, false, w.moe.status, stream);
     }
     if (st != EQ_OK) return st;
     ep_signal_done_kernel<<<1, 32, 0, stream>>>(*peers, epoch, w.epoch);

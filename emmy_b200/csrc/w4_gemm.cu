@@ -1,10 +1,10 @@
 // Grouped W4A16 GEMM of the expert-parallel MoE layer: 256-row blocks of one expert each, weights dequantised into shared
 // memory, on the tcgen05 tensor cores; and the dense prefill entry, which picks between w4_tmem.cu and w4_tmem2.cu.
 //
-// The int4 weight never exists as a 16-bit matrix in global memory.  A CTA owns a tile of 256 activation rows by BN output
+// The int4 weight never exists as a 16-bit matrix in global memory.  A CTA owns a tile of 256 activation rows by 256 weight
 // columns and walks K in steps of 64:
 //   warp 0        TMA producer: the 64-wide slice of the x rows, 128-byte swizzle, into the stage's A tile
-//   warp 1        MMA issuer: tcgen05.mma kind::f16, 128 x BN x 16 per instruction, f32 accumulators in TMEM (one
+//   warp 1        MMA issuer: tcgen05.mma kind::f16, 128 x 256 x 16 per instruction, f32 accumulators in TMEM (one
 //                 accumulator per 128 activation rows; both read the same B tile)
 //   warps 2..     dequant producers, then the epilogue.  A producer warp reads the packed nibbles of one 16-column
 //                 weight tile straight from global memory into registers (one 16-byte load per lane and K step,
@@ -25,43 +25,22 @@
 
 namespace eq {
 
-int w4_tmem_pair_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
-                              int* status, cudaStream_t stream);  // w4_tmem2.cu
-int w4_tmem_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
-                         bool promote, int* status, cudaStream_t stream);  // w4_tmem.cu
-
 namespace {
 
 constexpr int kGK = 64;             // K per stage: 128 bytes of 16-bit elements
 constexpr int kRowBytes = 128;
 
-// HALVES: 128-row activation blocks per CTA; BN: output columns per CTA; DW: dequant (and epilogue) warps;
-// AHEAD: items (two K steps each) whose packed bytes are in a warp's registers ahead of use.
-template <int HALVES, int BN, int DW, int AHEAD>
-struct GemmCfg {
-    static constexpr int kDequantWarps = DW;
-    static constexpr int kAhead = AHEAD;
-    static constexpr int kQuartets = DW / 4;                  // epilogue warp quartets (one warp per TMEM lane quarter)
-    static constexpr int kBoxHalves = HALVES == 2 ? 2 : 1;    // 128-row halves per TMA copy of the activation tile
-    // With more dequant warps than 16-column tiles the warps also split K: group r of them takes K step r of every item.
-    static constexpr int kTiles = BN / 16;
-    static constexpr int kKSplit = DW > kTiles ? DW / kTiles : 1;
-    static constexpr int kWarpsPerStep = DW / kKSplit;          // warps that fill (and arrive on) one stage
-    static constexpr int kTilesPerWarp = kTiles / kWarpsPerStep;
-    static constexpr int kThreads = 64 + 32 * kDequantWarps;
-    static constexpr int kTileA = HALVES * 128 * kRowBytes;
-    static constexpr int kTileB = BN * kRowBytes;
-    static constexpr int kStageBytes = kTileA + kTileB;
-    static constexpr int kStages = (196608 / kStageBytes) < 4 ? (196608 / kStageBytes) : 4;
-    static constexpr size_t kSmem = static_cast<size_t>(kStages) * kStageBytes + 1024 + 256;
-    static constexpr uint32_t kAccCols = HALVES * BN;
-    static constexpr uint32_t kTmemCols = kAccCols <= 32 ? 32 : kAccCols <= 64 ? 64 : kAccCols <= 128 ? 128 : kAccCols <= 256 ? 256 : 512;
-    static_assert(kTilesPerWarp >= 1 && kTilesPerWarp * kWarpsPerStep == kTiles && (kKSplit == 1 || kKSplit == 2),
-                  "every dequant warp needs whole weight tiles, and an item has two K steps to split");
-    static_assert(DW % 4 == 0 && BN % 64 == 0, "the epilogue works in warp quartets on 32-column chunks");
-    static_assert(kAccCols <= 512, "the accumulators must fit TMEM");
-};
-
+constexpr int kHalves = 2;              // 128-row activation blocks per CTA
+constexpr int kBN = 256;                // weight columns per CTA
+constexpr int kTileA = kHalves * 128 * kRowBytes, kTileB = kBN * kRowBytes;
+constexpr int kStages = 3;
+constexpr int kDequantWarps = kBN / 16; // one 16-column weight tile each; and epilogue warps, in quartets (one warp per TMEM lane quarter)
+constexpr int kQuartets = kDequantWarps / 4;
+constexpr int kAhead = 2;               // items (two K steps each) whose packed bytes are in a warp's registers ahead of use
+constexpr int kThreads = 64 + 32 * kDequantWarps;
+constexpr size_t kSmem = static_cast<size_t>(kStages) * (kTileA + kTileB) + 1024 + 256;
+constexpr uint32_t kTmemCols = kHalves * kBN;
+static_assert(kTmemCols == 512 && kSmem <= 227 * 1024, "all of TMEM, one CTA per SM");
 
 // 8-byte read-only load that stays where it is written (issued kAhead steps before its use).
 __device__ __forceinline__ uint2 ld_pinned_v2(const void* p) {
@@ -76,38 +55,6 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
 
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-template <typename ActT>
-struct ScaleMul;
-template <>
-struct ScaleMul<__half> {
-    static constexpr uint32_t kFmt = 0;
-    // raw scale bits -> the same value twice in the activation dtype; CVT: the scales are stored in the other 16-bit type
-    template <bool CVT>
-    static __device__ __forceinline__ uint32_t pair(uint32_t raw) {
-        if constexpr (CVT) raw = __half_as_ushort(__float2half_rn(__uint_as_float(raw << 16)));
-        return __byte_perm(raw, 0, 0x1010);
-    }
-    static __device__ __forceinline__ uint32_t mul(uint32_t v, uint32_t s) {
-        uint32_t r;
-        asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(s));
-        return r;
-    }
-};
-template <>
-struct ScaleMul<__nv_bfloat16> {
-    static constexpr uint32_t kFmt = 1;
-    template <bool CVT>
-    static __device__ __forceinline__ uint32_t pair(uint32_t raw) {
-        if constexpr (CVT) raw = __bfloat16_as_ushort(__float2bfloat16_rn(__half2float(__ushort_as_half(static_cast<unsigned short>(raw)))));
-        return __byte_perm(raw, 0, 0x1010);
-    }
-    static __device__ __forceinline__ uint32_t mul(uint32_t v, uint32_t s) {
-        uint32_t r;
-        asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(s));
-        return r;
-    }
-};
-
 // xg[m][k'] = x[m][perm[k']]
 template <typename ActT>
 __global__ void gather_cols_kernel(const ActT* __restrict__ x, const int32_t* __restrict__ perm, int64_t M, int64_t K,
@@ -118,33 +65,27 @@ __global__ void gather_cols_kernel(const ActT* __restrict__ x, const int32_t* __
     xg[idx] = x[m * K + perm[k]];
 }
 
-// kGrouped: blockIdx.y walks a device-side list of row blocks, each a run of rows of ONE expert in an expert-ordered
-// activation matrix; the weight is that expert's slice of a stacked tensor and output rows may be scattered through y_rows.
-// kGroupedSwiGLU: the same, with the first 128 columns of the CTA's B tile taken from the gate half and the last 128 from the
-// up half of a [gate | up] weight, and the epilogue writing act(silu(gate)) * up
-// (emmy/compiler/trace/huggingface.py:1663-1669) into a matrix of N / 2 columns.
-enum GemmMode { kGrouped = 1, kGroupedSwiGLU = 2 };
-
+// blockIdx.y walks a device-side list of row blocks, each a run of rows of ONE expert in an expert-ordered activation matrix; the
+// weight is that expert's slice of a stacked tensor.  SWIGLU: the first 128 columns of the CTA's B tile are taken from the gate
+// half and the last 128 from the up half of a [gate | up] weight, and the epilogue writes act(silu(gate)) * up
+// (emmy/compiler/trace/huggingface.py:1663-1669) into y, a matrix of N / 2 columns.  Otherwise every row has a destination of
+// its own.
 struct GroupArgs {
     const RowBlock* blocks;
     const int32_t* n_blocks;
-    const int32_t* y_rows;   // optional: output row m goes to row y_rows[m]
-    const uint64_t* y_ptrs;  // optional: output row m starts at address y_ptrs[m] (0 = drop the row); may be a peer GPU's memory
+    const uint64_t* y_ptrs;  // output row m starts at address y_ptrs[m] (0 = drop the row); may be a peer GPU's memory
     size_t expert_stride;    // bytes between the experts' repacked weights
 };
 
-template <typename ActT, int HALVES, int BN, int DW, int AHEAD, bool CVT, int MODE>
-__global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
+template <typename ActT, bool CVT, bool SWIGLU>
+__global__ void __launch_bounds__(kThreads)
     w4a16_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const unsigned char* __restrict__ wq, ActT* __restrict__ y,
                          int N, int K, int* __restrict__ status, const GroupArgs grp) {
-    using Cfg = GemmCfg<HALVES, BN, DW, AHEAD>;
-    constexpr int kStages = Cfg::kStages;
-    constexpr int kAhead = Cfg::kAhead;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* tiles_a = smem;
-    unsigned char* tiles_b = smem + kStages * Cfg::kTileA;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Cfg::kStageBytes);
+    unsigned char* tiles_b = smem + kStages * kTileA;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * (kTileA + kTileB));
     uint64_t* full_a = bars;                  // [kStages] TMA -> MMA
     uint64_t* full_b = bars + kStages;        // [kStages] dequant warps -> MMA
     uint64_t* empty = bars + 2 * kStages;     // [kStages] MMA -> producers
@@ -152,25 +93,25 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = blockIdx.x * BN;
+    const int n0 = blockIdx.x * kBN;
     if (static_cast<int>(blockIdx.y) >= *grp.n_blocks) return;  // the whole CTA, before any barrier exists
     const RowBlock rb = grp.blocks[blockIdx.y];
     const int m0 = rb.row0, m_end = rb.row0 + rb.rows;
     wq += static_cast<size_t>(rb.expert) * grp.expert_stride;
     const int items = K / 128;
     const int k_blocks = 2 * items;
-    const int live_halves = min(HALVES, (m_end - m0 + 127) / 128);  // 128-row blocks of this tile that hold rows
+    const int live_halves = min(kHalves, (m_end - m0 + 127) / 128);  // 128-row blocks of this tile that hold rows
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             tc::mbar_init(tc::smem_u32(full_a + s), 1);
-            tc::mbar_init(tc::smem_u32(full_b + s), Cfg::kWarpsPerStep);
+            tc::mbar_init(tc::smem_u32(full_b + s), kDequantWarps);
             tc::mbar_init(tc::smem_u32(empty + s), 1);
         }
         tc::mbar_init(tc::smem_u32(acc_ready), 1);
         tc::mbar_fence_init();
     }
-    if (warp == 1) tc::tmem_alloc(tc::smem_u32(tmem_slot), Cfg::kTmemCols);
+    if (warp == 1) tc::tmem_alloc(tc::smem_u32(tmem_slot), kTmemCols);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -186,29 +127,28 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
             int stage = 0;
             uint32_t phase = 0;
             bool first = true;
-            for (int kb = 0; kb < k_blocks; ++kb) {
+            int kb = 0;
+            for (; kb < k_blocks; ++kb) {
                 if (!first && !tc::mbar_wait(empty_addr + 8 * stage, phase ^ 1)) {
                     atomicExch(status, 1);
                     break;
                 }
                 const uint32_t bar = full_a_addr + 8 * stage;
-                // one copy per TMA box (Cfg::kBoxHalves 128-row halves); halves without rows are not fetched
-                constexpr int kBoxBytes = Cfg::kBoxHalves * 128 * kRowBytes;
-                const int boxes = (live_halves + Cfg::kBoxHalves - 1) / Cfg::kBoxHalves;
-                tc::mbar_expect_tx(bar, boxes * kBoxBytes);
-                for (int bx = 0; bx < boxes; ++bx)
-                    tc::tma_load_2d(a_base + stage * Cfg::kTileA + bx * kBoxBytes, &map_x, kb * kGK, m0 + 128 * Cfg::kBoxHalves * bx, bar);
+                tc::mbar_expect_tx(bar, kTileA);
+                tc::tma_load_2d(a_base + stage * kTileA, &map_x, kb * kGK, m0, bar);
                 if (++stage == kStages) {
                     stage = 0;
                     phase ^= 1;
                     first = false;
                 }
             }
+            // where a wait ran out nobody else has waited for these: the CTA does not end with a copy under way into its shared memory
+            for (int i = kb < kStages ? 0 : kb - kStages; i < kb; ++i) tc::mbar_wait(full_a_addr + 8 * (i % kStages), (i / kStages) & 1);
         }
     } else if (warp == 1) {
         // ---- MMA issuer
         if (tc::elect_one()) {
-            constexpr uint32_t idesc = tc::instr_desc(ScaleMul<ActT>::kFmt, ScaleMul<ActT>::kFmt, 128, BN);
+            constexpr uint32_t idesc = tc::instr_desc(tm::Mul<ActT>::kFmt, tm::Mul<ActT>::kFmt, 128, kBN);
             int stage = 0;
             uint32_t phase = 0;
             for (int kb = 0; kb < k_blocks; ++kb) {
@@ -219,14 +159,14 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
                     break;
                 }
                 tc::fence_after_sync();
-                const uint32_t a_addr = a_base + stage * Cfg::kTileA, b_addr = b_base + stage * Cfg::kTileB;
+                const uint32_t a_addr = a_base + stage * kTileA, b_addr = b_base + stage * kTileB;
 #pragma unroll
                 for (int ks = 0; ks < kGK / 16; ++ks) {
                     const uint64_t db = tc::smem_desc_k_sw128(b_addr + ks * 32);
 #pragma unroll
-                    for (int hh = 0; hh < HALVES; ++hh)
+                    for (int hh = 0; hh < kHalves; ++hh)
                         if (hh < live_halves)
-                            tc::mma_f16(tmem_base + hh * BN, tc::smem_desc_k_sw128(a_addr + hh * 128 * kRowBytes + ks * 32), db, idesc, kb > 0 || ks > 0);
+                            tc::mma_f16(tmem_base + hh * kBN, tc::smem_desc_k_sw128(a_addr + hh * 128 * kRowBytes + ks * 32), db, idesc, kb > 0 || ks > 0);
                 }
                 tc::mma_commit(empty_addr + 8 * stage);
                 if (++stage == kStages) {
@@ -235,103 +175,72 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
                 }
             }
             tc::mma_commit(tc::smem_u32(acc_ready));  // on a broken pipeline too: the epilogue must not sit out its wait
+            tc::mbar_wait(tc::smem_u32(acc_ready), 0);  // nor does TMEM go back with an MMA under way
         }
     } else {
         // ---- dequant producers
         const int dw = warp - 2;
-        const int kgrp = dw / Cfg::kWarpsPerStep;  // which K step of an item this warp fills when the warps split K
         const int g = lane & 7, h = (lane >> 3) & 1, jj = lane >> 4;
         // Shared-memory byte offsets of the lane's four 16-byte chunks inside a B tile: row r = 16 tile + g (+8) is an
         // output column, chunk q = 4 jj + 2 high + h of its 128 bytes is swizzled with r & 7 = g.
-        const unsigned char* wp[Cfg::kTilesPerWarp];   // the lane's 16 bytes of K step 0 of item 0; K step 1 is 32 bytes on
-        const unsigned char* mp[Cfg::kTilesPerWarp];   // its scale / zero record of item 0
-        uint32_t off_lo[Cfg::kTilesPerWarp];
-        bool live[Cfg::kTilesPerWarp];
-#pragma unroll
-        for (int nt = 0; nt < Cfg::kTilesPerWarp; ++nt) {
-            const int tile_in_cta = (dw % Cfg::kWarpsPerStep) * Cfg::kTilesPerWarp + nt;
-            int tile = n0 / 16 + tile_in_cta;
-            if constexpr (MODE == kGroupedSwiGLU) {
-                constexpr int kHalfTiles = BN / 32;  // gate tiles of this CTA, then as many up tiles
-                const int col_tile = n0 / 32 + (tile_in_cta % kHalfTiles);
-                tile = col_tile < N / 32 ? col_tile + (tile_in_cta / kHalfTiles) * (N / 32) : N / 16;
-            }
-            live[nt] = tile < N / 16;
-            const unsigned char* rec = wq + static_cast<size_t>(live[nt] ? tile : 0) * items * kItemBytes;
-            wp[nt] = rec + h * 512 + (4 * g + jj) * 16;
-            mp[nt] = rec + 1024 + g * 8;
-            off_lo[nt] = static_cast<uint32_t>((tile_in_cta * 16 + g) * kRowBytes + (((4 * jj + h) ^ g) << 4));
+        int tile = n0 / 16 + dw;
+        if constexpr (SWIGLU) {
+            constexpr int kHalfTiles = kBN / 32;  // gate tiles of this CTA, then as many up tiles
+            const int col_tile = n0 / 32 + dw % kHalfTiles;
+            tile = col_tile < N / 32 ? col_tile + (dw / kHalfTiles) * (N / 32) : N / 16;
         }
+        const bool live = tile < N / 16;
+        const unsigned char* rec = wq + static_cast<size_t>(live ? tile : 0) * items * kItemBytes;
+        const unsigned char* wp = rec + h * 512 + (4 * g + jj) * 16;  // the lane's 16 bytes of K step 0 of item 0; K step 1 is 32 bytes on
+        const unsigned char* mp = rec + 1024 + g * 8;                 // its scale / zero record of item 0
+        const uint32_t off_lo = static_cast<uint32_t>((dw * 16 + g) * kRowBytes + (((4 * jj + h) ^ g) << 4));
         // register ring of whole items (two K steps each)
-        uint4 w0[kAhead][Cfg::kTilesPerWarp], w1[kAhead][Cfg::kTilesPerWarp];
-        uint2 meta[kAhead][Cfg::kTilesPerWarp];
-        const int my_items = items;
+        uint4 w0[kAhead], w1[kAhead];
+        uint2 meta[kAhead];
 #pragma unroll
         for (int d = 0; d < kAhead; ++d) {
-            if (d < my_items) {
-#pragma unroll
-                for (int nt = 0; nt < Cfg::kTilesPerWarp; ++nt) {
-                    if (Cfg::kKSplit == 1 || kgrp == 0) w0[d][nt] = ld_stream_v4(wp[nt] + static_cast<size_t>(d) * kItemBytes);
-                    if (Cfg::kKSplit == 1 || kgrp == 1) w1[d][nt] = ld_stream_v4(wp[nt] + static_cast<size_t>(d) * kItemBytes + 32);
-                    meta[d][nt] = ld_pinned_v2(mp[nt] + static_cast<size_t>(d) * kItemBytes);
-                }
+            if (d < items) {
+                w0[d] = ld_stream_v4(wp + static_cast<size_t>(d) * kItemBytes);
+                w1[d] = ld_stream_v4(wp + static_cast<size_t>(d) * kItemBytes + 32);
+                meta[d] = ld_pinned_v2(mp + static_cast<size_t>(d) * kItemBytes);
             }
         }
         bool broken = false, first = true;
         int stage = 0;
         uint32_t phase = 0;
-        for (int it0 = 0; it0 < my_items && !broken; it0 += kAhead) {
+        for (int it0 = 0; it0 < items && !broken; it0 += kAhead) {
 #pragma unroll
             for (int d = 0; d < kAhead; ++d) {
                 const int it = it0 + d;
-                if (it >= my_items || broken) continue;
+                if (it >= items || broken) continue;
                 // the item's constants: exact-dequant zero terms and the scale pair of columns g and g + 8
-                typename Frag<ActT>::Zero z_lo[Cfg::kTilesPerWarp], z_hi[Cfg::kTilesPerWarp];
-                uint32_t s_lo[Cfg::kTilesPerWarp], s_hi[Cfg::kTilesPerWarp];
-#pragma unroll
-                for (int nt = 0; nt < Cfg::kTilesPerWarp; ++nt) {
-                    const uint2 mt = meta[d][nt];
-                    z_lo[nt] = Frag<ActT>::zero(__byte_perm(mt.y, 0, 0x1010));
-                    z_hi[nt] = Frag<ActT>::zero(__byte_perm(mt.y, 0, 0x3232));
-                    s_lo[nt] = ScaleMul<ActT>::template pair<CVT>(mt.x & 0xFFFFu);
-                    s_hi[nt] = ScaleMul<ActT>::template pair<CVT>(mt.x >> 16);
-                }
+                const typename Frag<ActT>::Zero z_lo = Frag<ActT>::zero(__byte_perm(meta[d].y, 0, 0x1010));
+                const typename Frag<ActT>::Zero z_hi = Frag<ActT>::zero(__byte_perm(meta[d].y, 0, 0x3232));
+                const uint32_t s_lo = tm::Mul<ActT>::template pair<CVT>(meta[d].x & 0xFFFFu), s_hi = tm::Mul<ActT>::template pair<CVT>(meta[d].x >> 16);
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
                     if (broken) continue;
-                    if (Cfg::kKSplit == 2 && t != kgrp) {  // the other warp group's K step
-                        if (++stage == kStages) {
-                            stage = 0;
-                            phase ^= 1;
-                            first = false;
-                        }
-                        continue;
-                    }
                     if (!first && !tc::mbar_wait(empty_addr + 8 * stage, phase ^ 1)) {
                         if (lane == 0) atomicExch(status, 4);
                         broken = true;
                         continue;
                     }
-                    const uint32_t tile_addr = b_base + stage * Cfg::kTileB;
+                    const uint4 w = t == 0 ? w0[d] : w1[d];
+                    const uint32_t wv[4] = {w.x, w.y, w.z, w.w};
+                    uint32_t a[4][4];
 #pragma unroll
-                    for (int nt = 0; nt < Cfg::kTilesPerWarp; ++nt) {
-                        const uint4 w = t == 0 ? w0[d][nt] : w1[d][nt];
-                        const uint32_t wv[4] = {w.x, w.y, w.z, w.w};
-                        uint32_t a[4][4];
-#pragma unroll
-                        for (int wi = 0; wi < 4; ++wi) Frag<ActT>::expand(wv[wi], z_lo[nt], z_hi[nt], a[wi]);
-                        // a[wi][0]: column g, low run; [2]: column g, high run; [1] / [3]: the same for column g + 8
-                        if (live[nt]) {
-                            const uint32_t addr = tile_addr + off_lo[nt];
-                            st_shared_v4(addr, ScaleMul<ActT>::mul(a[0][0], s_lo[nt]), ScaleMul<ActT>::mul(a[1][0], s_lo[nt]),
-                                         ScaleMul<ActT>::mul(a[2][0], s_lo[nt]), ScaleMul<ActT>::mul(a[3][0], s_lo[nt]));
-                            st_shared_v4(addr ^ 32u, ScaleMul<ActT>::mul(a[0][2], s_lo[nt]), ScaleMul<ActT>::mul(a[1][2], s_lo[nt]),
-                                         ScaleMul<ActT>::mul(a[2][2], s_lo[nt]), ScaleMul<ActT>::mul(a[3][2], s_lo[nt]));
-                            st_shared_v4(addr + 8 * kRowBytes, ScaleMul<ActT>::mul(a[0][1], s_hi[nt]), ScaleMul<ActT>::mul(a[1][1], s_hi[nt]),
-                                         ScaleMul<ActT>::mul(a[2][1], s_hi[nt]), ScaleMul<ActT>::mul(a[3][1], s_hi[nt]));
-                            st_shared_v4((addr ^ 32u) + 8 * kRowBytes, ScaleMul<ActT>::mul(a[0][3], s_hi[nt]), ScaleMul<ActT>::mul(a[1][3], s_hi[nt]),
-                                         ScaleMul<ActT>::mul(a[2][3], s_hi[nt]), ScaleMul<ActT>::mul(a[3][3], s_hi[nt]));
-                        }
+                    for (int wi = 0; wi < 4; ++wi) Frag<ActT>::expand(wv[wi], z_lo, z_hi, a[wi]);
+                    // a[wi][0]: column g, low run; [2]: column g, high run; [1] / [3]: the same for column g + 8
+                    if (live) {
+                        const uint32_t addr = b_base + stage * kTileB + off_lo;
+                        auto put = [&](uint32_t at, int run, uint32_t sc) {
+                            st_shared_v4(at, tm::Mul<ActT>::mul(a[0][run], sc), tm::Mul<ActT>::mul(a[1][run], sc), tm::Mul<ActT>::mul(a[2][run], sc),
+                                         tm::Mul<ActT>::mul(a[3][run], sc));
+                        };
+                        put(addr, 0, s_lo);
+                        put(addr ^ 32u, 2, s_lo);
+                        put(addr + 8 * kRowBytes, 1, s_hi);
+                        put((addr ^ 32u) + 8 * kRowBytes, 3, s_hi);
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
@@ -342,14 +251,11 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
                         first = false;
                     }
                 }
-                if (it + kAhead < my_items) {  // refill this ring slot
-#pragma unroll
-                    for (int nt = 0; nt < Cfg::kTilesPerWarp; ++nt) {
-                        const size_t off = static_cast<size_t>(it + kAhead) * kItemBytes;
-                        if (Cfg::kKSplit == 1 || kgrp == 0) w0[d][nt] = ld_stream_v4(wp[nt] + off);
-                        if (Cfg::kKSplit == 1 || kgrp == 1) w1[d][nt] = ld_stream_v4(wp[nt] + off + 32);
-                        meta[d][nt] = ld_pinned_v2(mp[nt] + off);
-                    }
+                if (it + kAhead < items) {  // refill this ring slot
+                    const size_t off = static_cast<size_t>(it + kAhead) * kItemBytes;
+                    w0[d] = ld_stream_v4(wp + off);
+                    w1[d] = ld_stream_v4(wp + off + 32);
+                    meta[d] = ld_pinned_v2(mp + off);
                 }
             }
         }
@@ -360,31 +266,58 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
         const bool ok = __all_sync(0xFFFFFFFFu, tc::mbar_wait(tc::smem_u32(acc_ready), 0));
         if (!ok && lane == 0) atomicExch(status, 3);
         tc::fence_after_sync();
-        // Work units: (128-row half, 32-column chunk of the output), dealt round-robin to the warp quartets.  Everything
-        // that decides whether a unit runs is warp-uniform: the TMEM loads are warp-wide instructions.
-        constexpr int kChunks = (MODE == kGroupedSwiGLU ? BN / 2 : BN) / 32;
-        // Rows that leave for their own addresses (possibly on a peer GPU): a thread's 64 bytes of its own row would make
-        // every warp-wide store 32 separate 16-byte pieces, which NVLink carries at a fraction of its rate (measured: the
-        // expert-parallel down projection took 480 us against 195 us with local stores).  The warp turns its 32 rows x 64
-        // columns in shared memory (the stages are idle once the accumulator is complete) and stores 128 contiguous bytes
-        // of one row with every eight lanes.
-        bool turned = false;
-        if constexpr (MODE == kGrouped) turned = N % 64 == 0;  // scattered local rows (y_rows) gain from whole lines too
-        if (turned) {
-            constexpr int kChunks64 = BN / 64;
+        // Work units: (128-row half, chunk of columns), dealt round-robin to the warp quartets.  Everything that decides whether
+        // a unit runs is warp-uniform: the TMEM loads are warp-wide instructions.
+        if constexpr (SWIGLU) {
+            // gate columns [0, 128) and up columns [128, 256) of the accumulator -> 128 columns of the output
+            constexpr int kChunks = kBN / 64;
+            const int out_n = N / 2, out0 = n0 / 2;
+#pragma unroll 1
+            for (int unit = quartet; ok && unit < kHalves * kChunks; unit += kQuartets) {
+                const int half = unit / kChunks, c = (unit - half * kChunks) * 32;
+                if (half >= live_halves) break;
+                const int m = m0 + half * 128 + quarter * 32 + lane;
+                const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * kBN;
+                uint32_t rg[32], ru[32];
+                tc::tmem_ld_32x32(t_row + c, rg);
+                tc::tmem_ld_32x32(t_row + kBN / 2 + c, ru);
+                tc::tmem_ld_wait();
+                if (m < m_end && out0 + c < out_n) {
+                    ActT* dst = y + static_cast<size_t>(m) * out_n + out0 + c;
+                    uint32_t packed[16];
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        const float g = to_float(from_float<ActT>(__uint_as_float(rg[i])));
+                        const float u = to_float(from_float<ActT>(__uint_as_float(ru[i])));
+                        const float sg = to_float(from_float<ActT>(g / (1.f + expf(-g))));
+                        const uint32_t bits = tm::bits16<ActT>(sg * u);
+                        if (i & 1)
+                            packed[i >> 1] |= bits << 16;
+                        else
+                            packed[i >> 1] = bits;
+                    }
+                    // (a chunk is whole: the expert's intermediate size is a multiple of 128)
+#pragma unroll
+                    for (int v = 0; v < 4; ++v)
+                        reinterpret_cast<uint4*>(dst)[v] = make_uint4(packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
+                }
+            }
+        } else {
+            // Rows leave for their own addresses (possibly on a peer GPU): a thread's 64 bytes of its own row would make every
+            // warp-wide store 32 separate 16-byte pieces, which NVLink carries at a fraction of its rate (measured: the
+            // expert-parallel down projection took 480 us against 195 us with local stores).  The warp turns its 32 rows x 64
+            // columns in shared memory (the stages are idle once the accumulator is complete) and stores 128 contiguous bytes
+            // of one row with every eight lanes.
+            constexpr int kChunks = kBN / 64;
             unsigned char* stg = smem + dw * 4096;  // [32 rows][8 x 16 B], chunk v of row r at v ^ (r & 7)
             const uint32_t stg_w = tc::smem_u32(stg) + lane * 128;
 #pragma unroll 1
-            for (int unit = quartet; ok && unit < HALVES * kChunks64; unit += Cfg::kQuartets) {
-                const int half = unit / kChunks64, c = (unit - half * kChunks64) * 64;
+            for (int unit = quartet; ok && unit < kHalves * kChunks; unit += kQuartets) {
+                const int half = unit / kChunks, c = (unit - half * kChunks) * 64;
                 if (half >= live_halves) break;
-                const int row0 = m0 + half * 128 + quarter * 32;
-                const int m = row0 + lane;
-                uint64_t mine = 0ull;  // lane r holds row r's destination
-                if (m < m_end)
-                    mine = grp.y_ptrs ? grp.y_ptrs[m]
-                                      : reinterpret_cast<uint64_t>(y + (grp.y_rows ? static_cast<size_t>(grp.y_rows[m]) : static_cast<size_t>(m)) * N);
-                const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * BN;
+                const int m = m0 + half * 128 + quarter * 32 + lane;
+                const uint64_t mine = m < m_end ? grp.y_ptrs[m] : 0ull;  // lane r holds row r's destination
+                const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * kBN;
 #pragma unroll
                 for (int part = 0; part < 2; ++part) {
                     uint32_t r[32];
@@ -394,13 +327,9 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
                     for (int v = 0; v < 4; ++v) {
                         uint32_t pk[4];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const ActT o0 = from_float<ActT>(__uint_as_float(r[8 * v + 2 * i])), o1 = from_float<ActT>(__uint_as_float(r[8 * v + 2 * i + 1]));
-                            pk[i] = static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(&o0)) |
-                                    (static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(&o1)) << 16);
-                        }
-                        const uint32_t at = stg_w + (((4 * part + v) ^ (lane & 7)) << 4);
-                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+                        for (int i = 0; i < 4; ++i)
+                            pk[i] = tm::bits16<ActT>(__uint_as_float(r[8 * v + 2 * i])) | (tm::bits16<ActT>(__uint_as_float(r[8 * v + 2 * i + 1])) << 16);
+                        st_shared_v4(stg_w + (((4 * part + v) ^ (lane & 7)) << 4), pk[0], pk[1], pk[2], pk[3]);
                     }
                 }
                 __syncwarp();
@@ -416,107 +345,27 @@ __global__ void __launch_bounds__(GemmCfg<HALVES, BN, DW, AHEAD>::kThreads)
                 __syncwarp();
             }
         }
-#pragma unroll 1
-        for (int unit = quartet; ok && !turned && unit < HALVES * kChunks; unit += Cfg::kQuartets) {
-            const int half = unit / kChunks, c = (unit - half * kChunks) * 32;
-            if (half >= live_halves) break;
-            const int m = m0 + half * 128 + quarter * 32 + lane;
-            bool row_ok = m < m_end;
-            size_t out_row = static_cast<size_t>(m);
-            ActT* out_base = y;
-            if (row_ok && grp.y_ptrs) {
-                // the row's own destination: results go straight to the rank that owns the token
-                out_base = reinterpret_cast<ActT*>(grp.y_ptrs[m]);
-                out_row = 0;
-                row_ok = out_base != nullptr;
-            } else if (row_ok && grp.y_rows) {
-                out_row = static_cast<size_t>(grp.y_rows[m]);
-            }
-            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * BN;
-            if constexpr (MODE == kGroupedSwiGLU) {
-                // gate columns [0, BN/2) and up columns [BN/2, BN) of the accumulator -> BN/2 columns of the output
-                const int out_n = N / 2, out0 = n0 / 2;
-                {
-                    uint32_t rg[32], ru[32];
-                    tc::tmem_ld_32x32(t_row + c, rg);
-                    tc::tmem_ld_32x32(t_row + BN / 2 + c, ru);
-                    tc::tmem_ld_wait();
-                    if (row_ok && out0 + c < out_n) {
-                        ActT* dst = out_base + out_row * out_n + out0 + c;
-                        uint32_t packed[16];
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const float g = to_float(from_float<ActT>(__uint_as_float(rg[i])));
-                            const float u = to_float(from_float<ActT>(__uint_as_float(ru[i])));
-                            const ActT sg = from_float<ActT>(g / (1.f + expf(-g)));
-                            const ActT o = from_float<ActT>(to_float(sg) * u);
-                            const uint32_t bits = *reinterpret_cast<const uint16_t*>(&o);
-                            if (i & 1)
-                                packed[i >> 1] |= bits << 16;
-                            else
-                                packed[i >> 1] = bits;
-                        }
-                        if (out0 + c + 32 <= out_n) {
-#pragma unroll
-                            for (int v = 0; v < 4; ++v)
-                                reinterpret_cast<uint4*>(dst)[v] = make_uint4(packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                                if (out0 + c + i < out_n) reinterpret_cast<uint16_t*>(dst)[i] = static_cast<uint16_t>(packed[i >> 1] >> (16 * (i & 1)));
-                        }
-                    }
-                }
-            } else {
-                {
-                    uint32_t r[32];
-                    tc::tmem_ld_32x32(t_row + c, r);
-                    tc::tmem_ld_wait();
-                    if (row_ok && n0 + c < N) {
-                        ActT* dst = out_base + out_row * N + n0 + c;
-                        if (n0 + c + 32 <= N) {
-                            uint32_t packed[16];
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                const ActT o0 = from_float<ActT>(__uint_as_float(r[2 * i])), o1 = from_float<ActT>(__uint_as_float(r[2 * i + 1]));
-                                packed[i] = static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(&o0)) |
-                                            (static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(&o1)) << 16);
-                            }
-#pragma unroll
-                            for (int v = 0; v < 4; ++v)
-                                reinterpret_cast<uint4*>(dst)[v] = make_uint4(packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                                if (n0 + c + i < N) dst[i] = from_float<ActT>(__uint_as_float(r[i]));
-                        }
-                    }
-                }
-            }
-        }
     }
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 1) {
         tc::fence_after_sync();
-        tc::tmem_dealloc(tmem_base, Cfg::kTmemCols);
+        tc::tmem_dealloc(tmem_base, kTmemCols);
     }
 }
 
-template <typename ActT, int HALVES, int BN, int DW, int AHEAD, int MODE>
-int launch_cfg(const unsigned char* wq, int scale_dtype, const ActT* x, ActT* y, int64_t M, int64_t N, int64_t K, int* status,
-               const GroupArgs& grp, unsigned grid_y, cudaStream_t stream) {
-    using Cfg = GemmCfg<HALVES, BN, DW, AHEAD>;
+template <typename ActT, bool SWIGLU>
+int launch_grouped(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t R, int64_t N, int64_t K, int* status, const GroupArgs& grp,
+                   int max_blocks, cudaStream_t stream) {
     CUtensorMap map_x;
-    const CUtensorMapDataType elem = ScaleMul<ActT>::kFmt == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    const int box_rows = 128 * Cfg::kBoxHalves;
-    int st = make_tensor_map_2d(&map_x, x, elem, 2, M, K, K * 2, box_rows, kGK, CU_TENSOR_MAP_SWIZZLE_128B);
+    const CUtensorMapDataType elem = tm::Mul<ActT>::kFmt == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    const int st = make_tensor_map_2d(&map_x, x, elem, 2, R, K, K * 2, 128 * kHalves, kGK, CU_TENSOR_MAP_SWIZZLE_128B);
     if (st != EQ_OK) return st;
-    const bool cvt = scale_dtype != (ScaleMul<ActT>::kFmt == 0 ? EQ_F16 : EQ_BF16);
-    auto kernel = cvt ? w4a16_gemm_tc_kernel<ActT, HALVES, BN, DW, AHEAD, true, MODE> : w4a16_gemm_tc_kernel<ActT, HALVES, BN, DW, AHEAD, false, MODE>;
-    EQ_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmem)));
-    dim3 grid(static_cast<unsigned>(ceil_div(N, BN)), grid_y);
-    kernel<<<grid, Cfg::kThreads, Cfg::kSmem, stream>>>(map_x, wq, y, static_cast<int>(N), static_cast<int>(K), status, grp);
+    const bool cvt = scale_dtype != (tm::Mul<ActT>::kFmt == 0 ? EQ_F16 : EQ_BF16);
+    auto kernel = cvt ? w4a16_gemm_tc_kernel<ActT, true, SWIGLU> : w4a16_gemm_tc_kernel<ActT, false, SWIGLU>;
+    EQ_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)));
+    const dim3 grid(static_cast<unsigned>(ceil_div(N, kBN)), static_cast<unsigned>(max_blocks));
+    kernel<<<grid, kThreads, kSmem, stream>>>(map_x, wq, static_cast<ActT*>(y), static_cast<int>(N), static_cast<int>(K), status, grp);
     EQ_LAUNCH_OK("w4a16_gemm_tc_kernel");
     return EQ_OK;
 }
@@ -530,7 +379,7 @@ int launch_typed(const unsigned char* wq, int scale_dtype, const int32_t* perm, 
         EQ_LAUNCH_OK("gather_cols_kernel");
         x = gathered;
     }
-    const int act = ScaleMul<ActT>::kFmt == 0 ? EQ_F16 : EQ_BF16;
+    const int act = tm::Mul<ActT>::kFmt == 0 ? EQ_F16 : EQ_BF16;
     if (!w4_tmem_pairs(M, N, K)) return w4_tmem_dense_launch(wq, scale_dtype, x, y, M, N, K, act, false, false, status, stream);
     return w4_tmem_pair_dense_launch(wq, scale_dtype, x, y, M, N, K, act, false, status, stream);
 }
@@ -547,24 +396,19 @@ int w4_gemm_tc_launch(const unsigned char* wq, int scale_dtype, const int32_t* p
                                        N, K, static_cast<__nv_bfloat16*>(gathered), status, stream);
 }
 
-// Grouped expert GEMM on the tensor path.  x: [R][K] activations in expert order; blocks / n_blocks: device-side list of
-// row blocks of at most 256 rows; wq: E stacked repacked weights expert_stride bytes apart, each [N][K] logical.
-// swiglu: N is the width of the [gate | up] weight and y has N / 2 columns.  max_blocks bounds the grid.
+// Grouped expert GEMM of the expert-parallel layer.  x: [R][K] activations in expert order; blocks / n_blocks: device-side list
+// of row blocks of at most 256 rows; wq: E stacked repacked weights expert_stride bytes apart, each [N][K] logical, N and K
+// multiples of 128.  swiglu: N is the width of the [gate | up] weight, y has N / 2 columns and y_ptrs is not read; otherwise the
+// rows go to y_ptrs and y is not used.  max_blocks bounds the grid.
 int w4_gemm_tc_grouped_launch(const unsigned char* wq, size_t expert_stride, int scale_dtype, const void* x, void* y, int64_t R, int64_t N,
-                              int64_t K, int act_dtype, const RowBlock* blocks, const int32_t* n_blocks, int max_blocks,
-                              const int32_t* y_rows, const uint64_t* y_ptrs, bool swiglu, int* status, cudaStream_t stream) {
-    const GroupArgs grp = {blocks, n_blocks, y_rows, y_ptrs, expert_stride};
-    const unsigned gy = static_cast<unsigned>(max_blocks);
-    if (act_dtype == EQ_F16) {
-        const __half* xa = static_cast<const __half*>(x);
-        __half* ya = static_cast<__half*>(y);
-        return swiglu ? launch_cfg<__half, 2, 256, 16, 2, kGroupedSwiGLU>(wq, scale_dtype, xa, ya, R, N, K, status, grp, gy, stream)
-                      : launch_cfg<__half, 2, 256, 16, 2, kGrouped>(wq, scale_dtype, xa, ya, R, N, K, status, grp, gy, stream);
-    }
-    const __nv_bfloat16* xa = static_cast<const __nv_bfloat16*>(x);
-    __nv_bfloat16* ya = static_cast<__nv_bfloat16*>(y);
-    return swiglu ? launch_cfg<__nv_bfloat16, 2, 256, 16, 2, kGroupedSwiGLU>(wq, scale_dtype, xa, ya, R, N, K, status, grp, gy, stream)
-                  : launch_cfg<__nv_bfloat16, 2, 256, 16, 2, kGrouped>(wq, scale_dtype, xa, ya, R, N, K, status, grp, gy, stream);
+                              int64_t K, int act_dtype, const RowBlock* blocks, const int32_t* n_blocks, int max_blocks, const uint64_t* y_ptrs,
+                              bool swiglu, int* status, cudaStream_t stream) {
+    const GroupArgs grp = {blocks, n_blocks, y_ptrs, expert_stride};
+    if (act_dtype == EQ_F16)
+        return swiglu ? launch_grouped<__half, true>(wq, scale_dtype, x, y, R, N, K, status, grp, max_blocks, stream)
+                      : launch_grouped<__half, false>(wq, scale_dtype, x, y, R, N, K, status, grp, max_blocks, stream);
+    return swiglu ? launch_grouped<__nv_bfloat16, true>(wq, scale_dtype, x, y, R, N, K, status, grp, max_blocks, stream)
+                  : launch_grouped<__nv_bfloat16, false>(wq, scale_dtype, x, y, R, N, K, status, grp, max_blocks, stream);
 }
 
 }  // namespace eq

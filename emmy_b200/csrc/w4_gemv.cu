@@ -29,10 +29,6 @@ namespace eq {
 int w4_stream_launch(const W4Params& p, int act_dtype, cudaStream_t stream, bool* fits);  // w4_stream.cu
 int w4_gemv1_launch(const unsigned char* wq, int scale_dtype, const int32_t* perm, const void* x, void* y, int64_t N, int64_t K,
                     int act_dtype, uint32_t* xchg, int* status, cudaStream_t stream, bool* fits);  // w4_gemv1.cu
-int w4_tmem_pair_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
-                              int* status, cudaStream_t stream);  // w4_tmem2.cu
-int w4_tmem_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
-                         bool promote, int* status, cudaStream_t stream);  // w4_tmem.cu
 int w4_gemm_tc_launch(const unsigned char* wq, int scale_dtype, const int32_t* perm, const void* x, void* y, int64_t M, int64_t N,
                       int64_t K, int act_dtype, void* gathered, int* status, cudaStream_t stream);  // w4_gemm.cu
 
@@ -141,7 +137,6 @@ static W4Params w4_params(const void* wq, const int32_t* perm, const void* x, vo
     p.scale_dtype = scale_dtype;
     p.x_rows = nullptr;
     p.y_rows = nullptr;
-    p.y_ptrs = nullptr;
     return p;
 }
 
@@ -224,7 +219,8 @@ extern "C" const char* eq_w4a16_kernel(int64_t M, int64_t N, int64_t K, int has_
 // ---- gate / up + SwiGLU in one call ---------------------------------------------------------------------------
 // h[M, I] = act(silu(x W_gate)) * (x W_up) for a [gate | up] weight (the two projections concatenated along N, as the
 // reference stores them: emmy/compiler/trace/huggingface.py:1663-1669, 2110-2141), with the eager form's two roundings.
-// M > 16: the tensor path with gate and up tiles side by side in a CTA and the activation in the epilogue; fewer rows: the [gate | up] linear into scratch, then an elementwise pass.
+// M > 16: the tensor path with gate and up tiles side by side in a CTA and the activation in the epilogue; fewer rows: the
+// [gate | up] linear into scratch, then an elementwise pass.
 namespace eq {
 namespace {
 

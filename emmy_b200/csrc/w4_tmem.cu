@@ -490,10 +490,7 @@ int launch_dense(W4TmemArgs a, const void* x, int scale_dtype, cudaStream_t stre
 
 template <typename ActT>
 int dense_typed(const W4TmemArgs& a, const void* x, int scale_dtype, bool swiglu, bool promote, cudaStream_t stream) {
-    if (promote) {
-        if (a.M <= 16) return swiglu ? launch_dense<ActT, 16, true, true>(a, x, scale_dtype, stream) : launch_dense<ActT, 16, true, false>(a, x, scale_dtype, stream);
-        return swiglu ? launch_dense<ActT, 32, true, true>(a, x, scale_dtype, stream) : launch_dense<ActT, 32, true, false>(a, x, scale_dtype, stream);
-    }
+    if (promote) return swiglu ? launch_dense<ActT, 32, true, true>(a, x, scale_dtype, stream) : launch_dense<ActT, 32, true, false>(a, x, scale_dtype, stream);
     // 65 to 128 rows of a short K, where the epilogue is the larger part, run as two row tiles of 64 on twice as many CTAs (128
     // rows: 512 x 4096 5.8 -> 4.3 us, 512 x 14336 7.4 -> 5.8, 896 x 11136 9.2 -> 6.7; at K=1024 the second expansion costs more)
     if (a.M <= 64 || (!swiglu && a.M <= 128 && a.K <= 896)) return swiglu ? launch_dense<ActT, 64, false, true>(a, x, scale_dtype, stream) : launch_dense<ActT, 64, false, false>(a, x, scale_dtype, stream);
@@ -525,12 +522,9 @@ int grouped_typed(const W4TmemArgs& a, const void* x, int64_t R, int scale_dtype
 
 }  // namespace
 
-// Grouped expert GEMM: x [R][K] in expert order; blocks / n_blocks: device-side list of row blocks of at most block_rows
-// (16 or 128) rows of one expert each; wq: stacked repacked weights expert_stride bytes apart.  swiglu: N is the width of
-// the [gate | up] weight, y has N / 2 columns.
 int w4_tmem_grouped_launch(const unsigned char* wq, size_t expert_stride, int scale_dtype, const void* x, void* y, int64_t R, int64_t N, int64_t K,
-                           int act_dtype, const RowBlock* blocks, const int32_t* n_blocks, int block_rows, const int32_t* y_rows, const uint64_t* y_ptrs,
-                           bool swiglu, int* status, cudaStream_t stream) {
+                           int act_dtype, const RowBlock* blocks, const int32_t* n_blocks, int block_rows, const int32_t* y_rows, bool swiglu, int* status,
+                           cudaStream_t stream) {
     W4TmemArgs a = {};
     a.wq = wq;
     a.y = y;
@@ -541,7 +535,6 @@ int w4_tmem_grouped_launch(const unsigned char* wq, size_t expert_stride, int sc
     a.blocks = blocks;
     a.n_blocks = n_blocks;
     a.y_rows = y_rows;
-    a.y_ptrs = y_ptrs;
     a.expert_stride = expert_stride;
     return act_dtype == EQ_F16 ? grouped_typed<__half>(a, x, R, scale_dtype, swiglu, block_rows, stream)
                                : grouped_typed<__nv_bfloat16>(a, x, R, scale_dtype, swiglu, block_rows, stream);

@@ -1,4 +1,4 @@
-// Arguments of the W4A16 kernel with the weights in tensor memory (w4_tmem.cu).
+// W4A16 with the weights in tensor memory (w4_tmem.cu, w4_tmem2.cu): which calls, launch functions, shared device code.
 #pragma once
 #include "tc_common.cuh"
 #include "w4_tile.cuh"
@@ -47,6 +47,19 @@ inline W4Route w4_route(int64_t M, int64_t N, int64_t K, bool perm, bool swiglu)
     return w4_tmem_pairs(M, N, K) ? W4Route::kPairs : W4Route::kScaled;
 }
 
+// w4_tmem.cu.  Dense: y[M, N] = x W, or with swiglu act(silu(gate)) * up of a [gate | up] weight of N columns; promote: scales on
+// f32 sums (at most 32 rows).  status: one word, set by a bounded wait that ran out.
+int w4_tmem_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
+                         bool promote, int* status, cudaStream_t stream);
+// Grouped: x [R][K] in expert order; blocks / n_blocks: device-side list of row blocks of at most block_rows (16 or 128) rows of
+// one expert each; wq: stacked repacked weights expert_stride bytes apart; y_rows (optional): output row m goes to row y_rows[m].
+int w4_tmem_grouped_launch(const unsigned char* wq, size_t expert_stride, int scale_dtype, const void* x, void* y, int64_t R, int64_t N, int64_t K,
+                           int act_dtype, const RowBlock* blocks, const int32_t* n_blocks, int block_rows, const int32_t* y_rows, bool swiglu, int* status,
+                           cudaStream_t stream);
+// w4_tmem2.cu
+int w4_tmem_pair_dense_launch(const unsigned char* wq, int scale_dtype, const void* x, void* y, int64_t M, int64_t N, int64_t K, int act_dtype, bool swiglu,
+                              int* status, cudaStream_t stream);
+
 struct W4TmemArgs {
     const unsigned char* wq;   // repacked weight (of expert 0)
     void* y;
@@ -58,7 +71,6 @@ struct W4TmemArgs {
     const RowBlock* blocks;
     const int32_t* n_blocks;
     const int32_t* y_rows;     // optional: output row m goes to row y_rows[m]
-    const uint64_t* y_ptrs;    // optional: output row m starts at address y_ptrs[m] (0 = drop the row)
     size_t expert_stride;
 };
 
@@ -200,12 +212,8 @@ __device__ __forceinline__ void emit16(const W4TmemArgs& a, const float (&v)[16]
             const uint32_t w = (lane & 1) ? __byte_perm(p, pn, 0x3276) : __byte_perm(p, pn, 0x5410);
             const int r = c + i + (lane & 1);
             if (live && r < rows) {
-                ActT* dst;
-                if (GROUPED && a.y_ptrs)
-                    dst = reinterpret_cast<ActT*>(a.y_ptrs[row0 + r]);  // null: drop the row
-                else
-                    dst = static_cast<ActT*>(a.y) + (GROUPED && a.y_rows ? static_cast<size_t>(a.y_rows[row0 + r]) : static_cast<size_t>(row0 + r)) * a.N;
-                if (!GROUPED || dst) *reinterpret_cast<uint32_t*>(dst + ch) = w;
+                const size_t row = GROUPED && a.y_rows ? static_cast<size_t>(a.y_rows[row0 + r]) : static_cast<size_t>(row0 + r);
+                *reinterpret_cast<uint32_t*>(static_cast<ActT*>(a.y) + row * a.N + ch) = w;
             }
         }
     }

@@ -191,9 +191,12 @@ def w4a16_gate_up_swiglu(x: torch.Tensor, w: W4Weight, workspace: torch.Tensor |
         raise ValueError(f"x has {k} features, the weight {w.k}; the [gate | up] width {w.n} must be a multiple of 32")
     inter = w.n // 2
     h = out if out is not None else torch.empty((m, inter), dtype=x.dtype, device=x.device)
-    need = L.load().eq_w4a16_gate_up_workspace_bytes(m, inter, k)
-    # up to 16 rows take kernels that meet in a workspace which is zero between calls; more rows read nothing of it
-    ws = workspace if workspace is not None else torch.zeros(max(need, 256), dtype=torch.uint8, device=x.device) if m <= 16 else _scratch(need, x.device)
+    if workspace is not None:
+        ws = workspace
+    elif m <= 16:  # kernels that meet in a workspace which is zero between calls, and scratch behind it that is not
+        ws = torch.zeros(max(L.load().eq_w4a16_gate_up_workspace_bytes(m, inter, k), 256), dtype=torch.uint8, device=x.device)
+    else:  # only the status word is used: the linear's kept buffer, where w4a16_status finds it
+        ws = w4a16_workspace(m, w.n, x.device, k)
     L.check(L.load().eq_w4a16_gate_up_swiglu(_ptr(w.wq), _DTYPE[w.scale_dtype], _ptr(w.perm), w.k, inter, w.group, _ptr(x), m, _DTYPE[x.dtype],
                                              _ptr(h), _ptr(ws), ws.numel(), _stream()))
     return h

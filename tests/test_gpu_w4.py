@@ -563,6 +563,29 @@ def test_pair_tiles_scattered_act_order(m):
     assert not ws.any()
 
 
+def test_gate_up_default_workspace_carries_the_status():
+    """Above 16 rows a call without a workspace takes the buffer that is kept per stream: nothing is allocated, and a status word
+    that is set there is reported and cleared."""
+    from emmy_b200 import ops
+
+    m, k, inter = 200, 256, 1024
+    parts = [_awq(k, inter, "f16", False, seed=i)[1] for i in range(2)]
+    w = ops.w4_concat([ops.w4_repack(*p, 128, "awq") for p in parts])
+    x, h = act(synth.activations(m, k, "f16"), "f16"), torch.empty(m, inter, dtype=torch.float16, device="cuda")
+    ops.w4a16_gate_up_swiglu(x, w, out=h)
+    ws = ops.w4a16_workspace(m, w.n, x.device, k)
+    ops.w4a16_status(ws, m, w.n)
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    ops.w4a16_gate_up_swiglu(x, w, out=h)
+    assert torch.cuda.max_memory_allocated() == before
+    ws[:4].view(torch.int32).fill_(3)
+    ops.w4a16_gate_up_swiglu(x, w, out=h)
+    with pytest.raises(ops.L.EmmyqError):
+        ops.w4a16_status(ops.w4a16_workspace(m, w.n, x.device, k), m, w.n)
+    ops.w4a16_status(ws, m, w.n)
+
+
 @pytest.mark.parametrize("m,n", [(20, 256), (64, 256), (300, 9488)])
 def test_linear_behind_a_kernel_that_takes_a_second(m, n):
     """The tensor-path kernels are resident while the kernel before them still runs, and that kernel may take longer than

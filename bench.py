@@ -9,14 +9,14 @@ Headline (`gptq_llama8b_mlp_m1`): the W4A16 M=1 GEMV on GPTQ act-order weights w
 and down projections (96 GEMVs, 2.9 GB of packed weights, far larger than L2, so every step streams its weights from
 HBM).  Metric: algorithmic HBM bytes per second.
 
-The same JSON line carries `extra`: one record per other call of the path at the benchmark shapes (AWQ and GPTQ at
+Ahead of that line, one line `extra {...}` per other call of the path at the benchmark shapes (AWQ and GPTQ at
 their row counts, FP8 and NVFP4 linears, the MoE layer; with N > 1 also the sharded layers), each timed the same way:
 one CUDA graph per step over weight copies that exceed L2, ten samples of the replay region, median / min / max, the
 roofline floor that binds (the higher of bytes / HBM bandwidth and flops / tensor peak), and the end-to-end figure
 with pinned host buffers.  `--workload NAME` runs one of them alone under the headline's contract (these are the
 commands the profiles were made with).
 
-Prints ONE JSON line on rank 0.  Launched by torchrun for N > 1 (one rank per GPU); every rank then owns its own
+Prints ONE JSON line on rank 0, the last one.  Launched by torchrun for N > 1 (one rank per GPU); every rank then owns its own
 32-layer stack (weak scaling: independent layers, no data-path collective).
 """
 
@@ -372,7 +372,7 @@ def wl_fp8(device, rank, m, n=GEMM_N, k=GEMM_K):
 
     return dict(step=step, calls=copies, kernels_per_call=2, alg_bytes=n * k + n * 4 + m * k * 2 + m * n * 2, flops=2.0 * m * k * n, peak_mult=2.0,
                 h2d=[(x, x_host)], d2h=[(y_host, y)], status=lambda: ops.fp8_status(wsp, m, k),
-                kernel="fp8_gemm_tc_kernel<__nv_bfloat16>" if m > 16 else "fp8_decode_tc_kernel<__nv_bfloat16>",
+                kernel="fp8_gemm_tc_kernel<__nv_bfloat16>" if m > 64 else "fp8_decode_tc_kernel<__nv_bfloat16>",
                 dtype="e4m3 weights and activations, f32 accumulate, bf16 out")
 
 
@@ -395,7 +395,7 @@ def wl_nvfp4(device, rank, m, n=GEMM_N, k=GEMM_K):
 
     return dict(step=step, calls=copies, kernels_per_call=2, alg_bytes=n * k // 2 + n * k // 16 + 4 + m * k * 2 + m * n * 2, flops=2.0 * m * k * n,
                 peak_mult=4.0, h2d=[(x, x_host)], d2h=[(y_host, y)], status=lambda: o4.nvfp4_status(wsp, m, k),
-                kernel="nvfp4_gemm_tc_kernel<__nv_bfloat16>", dtype="e2m1 weights and activations with e4m3 block scales, f32 accumulate, bf16 out")
+                kernel=f"nvfp4_{'decode' if m <= 16 else 'gemm_tc' if m <= 1792 else 'gemm_tc_wide'}_kernel<__nv_bfloat16>", dtype="e2m1 weights and activations with e4m3 block scales, f32 accumulate, bf16 out")
 
 
 MOE = dict(e=128, topk=8, hidden=2048, inter=768)
@@ -547,7 +547,7 @@ def wl_tp_mlp(device, rank, world, m):
 
 
 def measure(wl, device, world, steps, clocks, name, metric, unit, workload):
-    """Times one workload and returns its `extra` record."""
+    """Times one workload and returns its record."""
     stream = torch.cuda.Stream(device)
     timer = Timer(wl["step"], stream, device, world, capture=wl.get("capture", True))
     with torch.cuda.stream(stream):
@@ -716,8 +716,9 @@ def run_ours(args, rank, world, local_rank):
                     "note": f"{SAMPLES} repeats of the {args.steps}-step region after the contract's region; hot_l2: one layer's weights (92 MB) replayed, resident in L2"},
         "clocks": headline_clocks,
         "cpu_baseline": cpu_baseline(sample_layers=1),
-        "extra": extras,
     }
+    for rec in extras:  # lines of their own: the headline stays short enough to be read from the end of the output
+        print("extra " + json.dumps(rec))
     print(json.dumps(line), flush=True)
 
 

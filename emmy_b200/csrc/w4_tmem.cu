@@ -197,7 +197,6 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
         int stage = wg, phase = 1, ring_at = wg;  // stage and (inverted) use parity of that item; its scales' slot
         uint32_t slot = my_ring;
         bool first = true, broken = false;
-        bool waited = false;  // behind griddepcontrol.wait
         int n_unit = 0;
         const int g = lane >> 2, j = lane & 3;
         const uint32_t a_lane = tmem_a + (static_cast<uint32_t>(32 * q) << 16);
@@ -213,16 +212,10 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                 prefetch();  // refills the slot just read
                 slot += 2 * kItemBytes;
                 if (slot == my_ring + D * 2 * kItemBytes) slot = my_ring;
-                if (!first) {
-                    if (!GROUPED && !waited) {
-                        asm volatile("griddepcontrol.wait;" ::: "memory");  // bounded waits count from the moment x exists
-                        waited = true;
-                    }
-                    if (!__all_sync(0xFFFFFFFFu, wait_asleep(empty + 8 * stage, phase))) {
-                        if (lane == 0) atomicExch(a.status, 4);
-                        broken = true;
-                        break;
-                    }
+                if (!first && !__all_sync(0xFFFFFFFFu, wait_asleep(empty + 8 * stage, phase))) {
+                    if (lane == 0) atomicExch(a.status, 4);
+                    broken = true;
+                    break;
                 }
                 tc::fence_after_sync();
                 if constexpr (PROMOTE) {
@@ -244,15 +237,14 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                 if (stage >= S) {
                     stage -= S;
                     phase ^= 1;
+                    // every stage is filled: from here on the warp waits, and its bounded waits count from the moment x exists
+                    if (!GROUPED && first) asm volatile("griddepcontrol.wait;" ::: "memory");
                     first = false;
                 }
             }
             next -= n_items;
             if constexpr (!PROMOTE) {
-                if (!GROUPED && !waited) {
-                    asm volatile("griddepcontrol.wait;" ::: "memory");  // y and the workspace may be in use by the previous grid
-                    waited = true;
-                }
+                if (!GROUPED && first) asm volatile("griddepcontrol.wait;" ::: "memory");  // y may be in use by the previous grid, too
                 const bool ok = __all_sync(0xFFFFFFFFu, wait_asleep(acc_full, n_unit & 1));
                 if (!ok && lane == 0) atomicExch(a.status, 3);
                 broken |= !ok;

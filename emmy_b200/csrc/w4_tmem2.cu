@@ -143,7 +143,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
         int next = wg;  // this warp's next item (every fourth of the pair's sequence), from the start of the current unit
         uint32_t slot = my_ring, phase = 1;
-        bool first = true, broken = false, waited = false;
+        bool first = true, broken = false;
         int n_unit = 0;
         const uint32_t a_dst = tmem_a + (static_cast<uint32_t>(32 * q) << 16) + 64 * wg;
         const uint32_t my_full = lead_full_a + 8 * wg, my_empty = empty_a + 8 * wg;
@@ -158,18 +158,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 prefetch();  // refills the slot just read
                 slot += 2 * kItemBytes;
                 if (slot == my_ring + kDepth * 2 * kItemBytes) slot = my_ring;
-                if (!first) {
-                    if (!waited) {
-                        asm volatile("griddepcontrol.wait;" ::: "memory");  // bounded waits count from the moment x exists
-                        waited = true;
-                    }
-                    if (!__all_sync(0xFFFFFFFFu, wait_asleep(my_empty, phase))) {
-                        if (lane == 0) atomicExch(a.status, 4);
-                        broken = true;
-                        break;
-                    }
+                if (!first && !__all_sync(0xFFFFFFFFu, wait_asleep(my_empty, phase))) {
+                    if (lane == 0) atomicExch(a.status, 4);
+                    broken = true;
+                    break;
                 }
-                first = false;
                 phase ^= 1;
                 tc::fence_after_sync();
                 expand_item<ActT, CVT, false>(w, a_dst);
@@ -177,15 +170,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) tc::arrive_pair(my_full);
+                // the stage is filled: from here on the warp waits, and its bounded waits count from the moment x exists
+                if (first) asm volatile("griddepcontrol.wait;" ::: "memory");
+                first = false;
             }
             next -= items;
             // ---- epilogue: group wg takes the 16-row chunks wg, wg + 4, ...
             int col, row0, rows;
             locate(u, col, row0, rows);
-            if (!waited) {
-                asm volatile("griddepcontrol.wait;" ::: "memory");  // y may be in use by the previous grid
-                waited = true;
-            }
+            if (first) asm volatile("griddepcontrol.wait;" ::: "memory");  // (no item yet) y may be in use by the previous grid, too
             if (!__all_sync(0xFFFFFFFFu, wait_asleep(acc_full, n_unit & 1))) {
                 if (lane == 0) atomicExch(a.status, 3);
                 break;

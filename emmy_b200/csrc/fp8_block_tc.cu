@@ -27,7 +27,7 @@ constexpr int kTileA = kBM * kBK;
 // BN = 256: two weight scale blocks per CTA, eight promotion warps, four 48 KB stages, all of TMEM.  BN = 128 (calls of
 // at most 128 rows, where the grid is one row of CTAs): twice as many CTAs stream the weight, six 32 KB stages.
 //
-// The promotion bounds the kernel: a K block takes about 950 cycles against 512 of MMA (128 x 256 x 128 products at 8192 a
+// The promotion bounds the kernel: a K block takes about 1050 cycles against 512 of MMA (128 x 256 x 128 products at 8192 a
 // clock), for 128 adds and 16 KB of TMEM reads per warp and block.  So a block's factor is loaded one block ahead, off the
 // path behind the wait: K=5120 N=17408, 300 rows 62.8 -> 56.0 us, 2048 rows 237 -> 210, 8192 rows 878 -> 797.
 // Measured on top of that and dropped: reading the accumulator in pieces of 16 columns, one under way while the other is

@@ -24,8 +24,8 @@
 // Why the roles are this way round: with rows as the MMA's M a 64-row call pads every MMA to 128 rows and pushes each
 // dequantised byte through shared memory twice (store, operand read).  Measured against that form (us, rows as M, dequant
 // through shared memory -> here; K=4096 N=14336 | K=14336 N=4096 | K=N=4096): 64 rows 33.0 -> 17.1 | 31.3 -> 17.2 | 18.2 ->
-// 11.1; 128 rows 35.6 -> 21.5 | 39.7 -> 22.6; 256 rows of K=N=4096 50.2 -> 16.5; the MLP of hidden 4096, intermediate 14336:
-// 64 rows 81 -> 45, 128 rows 90 -> 58.
+// 11.1; 128 rows 35.6 -> 21.5 | 39.7 -> 22.6; 256 rows of K=N=4096 50.2 -> 16.5; an MLP of hidden 4096, intermediate 14336,
+// 64 rows, over more layers than the L2 holds: 81 -> 47 to 49.
 //
 // What bounds it: issue slots.  An item costs an SM about 1600 warp instructions (eight nibbles: five integer and eight half
 // instructions and one shared read) against the 380 cycles HBM needs for its bytes; two CTAs of ten or fourteen warps are what

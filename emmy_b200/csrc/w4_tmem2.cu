@@ -12,7 +12,7 @@
 // TMEM: 256 accumulator columns + 4 stages of 64 columns of A = 512.  (Two accumulators of 192 columns and two stages,
 // with the epilogue under the next unit's main loop, measured slower: the stages are what hides the expansion's latency.)
 // Measured (us, one-CTA 256 x 256 tiles with the dequant through shared memory -> here): K=4096 N=14336, 2048 rows 232.6 ->
-// 182.4; the MLP of hidden 4096, intermediate 14336: 300 rows 196 -> 134, 1024 rows 366 -> 277, 4096 rows 1204 -> 1076.
+// 182.4; [gate | up] of hidden 4096, intermediate 14336: 300 rows 111 -> 82, 1024 rows 242 -> 190, 4096 rows 841 -> 724.
 // Persistent over units (column tile of 256, row tile); A holds (q - z) * scale in the activation dtype, f32 accumulation
 // over all of K.
 #include "tc_common.cuh"

@@ -111,7 +111,7 @@ def gptq_weight(request):
 @pytest.mark.parametrize("m", [1, 4, 16, 64, 256])
 def test_gptq_llama_mlp(m, gptq_weight):
     """Both Llama-3.1-8B MLP shapes against the oracle's dequantize-then-matmul; K = 14336, N = 4096 at M = 64 is the
-    split-K form of the tensor path (partial sums meet in the workspace)."""
+    tensor path with K slices (partial tiles meet in distributed shared memory, in a fixed order)."""
     from emmy_b200 import ops
 
     k, n, qw, qz, sc, gi, w = gptq_weight

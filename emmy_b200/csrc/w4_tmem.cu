@@ -197,6 +197,7 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
         int stage = wg, phase = 1, ring_at = wg;  // stage and (inverted) use parity of that item; its scales' slot
         uint32_t slot = my_ring;
         bool first = true, broken = false;
+        bool waited = false;  // behind griddepcontrol.wait
         int n_unit = 0;
         const int g = lane >> 2, j = lane & 3;
         const uint32_t a_lane = tmem_a + (static_cast<uint32_t>(32 * q) << 16);
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                 prefetch();  // refills the slot just read
                 slot += 2 * kItemBytes;
                 if (slot == my_ring + D * 2 * kItemBytes) slot = my_ring;
-                if (!first && !__all_sync(0xFFFFFFFFu, wait_asleep(empty + 8 * stage, phase))) {
+                if (!first && !__all_sync(0xFFFFFFFFu, wait_asleep<!GROUPED>(empty + 8 * stage, phase))) {
                     if (lane == 0) atomicExch(a.status, 4);
                     broken = true;
                     break;
@@ -237,14 +238,15 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                 if (stage >= S) {
                     stage -= S;
                     phase ^= 1;
-                    // every stage is filled: from here on the warp waits, and its bounded waits count from the moment x exists
-                    if (!GROUPED && first) asm volatile("griddepcontrol.wait;" ::: "memory");
                     first = false;
                 }
             }
             next -= n_items;
             if constexpr (!PROMOTE) {
-                if (!GROUPED && first) asm volatile("griddepcontrol.wait;" ::: "memory");  // y may be in use by the previous grid, too
+                if (!GROUPED && !waited) {
+                    asm volatile("griddepcontrol.wait;" ::: "memory");  // y may be in use by the previous grid
+                    waited = true;
+                }
                 const bool ok = __all_sync(0xFFFFFFFFu, wait_asleep(acc_full, n_unit & 1));
                 if (!ok && lane == 0) atomicExch(a.status, 3);
                 broken |= !ok;
@@ -269,8 +271,7 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
     } else if (PROMOTE && warp < kDW + 4) {
         // ---- promotion: sums[r] += scale * accumulator, then the epilogue
         int seq = 0;
-        bool broken = false;
-        if constexpr (!GROUPED) asm volatile("griddepcontrol.wait;" ::: "memory");  // as the dequant warps: waits, and y in use until then
+        bool broken = false, waited = false;
         const uint32_t t_row = tmem_base + (static_cast<uint32_t>(32 * q) << 16);
         for (int u = blockIdx.x; u < units && !broken; u += gridDim.x) {
             int col, row0, rows, item0, n_items, expert;
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
             for (int i = 0; i < NB; ++i) sum[i] = 0.f;
             for (int it = 0; it < n_items; ++it, ++seq) {
                 const int b = seq & 1;
-                if (!__all_sync(0xFFFFFFFFu, wait_asleep(acc_full + 8 * b, (seq >> 1) & 1))) {
+                if (!__all_sync(0xFFFFFFFFu, wait_asleep<!GROUPED>(acc_full + 8 * b, (seq >> 1) & 1))) {
                     if (lane == 0) atomicExch(a.status, 3);
                     broken = true;
                     break;
@@ -298,6 +299,10 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(acc_empty + 8 * b);
+            }
+            if (!GROUPED && !waited) {
+                asm volatile("griddepcontrol.wait;" ::: "memory");
+                waited = true;
             }
 #pragma unroll
             for (int c = 0; c < NB; c += 16) {
@@ -333,25 +338,24 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                             tc::tma_load_2d(dst + half * (NB * 128) + bx * (Cfg::kBoxRows * 128), &map_x, (item0 + it) * 128 + half * kGK, row0 + bx * Cfg::kBoxRows, bar);
                 }
             }
-            // where a wait ran out nobody else has waited for these: the CTA does not end with a copy under way into its shared memory
-            for (int i = seq < S ? 0 : seq - S; i < seq; ++i) wait_asleep(full_b + 8 * (i % S), (i / S) & 1);
+            if (broken)  // nobody else waits for these: the CTA does not end with a copy under way into its shared memory
+                for (int i = seq < S ? 0 : seq - S; i < seq; ++i) wait_asleep(full_b + 8 * (i % S), (i / S) & 1);
         }
     } else {
         if (tc::elect_one()) {
-            if constexpr (!GROUPED) asm volatile("griddepcontrol.wait;" ::: "memory");  // as the dequant warps
             int seq = 0, n_unit = 0;
             bool broken = false;
             for (int u = blockIdx.x; u < units && !broken; u += gridDim.x, ++n_unit) {
                 int col, row0, rows, item0, n_items, expert;
                 locate(u, col, row0, rows, item0, n_items, expert);
                 const uint32_t idesc = tc::instr_desc(Mul<ActT>::kFmt, Mul<ActT>::kFmt, 128, static_cast<uint32_t>((rows + 15) & ~15));
-                if (!PROMOTE && n_unit > 0) broken = !wait_asleep(acc_empty, (n_unit - 1) & 1);
+                if (!PROMOTE && n_unit > 0) broken = !wait_asleep<!GROUPED>(acc_empty, (n_unit - 1) & 1);
                 for (int it = 0; it < n_items && !broken; ++it, ++seq) {
                     const int stage = seq % S, b = PROMOTE ? (seq & 1) : 0;
                     const uint32_t parity = (seq / S) & 1;
-                    bool ok = !PROMOTE || seq < 2 || wait_asleep(acc_empty + 8 * b, ((seq >> 1) - 1) & 1);
-                    ok = ok && wait_asleep(full_b + 8 * stage, parity);
-                    ok = ok && wait_asleep(full_a + 8 * stage, parity);
+                    bool ok = !PROMOTE || seq < 2 || wait_asleep<!GROUPED>(acc_empty + 8 * b, ((seq >> 1) - 1) & 1);
+                    ok = ok && wait_asleep<!GROUPED>(full_b + 8 * stage, parity);
+                    ok = ok && wait_asleep<!GROUPED>(full_a + 8 * stage, parity);
                     if (!ok) {
                         broken = true;
                         break;
@@ -368,7 +372,8 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                 if (!PROMOTE) tc::mma_commit(acc_full);
                 if (broken) {
                     atomicExch(a.status, 2);
-                    // the columns are freed below: not with an MMA under way
+                    // neither shared memory nor TMEM goes back with a copy (one that was never issued runs out) or an MMA under way
+                    for (int i = seq; i < seq + S; ++i) wait_asleep(full_b + 8 * (i % S), (i / S) & 1);
                     if (!PROMOTE) wait_asleep(acc_full, n_unit & 1);
                     if (PROMOTE && seq > 0) wait_asleep(acc_full + 8 * ((seq - 1) & 1), ((seq - 1) >> 1) & 1);
                 }

@@ -79,8 +79,13 @@ namespace tm {
 
 // Bounded wait as tc::mbar_wait, but the thread sleeps in the barrier unit between looks: with dequantisation bound by issue
 // slots, spinning TMA and MMA threads would take theirs.
+// DEPENDENT: in a programmatic dependent the warps wait for each other while the grid before it may still run, for as long as
+// it likes: a wait that runs out is taken once more from the end of that grid.  (griddepcontrol.wait ahead of the first wait
+// does that too, but costs 0.3 to 0.6 us of a 16 us launch where launches follow each other.)
+template <bool DEPENDENT = false>
 __device__ __forceinline__ bool wait_asleep(uint32_t bar, uint32_t parity) {
-    const long long start = clock64();
+    bool again = DEPENDENT;
+    long long start = clock64();
     for (;;) {
         uint32_t ok;
         asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
@@ -88,7 +93,12 @@ __device__ __forceinline__ bool wait_asleep(uint32_t bar, uint32_t parity) {
                      : "r"(bar), "r"(parity), "r"(1000000u)
                      : "memory");
         if (ok) return true;
-        if (clock64() - start > tc::kWaitCycles) return false;
+        if (clock64() - start > tc::kWaitCycles) {
+            if (!again) return false;
+            again = false;
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            start = clock64();
+        }
     }
 }
 

@@ -143,7 +143,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
         int next = wg;  // this warp's next item (every fourth of the pair's sequence), from the start of the current unit
         uint32_t slot = my_ring, phase = 1;
-        bool first = true, broken = false;
+        bool first = true, broken = false, waited = false;
         int n_unit = 0;
         const uint32_t a_dst = tmem_a + (static_cast<uint32_t>(32 * q) << 16) + 64 * wg;
         const uint32_t my_full = lead_full_a + 8 * wg, my_empty = empty_a + 8 * wg;
@@ -158,11 +158,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 prefetch();  // refills the slot just read
                 slot += 2 * kItemBytes;
                 if (slot == my_ring + kDepth * 2 * kItemBytes) slot = my_ring;
-                if (!first && !__all_sync(0xFFFFFFFFu, wait_asleep(my_empty, phase))) {
+                if (!first && !__all_sync(0xFFFFFFFFu, wait_asleep<true>(my_empty, phase))) {
                     if (lane == 0) atomicExch(a.status, 4);
                     broken = true;
                     break;
                 }
+                first = false;
                 phase ^= 1;
                 tc::fence_after_sync();
                 expand_item<ActT, CVT, false>(w, a_dst);
@@ -170,15 +171,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) tc::arrive_pair(my_full);
-                // the stage is filled: from here on the warp waits, and its bounded waits count from the moment x exists
-                if (first) asm volatile("griddepcontrol.wait;" ::: "memory");
-                first = false;
             }
             next -= items;
             // ---- epilogue: group wg takes the 16-row chunks wg, wg + 4, ...
             int col, row0, rows;
             locate(u, col, row0, rows);
-            if (first) asm volatile("griddepcontrol.wait;" ::: "memory");  // (no item yet) y may be in use by the previous grid, too
+            if (!waited) {
+                asm volatile("griddepcontrol.wait;" ::: "memory");  // y may be in use by the previous grid
+                waited = true;
+            }
             if (!__all_sync(0xFFFFFFFFu, wait_asleep(acc_full, n_unit & 1))) {
                 if (lane == 0) atomicExch(a.status, 3);
                 break;
@@ -227,24 +228,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                                              lead_full_b + 8 * stage);
                 }
             }
-            // where a wait ran out nobody else has waited for these: the pair does not end with a copy under way into either CTA's
-            // rows (the even CTA's barriers count both)
-            if (rank == 0)
+            // nobody else waits for these: the pair does not end with a copy under way into either CTA's rows (the even CTA's
+            // barriers count both)
+            if (broken && rank == 0)
                 for (int i = seq < kStagesB ? 0 : seq - kStagesB; i < seq; ++i) wait_asleep(full_b + 8 * (i % kStagesB), (i / kStagesB) & 1);
         }
     } else if (rank == 0) {
         if (tc::elect_one()) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");  // as the dequant warps
             int seq = 0, n_unit = 0;
             bool broken = false;
             for (int u = cluster; u < units && !broken; u += clusters, ++n_unit) {
                 int col, row0, rows;
                 locate(u, col, row0, rows);
                 const uint32_t idesc = tc::instr_desc(Mul<ActT>::kFmt, Mul<ActT>::kFmt, 256, static_cast<uint32_t>((rows + 15) & ~15));
-                if (n_unit > 0) broken = !wait_asleep(acc_empty, (n_unit - 1) & 1);
+                if (n_unit > 0) broken = !wait_asleep<true>(acc_empty, (n_unit - 1) & 1);
                 for (int it = 0; it < items && !broken; ++it, ++seq) {
                     const int sa = seq % kStagesA, sb = seq % kStagesB;
-                    if (!wait_asleep(full_b + 8 * sb, (seq / kStagesB) & 1) || !wait_asleep(full_a + 8 * sa, (seq / kStagesA) & 1)) {
+                    if (!wait_asleep<true>(full_b + 8 * sb, (seq / kStagesB) & 1) || !wait_asleep<true>(full_a + 8 * sa, (seq / kStagesA) & 1)) {
                         broken = true;
                         break;
                     }
@@ -260,7 +260,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 tc::commit_pair(acc_full);
                 if (broken) {
                     atomicExch(a.status, 2);
-                    wait_asleep(acc_full, n_unit & 1);  // the columns are freed below: not with an MMA under way
+                    // neither shared memory nor TMEM goes back with a copy (one that was never issued runs out) or an MMA under way
+                    for (int i = seq; i < seq + kStagesB; ++i) wait_asleep(full_b + 8 * (i % kStagesB), (i / kStagesB) & 1);
+                    wait_asleep(acc_full, n_unit & 1);
                 }
             }
         }

@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(kDtThreads, 2)
                 const int s = kb % kDtStages;
                 if (!tc::mbar_wait(tc::smem_u32(empty + s), ((kb / kDtStages) - 1) & 1)) {
                     atomicExch(status, 1);
+                    tc::drain_copies(full, kb - kDtStages, kb, kDtStages);
                     break;
                 }
                 const uint32_t bar = tc::smem_u32(full + s);
@@ -197,6 +198,7 @@ __global__ void __launch_bounds__(kDtThreads, 2)
                 const int s = kb % kDtStages;
                 if (!tc::mbar_wait(tc::smem_u32(full + s), (kb / kDtStages) & 1)) {
                     atomicExch(status, 2);
+                    tc::drain_copies(full, kb, min(kb + kDtStages, k_blocks), kDtStages);
                     break;
                 }
                 tc::fence_after_sync();
@@ -307,6 +309,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                 const int s = kb % kStages;
                 if (kb >= kStages && !tc::mbar_wait(tc::smem_u32(empty + s), ((kb / kStages) - 1) & 1)) {
                     atomicExch(status, 1);
+                    tc::drain_copies(full, kb - kStages, kb, kStages);
                     break;
                 }
                 const uint32_t bar = tc::smem_u32(full + s);
@@ -323,6 +326,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                 const int s = kb % kStages;
                 if (!tc::mbar_wait(tc::smem_u32(full + s), (kb / kStages) & 1)) {
                     atomicExch(status, 2);
+                    tc::drain_copies(full, kb, min(kb + kStages, k_blocks), kStages);
                     break;
                 }
                 tc::fence_after_sync();

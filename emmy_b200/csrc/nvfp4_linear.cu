@@ -309,6 +309,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                 const int s = kb % kStages;
                 if (!tc::mbar_wait(tc::smem_u32(empty + s), ((kb / kStages) - 1) & 1)) {
                     atomicExch(status, 1);
+                    tc::drain_copies(full, kb - kStages, kb, kStages);
                     break;
                 }
                 const uint32_t bar = tc::smem_u32(full + s);
@@ -324,6 +325,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                 const int s = kb % kStages;
                 if (!tc::mbar_wait(tc::smem_u32(full + s), (kb / kStages) & 1)) {
                     atomicExch(status, 2);
+                    tc::drain_copies(full, kb, min(kb + kStages, k_blocks), kStages);
                     break;
                 }
                 tc::fence_after_sync();
@@ -463,6 +465,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
                 const int s = kb % kDecStages;
                 if (!tc::mbar_wait(tc::smem_u32(empty + s), ((kb / kDecStages) - 1) & 1)) {
                     atomicExch(status, 1);
+                    tc::drain_copies(full, kb - kDecStages, kb, kDecStages);
                     break;
                 }
                 const uint32_t bar = tc::smem_u32(full + s);
@@ -478,6 +481,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
                 const int s = kb % kDecStages;
                 if (!tc::mbar_wait(tc::smem_u32(full + s), (kb / kDecStages) & 1)) {
                     atomicExch(status, 2);
+                    tc::drain_copies(full, kb, min(kb + kDecStages, k_blocks), kDecStages);
                     break;
                 }
                 tc::fence_after_sync();
@@ -583,6 +587,7 @@ __global__ void __launch_bounds__(kWThreads, 1)
                 const int s = kb % kWStages;
                 if (kb >= kWStages && !tc::mbar_wait(tc::smem_u32(empty + s), ((kb / kWStages) - 1) & 1)) {
                     atomicExch(status, 1);
+                    tc::drain_copies(full, kb - kWStages, kb, kWStages);
                     break;
                 }
                 const uint32_t bar = tc::smem_u32(full + s);
@@ -604,6 +609,7 @@ __global__ void __launch_bounds__(kWThreads, 1)
                 const int s = kb % kWStages;
                 if (!tc::mbar_wait(tc::smem_u32(full + s), (kb / kWStages) & 1)) {
                     atomicExch(status, 2);
+                    tc::drain_copies(full, kb, min(kb + kWStages, k_blocks), kWStages);
                     break;
                 }
                 tc::fence_after_sync();

@@ -50,6 +50,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     return true;
 }
 
+// For a thread that gives up: the copies [from, to) of a ring of `stages` full barriers have landed when this returns, or were never
+// issued and ran out.  A CTA must not end with a copy under way into its shared memory.
+__device__ __forceinline__ void drain_copies(const uint64_t* full, int from, int to, int stages) {
+    for (int i = from < 0 ? 0 : from; i < to; ++i) mbar_wait(smem_u32(full + i % stages), (i / stages) & 1);
+}
+
 // ---- TMA ----------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
     asm volatile(

@@ -127,10 +127,10 @@ __global__ void __launch_bounds__(kThreads)
             int stage = 0;
             uint32_t phase = 0;
             bool first = true;
-            int kb = 0;
-            for (; kb < k_blocks; ++kb) {
+            for (int kb = 0; kb < k_blocks; ++kb) {
                 if (!first && !tc::mbar_wait(empty_addr + 8 * stage, phase ^ 1)) {
                     atomicExch(status, 1);
+                    tc::drain_copies(full_a, kb - kStages, kb, kStages);
                     break;
                 }
                 const uint32_t bar = full_a_addr + 8 * stage;
@@ -142,8 +142,6 @@ __global__ void __launch_bounds__(kThreads)
                     first = false;
                 }
             }
-            // where a wait ran out nobody else has waited for these: the CTA does not end with a copy under way into its shared memory
-            for (int i = kb < kStages ? 0 : kb - kStages; i < kb; ++i) tc::mbar_wait(full_a_addr + 8 * (i % kStages), (i / kStages) & 1);
         }
     } else if (warp == 1) {
         // ---- MMA issuer
@@ -156,6 +154,7 @@ __global__ void __launch_bounds__(kThreads)
                 const bool got_b = got_a && tc::mbar_wait(full_b_addr + 8 * stage, phase);
                 if (!got_b) {
                     atomicExch(status, 2);
+                    tc::drain_copies(full_a, kb, min(kb + kStages, k_blocks), kStages);
                     break;
                 }
                 tc::fence_after_sync();
@@ -175,7 +174,6 @@ __global__ void __launch_bounds__(kThreads)
                 }
             }
             tc::mma_commit(tc::smem_u32(acc_ready));  // on a broken pipeline too: the epilogue must not sit out its wait
-            tc::mbar_wait(tc::smem_u32(acc_ready), 0);  // nor does TMEM go back with an MMA under way
         }
     } else {
         // ---- dequant producers

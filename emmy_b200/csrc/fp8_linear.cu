@@ -9,12 +9,16 @@
 //                           are the MMA's A operand, the rows its B operand with N = 16 -- so one TMA thread streams the
 //                           weight, 108 KB CTAs of two consecutive launches share an SM, and the weights are requested
 //                           before griddepcontrol.wait (the quantize and the linear are both programmatic dependents).
-//   fp8_gemm_tc_kernel      M > 16 (prefill-shaped): tcgen05.mma kind::f8f6f4, 256x256 output tile per CTA, K-major
-//                           operands brought by TMA with the 128-byte swizzle through a 3-stage mbarrier ring,
-//                           f32 accumulators in TMEM, one producer warp, one MMA warp, eight epilogue warps that read
-//                           TMEM with tcgen05.ld, apply both scales and store bf16/f16.
+//   fp8_gemm_tc_kernel      64 < M <= 128: tcgen05.mma kind::f8f6f4, 128 x 128 output tile per CTA, K-major operands brought
+//                           by TMA with the 128-byte swizzle through a ring of stages, f32 accumulators in TMEM, one producer
+//                           warp, one MMA warp, eight epilogue warps that read TMEM with tcgen05.ld, apply both scales and
+//                           store bf16/f16.
+//   gemm_pair.cu            M > 128: 256 x 256 tiles on CTA pairs
 // Both scales are hoisted out of the contraction, as in the reference's own native FP8 path
 // (tests/compiler/passes/test_fp8_mma.py:111-120).
+#include <type_traits>
+
+#include "gemm_pair.cuh"
 #include "tc_common.cuh"
 
 namespace eq {
@@ -241,32 +245,21 @@ __global__ void __launch_bounds__(kDtThreads, 2)
 }
 
 // ------------------------------------------------------------------------------------------------ prefill-shaped
-// A CTA computes a 256 x 256 output tile as two 128-row MMAs that share one B tile in shared memory: per byte
-// brought in from L2 that is 256 flop, against 170 for a 128 x 256 tile, and L2 -> SM bandwidth is what bounds
-// this kernel (a 128 x 256 tile needs ~19 TB/s of it at the tensor peak).  The two f32 accumulators fill TMEM.
-// Calls with at most 128 rows (one row tile) run 128 x 128 tiles instead: twice as many CTAs stream the weight, deeper
-// stages, and two such CTAs fit an SM.
+// One row tile (at most 128 rows): 128 x 128 tiles, so that many CTAs stream the weight; deep stages, and two such CTAs fit an SM.
+constexpr int kBM = 128, kBN = 128;
 constexpr int kBK = 128;  // K step in bytes = e4m3 elements
+constexpr int kTileA = kBM * kBK, kTileB = kBN * kBK;
+constexpr int kStages = 6;
 constexpr int kEpilogueWarps = 8;
 constexpr int kGemmThreads = (2 + kEpilogueWarps) * 32;
+constexpr size_t kGemmSmem = static_cast<size_t>(kStages) * (kTileA + kTileB) + 1024 /*alignment*/ + 256 /*barriers*/ + kBN * sizeof(float) /*weight scales of the tile*/;
+constexpr uint32_t kTmemCols = kBN;
 
-template <int HALVES, int BN>
-struct Fp8Cfg {
-    static constexpr int kBM = 128 * HALVES;
-    static constexpr int kTileA = kBM * kBK, kTileB = BN * kBK;
-    static constexpr int kStages = HALVES == 2 ? 3 : 6;
-    static constexpr size_t kSmem = static_cast<size_t>(kStages) * (kTileA + kTileB) + 1024 /*alignment*/ + 256 /*barriers*/ + BN * sizeof(float) /*weight scales of the tile*/;
-    static constexpr uint32_t kTmemCols = HALVES * BN;
-};
-
-template <typename OutT, int HALVES, int BN>
+template <typename OutT>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                        const float* __restrict__ sx, const float* __restrict__ sw, OutT* __restrict__ y, int M, int N, int K,
                        int* __restrict__ status) {
-    using Cfg = Fp8Cfg<HALVES, BN>;
-    constexpr int kBM = Cfg::kBM, kBN = BN, kTileA = Cfg::kTileA, kTileB = Cfg::kTileB, kStages = Cfg::kStages;
-    constexpr uint32_t kTmemCols = Cfg::kTmemCols;
     extern __shared__ unsigned char smem_raw[];
     // the swizzled tiles need 1024-byte alignment
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -283,7 +276,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     // row tiles run fastest: the CTAs that share a weight tile are co-resident and the weight comes from DRAM once
     const int n0 = blockIdx.y * kBN, m0 = blockIdx.x * kBM;
     const int k_blocks = K / kBK;
-    const bool two_halves = HALVES == 2 && M - m0 > 128;  // the second 128 rows hold real rows
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -334,33 +326,26 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 #pragma unroll
                 for (int ks = 0; ks < kBK / 32; ++ks) {
                     // 32 bytes of K per instruction: step the descriptors' start address inside the swizzle atom
-                    const uint64_t db = tc::smem_desc_k_sw128(b_addr + ks * 32);
-                    tc::mma_f8f6f4(tmem_base, tc::smem_desc_k_sw128(a_addr + ks * 32), db, idesc, kb > 0 || ks > 0);
-                    if (two_halves)
-                        tc::mma_f8f6f4(tmem_base + kBN, tc::smem_desc_k_sw128(a_addr + 128 * kBK + ks * 32), db, idesc, kb > 0 || ks > 0);
+                    tc::mma_f8f6f4(tmem_base, tc::smem_desc_k_sw128(a_addr + ks * 32), tc::smem_desc_k_sw128(b_addr + ks * 32), idesc, kb > 0 || ks > 0);
                 }
                 tc::mma_commit(tc::smem_u32(empty + s));  // stage is free once these MMAs have read it
             }
             tc::mma_commit(tc::smem_u32(acc_ready));  // on a broken pipeline too, so that the epilogue does not sit out its wait
         }
     } else {
-        // ---- epilogue: warp w may touch TMEM lanes 32 (w % 4) .. +31.  Two row halves: warps 2..5 take rows 0..127,
-        //      6..9 rows 128..255; one row half: the two quartets take half of the columns each.
+        // ---- epilogue: warp w may touch TMEM lanes 32 (w % 4) .. +31; the two quartets of warps take half of the columns each
         const int quarter = warp & 3;
-        const int quartet = (warp - 2) >> 2;
-        const int half = HALVES == 2 ? quartet : 0;
-        const int c_begin = HALVES == 2 ? 0 : quartet * (kBN / 2);
-        const int c_end = HALVES == 2 ? kBN : c_begin + kBN / 2;
-        const int m = m0 + half * 128 + quarter * 32 + lane;
+        const int c_begin = ((warp - 2) >> 2) * (kBN / 2), c_end = c_begin + kBN / 2;
+        const int m = m0 + quarter * 32 + lane;
         const bool ok = tc::mbar_wait(tc::smem_u32(acc_ready), 0);
         if (!ok && lane == 0) atomicExch(status, 3);
         tc::fence_after_sync();
-        if (ok && (half == 0 || two_halves)) {
+        if (ok) {
             const float row_scale = m < M ? sx[m] : 0.f;
 #pragma unroll 1
             for (int c = c_begin; c < c_end; c += 32) {
                 uint32_t r[32];
-                tc::tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * kBN + c, r);
+                tc::tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + c, r);
                 tc::tmem_ld_wait();
                 if (m < M) {
                     OutT* dst = y + static_cast<size_t>(m) * N + n0 + c;
@@ -523,19 +508,18 @@ extern "C" size_t eq_fp8_workspace_bytes(int64_t M, int64_t K) {
     return align_up(static_cast<size_t>(M) * K, 256) + align_up(static_cast<size_t>(M) * sizeof(float), 256) + 256;
 }
 
-template <typename OutT, int HALVES, int BN>
+template <typename OutT>
 static int fp8_tc_launch(const uint8_t* w, const float* sw, int64_t N, int64_t K, const uint8_t* qx, const float* sx, int64_t M, OutT* y,
                          int* status, cudaStream_t stream) {
-    using Cfg = Fp8Cfg<HALVES, BN>;
     CUtensorMap map_a, map_b;
-    int st = make_tensor_map_2d(&map_a, qx, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K, K, Cfg::kBM, kBK, CU_TENSOR_MAP_SWIZZLE_128B);
+    int st = make_tensor_map_2d(&map_a, qx, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K, K, kBM, kBK, CU_TENSOR_MAP_SWIZZLE_128B);
     if (st != EQ_OK) return st;
-    st = make_tensor_map_2d(&map_b, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, BN, kBK, CU_TENSOR_MAP_SWIZZLE_128B);
+    st = make_tensor_map_2d(&map_b, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, kBN, kBK, CU_TENSOR_MAP_SWIZZLE_128B);
     if (st != EQ_OK) return st;
-    auto kernel = fp8_gemm_tc_kernel<OutT, HALVES, BN>;
-    EQ_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmem)));
-    dim3 grid(static_cast<unsigned>(ceil_div(M, Cfg::kBM)), static_cast<unsigned>(ceil_div(N, BN)));
-    kernel<<<grid, kGemmThreads, Cfg::kSmem, stream>>>(map_a, map_b, sx, sw, y, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K),
+    auto kernel = fp8_gemm_tc_kernel<OutT>;
+    EQ_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmem)));
+    dim3 grid(static_cast<unsigned>(ceil_div(M, kBM)), static_cast<unsigned>(ceil_div(N, kBN)));
+    kernel<<<grid, kGemmThreads, kGemmSmem, stream>>>(map_a, map_b, sx, sw, y, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K),
                                                        status);
     EQ_LAUNCH_OK("fp8_gemm_tc_kernel");
     return EQ_OK;
@@ -573,8 +557,9 @@ static int fp8_linear_launch(const uint8_t* w, const float* sw, int64_t N, int64
         if (bx == 32) return run(fp8_decode_tc_kernel<OutT, 32>, DtCfg<32>::kSmem);
         return run(fp8_decode_tc_kernel<OutT, 64>, DtCfg<64>::kSmem);
     }
-    if (M <= 128) return fp8_tc_launch<OutT, 1, 128>(w, sw, N, K, qx, sx, M, y, status, stream);
-    return fp8_tc_launch<OutT, 2, 256>(w, sw, N, K, qx, sx, M, y, status, stream);
+    if (M <= 128) return fp8_tc_launch<OutT>(w, sw, N, K, qx, sx, M, y, status, stream);
+    // (the 256 x 256 one-CTA tile this replaced had the same waves, a tile per SM instead of half a tile: slower at every size)
+    return fp8_pair_launch(qx, sx, w, sw, y, M, N, K, std::is_same<OutT, __half>::value ? EQ_F16 : EQ_BF16, status, stream);
 }
 
 static int fp8_linear_any(const char* who, const uint8_t* weight, const float* weight_scale, int64_t N, int64_t K, const void* x,

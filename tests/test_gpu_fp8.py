@@ -139,6 +139,14 @@ def test_fp8_linear_tile_edges(m, n, k):
     _check(synth.activations(m, k, "bf16", seed=n), bits, sw)
 
 
+@pytest.mark.parametrize("m,n,k", [(700, 16016, 128), (700, 16016, 896), (300, 12304, 1280)])
+def test_fp8_linear_many_tiles_per_pair(m, n, k):
+    """More 256 x 256 tiles than CTA pairs: a pair works through several of them with its two accumulators in turn, K runs
+    shorter, longer and no multiple of the ring of stages, ragged last row and column tiles.  Bound as in _check."""
+    bits, sw = synth.fp8_weight(n, k, seed=k)
+    _check(synth.activations(m, k, "bf16", seed=m), bits, sw)
+
+
 def test_fp8_linear_empty_batch():
     from emmy_b200 import ops
 

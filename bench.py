@@ -372,7 +372,7 @@ def wl_fp8(device, rank, m, n=GEMM_N, k=GEMM_K):
 
     return dict(step=step, calls=copies, kernels_per_call=2, alg_bytes=n * k + n * 4 + m * k * 2 + m * n * 2, flops=2.0 * m * k * n, peak_mult=2.0,
                 h2d=[(x, x_host)], d2h=[(y_host, y)], status=lambda: ops.fp8_status(wsp, m, k),
-                kernel="fp8_gemm_tc_kernel<__nv_bfloat16>" if m > 64 else "fp8_decode_tc_kernel<__nv_bfloat16>",
+                kernel="gemm_pair_kernel" if m > 128 else "fp8_gemm_tc_kernel<__nv_bfloat16>" if m > 64 else "fp8_decode_tc_kernel<__nv_bfloat16>",
                 dtype="e4m3 weights and activations, f32 accumulate, bf16 out")
 
 
@@ -395,7 +395,7 @@ def wl_nvfp4(device, rank, m, n=GEMM_N, k=GEMM_K):
 
     return dict(step=step, calls=copies, kernels_per_call=2, alg_bytes=n * k // 2 + n * k // 16 + 4 + m * k * 2 + m * n * 2, flops=2.0 * m * k * n,
                 peak_mult=4.0, h2d=[(x, x_host)], d2h=[(y_host, y)], status=lambda: o4.nvfp4_status(wsp, m, k),
-                kernel=f"nvfp4_{'decode' if m <= 16 else 'gemm_tc' if m <= 1792 else 'gemm_tc_wide'}_kernel<__nv_bfloat16>", dtype="e2m1 weights and activations with e4m3 block scales, f32 accumulate, bf16 out")
+                kernel="nvfp4_decode_kernel" if m <= 16 else "nvfp4_gemm_tc_kernel" if m <= 128 else "gemm_pair_kernel", dtype="e2m1 weights and activations with e4m3 block scales, f32 accumulate, bf16 out")
 
 
 MOE = dict(e=128, topk=8, hidden=2048, inter=768)

@@ -56,7 +56,7 @@ def nvfp4_tile_scales(scale_bits: torch.Tensor, k: int) -> torch.Tensor:
 
 
 def nvfp4_tile_weight_scales(scale_bits: torch.Tensor, k: int) -> torch.Tensor:
-    """weight_scale [N, K/16] -> the scale blob eq_nvfp4_linear reads (both tile groupings; load time)."""
+    """weight_scale [N, K/16] -> the scale blob eq_nvfp4_linear reads (load time)."""
     _need_cuda(scale_bits)
     rows = scale_bits.shape[0]
     out = torch.empty(L.load().eq_nvfp4_weight_scale_bytes(rows, k), dtype=torch.uint8, device=scale_bits.device)

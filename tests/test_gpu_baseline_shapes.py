@@ -49,7 +49,7 @@ def nvfp4_block():
 
 @pytest.mark.parametrize("m", [1, 128, 2048, 4096])
 def test_nvfp4_k5120_n17408(m, nvfp4_block):
-    """M = 2048 and 4096 run the 256 x 224 kernel through twenty K steps (its three-stage ring wraps six times)."""
+    """M = 2048 and 4096 run the CTA-pair kernel through twenty K steps a tile, several tiles per pair."""
     from emmy_b200 import ops_nvfp4 as o4
 
     n, k = 17408, 5120

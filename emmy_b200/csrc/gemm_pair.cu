@@ -101,10 +101,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
         tc::mbar_fence_init();
     }
+    __syncthreads();
+    tc::cluster_sync();  // both CTAs run, the peer's barriers exist
+    // Not before: an allocation for the pair that one CTA asks for while the other has not started can wait for ever.
     if (warp == 1) tc::tmem_alloc_pair(tc::smem_u32(tmem_slot), 512);
     tc::fence_before_sync();
     __syncthreads();
-    tc::cluster_sync();  // the peer's barriers exist from here on
+    tc::cluster_sync();
     tc::fence_after_sync();
     // With the TMEM columns in hand: a dependent grid that took them first and then waited for this one would never give them back.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -270,6 +273,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     tc::cluster_sync();  // neither CTA leaves while the other may still signal it or read its operands
     tc::fence_after_sync();
     if (warp == 1) tc::tmem_dealloc_pair(tmem_base, 512);
+    __syncwarp();
+    tc::cluster_sync();  // nor before the other has given its columns back
 }
 
 template <typename OutT, bool FP4>

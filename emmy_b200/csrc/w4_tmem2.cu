@@ -87,12 +87,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         tc::mbar_init(acc_empty, 2 * kDW);
         tc::mbar_fence_init();
     }
-    if (warp == kWarps - 1) {
-        tc::tmem_alloc_pair(tc::smem_u32(tmem_slot), kTmemCols);
-    }
+    __syncthreads();
+    tc::cluster_sync();  // both CTAs run, the peer's barriers exist
+    // Not before: an allocation for the pair that one CTA asks for while the other has not started can wait for ever.
+    if (warp == kWarps - 1) tc::tmem_alloc_pair(tc::smem_u32(tmem_slot), kTmemCols);
     tc::fence_before_sync();
     __syncthreads();
-    tc::cluster_sync();  // the peer's barriers exist from here on
+    tc::cluster_sync();
     tc::fence_after_sync();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // with the TMEM columns in hand (w4_tmem.cu)
     const uint32_t tmem_base = *tmem_slot;
@@ -273,6 +274,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     tc::cluster_sync();  // neither CTA leaves while the other may still signal it or read its rows
     tc::fence_after_sync();
     if (warp == kWarps - 1) tc::tmem_dealloc_pair(tmem_base, kTmemCols);
+    __syncwarp();
+    tc::cluster_sync();  // nor before the other has given its columns back
 }
 
 template <typename ActT, bool SWIGLU>

@@ -50,76 +50,113 @@ int w4_gemm_tc_grouped_launch(const unsigned char* wq, size_t expert_stride, int
 constexpr int kMaxTopK = 16;
 constexpr int kBadExpertId = 16;  // status code of a row whose expert id is out of range (1..4 are the tensor path's waits)
 
+// The kernels of a layer are programmatic dependents of one another: each is resident, past its launch latency, when the one
+// before it ends.  Every CTA waits before it touches global memory, and before it returns, so that the end of a grid implies the end
+// of all before it.
+__device__ __forceinline__ void dependent_start() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+static int launch_dependent(void (*kernel)(P...), int64_t grid, int block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(static_cast<unsigned>(block));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    return EQ_OK;
+}
+
 // ------------------------------------------------------------------------------------------------ router
-// One warp per token.  E <= 1024.
-__global__ void moe_route_kernel(const float* __restrict__ logits, int T, int E, int topk, int renorm, int32_t* __restrict__ ids,
-                                 float* __restrict__ scores) {
+// f32 -> a 32-bit key whose unsigned order is the float order, equal for both zeros; 0 for a NaN, which is never picked.
+__device__ __forceinline__ uint32_t route_key(float v) {
+    const uint32_t b = __float_as_uint(v + 0.f);
+    return v != v ? 0u : (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+
+// One warp per token, E <= 32 NV: a lane keeps its logits in registers, a round of the top-k is a scan of their keys and two
+// redux.sync (the maximum, then the lowest expert id that holds it), and a lane keeps each pick.  (Reading the logits again every
+// round and sorting in one lane's local memory took 10 us at 64 tokens of 128 experts and 17 us at 4096.)
+// status, counts (optional): cleared for the kernels behind it.
+template <int NV>
+__global__ void __launch_bounds__(256) moe_route_kernel(const float* __restrict__ logits, int T, int E, int topk, int renorm, int32_t* __restrict__ ids,
+                                                        float* __restrict__ scores, int32_t* __restrict__ status, int32_t* __restrict__ counts) {
+    dependent_start();
+    if (blockIdx.x == 0) {
+        if (status && threadIdx.x == 0) *status = 0;
+        if (counts)
+            for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = 0;
+    }
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= T) return;
     const float* lg = logits + static_cast<size_t>(warp) * E;
-    // softmax statistics
+    float v[NV];
+    uint32_t key[NV];
     float mx = -INFINITY;
-    for (int e = lane; e < E; e += 32) mx = fmaxf(mx, lg[e]);
+#pragma unroll
+    for (int b = 0; b < NV; ++b) {
+        const bool in = lane + 32 * b < E;
+        v[b] = in ? lg[lane + 32 * b] : -INFINITY;
+        key[b] = in ? route_key(v[b]) : 0u;
+        mx = fmaxf(mx, v[b]);
+    }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, off));
+    // softmax denominator
     float sum = 0.f;
-    for (int e = lane; e < E; e += 32) sum += expf(lg[e] - mx);
+#pragma unroll
+    for (int b = 0; b < NV; ++b)
+        if (lane + 32 * b < E) sum += expf(v[b] - mx);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, off);
-    // top-k by repeated arg-max on the logits (they order the experts as the probabilities do); ties -> lowest id
-    int pick_id[kMaxTopK];
-    float pick_p[kMaxTopK];
-    unsigned long long taken_lo = 0;  // this lane's experts already picked (bit = (e - lane) / 32)
-    float psum = 0.f;
+    // top-k on the logits (they order the experts as the probabilities do); ties -> lowest id.  Lane j keeps pick j.
+    int my_id = E - 1;
+    float my_p = 0.f;
     for (int j = 0; j < topk; ++j) {
-        float best = -INFINITY;
-        int best_e = 0x7FFFFFFF;
-        for (int e = lane, b = 0; e < E; e += 32, ++b) {
-            if ((taken_lo >> b) & 1ull) continue;
-            const float v = lg[e];
-            if (v > best || (v == best && e < best_e)) {
-                best = v;
-                best_e = e;
-            }
-        }
+        uint32_t best = 0;
+        int best_b = 0;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, off);
-            const int oe = __shfl_xor_sync(0xFFFFFFFFu, best_e, off);
-            if (ov > best || (ov == best && oe < best_e)) {
-                best = ov;
-                best_e = oe;
+        for (int b = 0; b < NV; ++b)
+            if (key[b] > best) {  // ascending id: the first of equal values stays
+                best = key[b];
+                best_b = b;
             }
+        const uint32_t win = __reduce_max_sync(0xFFFFFFFFu, best);
+        const uint32_t win_e = __reduce_min_sync(0xFFFFFFFFu, best == win && win ? static_cast<uint32_t>(lane + 32 * best_b) : 0xFFFFFFFFu);
+        if (win_e == static_cast<uint32_t>(lane + 32 * best_b) && win) {
+#pragma unroll
+            for (int b = 0; b < NV; ++b)
+                if (b == best_b) key[b] = 0u;
         }
-        if (best_e < E && (best_e & 31) == lane) taken_lo |= 1ull << (best_e >> 5);
-        const float pr = best_e < E ? expf(best - mx) / sum : 0.f;
-        pick_id[j] = best_e < E ? best_e : E - 1;
-        pick_p[j] = pr;
-        psum += pr;
+        if (win && lane == j) {
+            my_id = static_cast<int>(win_e);
+            const float value = __uint_as_float((win & 0x80000000u) ? (win & 0x7FFFFFFFu) : ~win);
+            my_p = expf(value - mx) / sum;
+        }
     }
-    if (lane == 0) {
-        // ascending expert id (insertion sort of at most 16 picks)
-        for (int a = 1; a < topk; ++a) {
-            const int id = pick_id[a];
-            const float pv = pick_p[a];
-            int b = a - 1;
-            while (b >= 0 && pick_id[b] > id) {
-                pick_id[b + 1] = pick_id[b];
-                pick_p[b + 1] = pick_p[b];
-                --b;
-            }
-            pick_id[b + 1] = id;
-            pick_p[b + 1] = pv;
-        }
-        for (int j = 0; j < topk; ++j) {
-            ids[static_cast<size_t>(warp) * topk + j] = pick_id[j];
-            scores[static_cast<size_t>(warp) * topk + j] = renorm ? pick_p[j] / psum : pick_p[j];
-        }
+    // the picks' probabilities are added in the order they were picked, then every pick goes to its place by ascending id
+    float psum = 0.f;
+    int place = 0;
+    for (int j = 0; j < topk; ++j) {
+        psum += __shfl_sync(0xFFFFFFFFu, my_p, j);
+        const int other = __shfl_sync(0xFFFFFFFFu, my_id, j);
+        place += other < my_id || (other == my_id && j < lane) ? 1 : 0;
+    }
+    if (lane < topk) {
+        ids[static_cast<size_t>(warp) * topk + place] = my_id;
+        scores[static_cast<size_t>(warp) * topk + place] = renorm ? my_p / psum : my_p;
     }
 }
 
 // ------------------------------------------------------------------------------------------------ permute
 __global__ void moe_count_kernel(const int32_t* __restrict__ eid, int R, int E, int32_t* __restrict__ counts, int32_t* status) {
+    dependent_start();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= R) return;
     const int e = eid[r];
@@ -160,6 +197,7 @@ __device__ __forceinline__ int2 scan_experts(const int32_t* cnt, int E, int bloc
 __global__ void moe_plan_kernel(const int32_t* __restrict__ counts, int E, int block_rows, int32_t* __restrict__ offsets,
                                 int32_t* __restrict__ cursor, RowBlock* __restrict__ blocks, int32_t* __restrict__ n_blocks,
                                 int max_blocks) {
+    dependent_start();
     extern __shared__ int32_t sh[];  // [E] counts -> offsets, [E] block offsets
     int32_t* off = sh;
     int32_t* boff = sh + E;
@@ -196,6 +234,7 @@ __global__ void moe_plan_kernel(const int32_t* __restrict__ counts, int E, int b
 __global__ void moe_scatter_kernel(const int32_t* __restrict__ eid, const int32_t* __restrict__ src_row, int R, int E,
                                    const int32_t* __restrict__ offsets, int32_t* __restrict__ cursor, int32_t* __restrict__ src_of,
                                    int32_t* __restrict__ dst_of, int src_div) {
+    dependent_start();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= R) return;
     const int e = eid[r];
@@ -210,6 +249,7 @@ constexpr int kSmallPlanRows = 8192;
 __global__ void moe_plan_small_kernel(const int32_t* __restrict__ eid, const int32_t* __restrict__ src_row, int src_div, int R, int E, int block_rows,
                                       int32_t* __restrict__ offsets, RowBlock* __restrict__ blocks, int32_t* __restrict__ n_blocks, int max_blocks,
                                       int32_t* __restrict__ src_of, int32_t* __restrict__ dst_of, int32_t* __restrict__ status) {
+    dependent_start();
     extern __shared__ int32_t sh[];  // counts -> cursors [E], offsets [E], block offsets [E]
     int32_t* cnt = sh;
     int32_t* off = sh + E;
@@ -262,6 +302,7 @@ __global__ void moe_plan_small_kernel(const int32_t* __restrict__ eid, const int
 // xp[pos][:] = x[src_of[pos]][:], 16 bytes per thread.
 __global__ void moe_gather_rows_kernel(const uint4* __restrict__ x, const int32_t* __restrict__ src_of, const int32_t* __restrict__ total_rows,
                                        int row_vec, uint4* __restrict__ xp) {
+    dependent_start();
     // a grid-stride loop over the rows that exist: the row list of an expert-parallel receive buffer is mostly empty
     // slots (world x capacity), and a thread per slot would launch hundreds of thousands of CTAs that only return
     const int64_t total = static_cast<int64_t>(*total_rows) * row_vec;
@@ -334,6 +375,7 @@ __global__ void moe_swiglu_kernel(const ActT* __restrict__ gu, const int32_t* __
 template <typename ActT>
 __global__ void moe_combine_kernel(const ActT* __restrict__ out_rows, const float* __restrict__ scores, int T, int topk, int H,
                                    ActT* __restrict__ y) {
+    dependent_start();
     const int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (idx >= static_cast<int64_t>(T) * H) return;
     const int64_t t = idx / H, hcol = idx % H;
@@ -350,6 +392,7 @@ __global__ void moe_combine_kernel(const ActT* __restrict__ out_rows, const floa
 template <typename ActT>
 __global__ void moe_combine_vec_kernel(const uint4* __restrict__ out_rows, const float* __restrict__ scores, int T, int topk, int H8,
                                        uint4* __restrict__ y) {
+    dependent_start();
     const int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (idx >= static_cast<int64_t>(T) * H8) return;
     const int64_t t = idx / H8, c = idx - t * H8;
@@ -446,31 +489,28 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
     const bool tensor = tensor_path(R, E), streamable = moe_stream_fits(w.max_blocks, 2 * I) && moe_stream_fits(w.max_blocks, H);
     const bool tmem = tensor || (R >= (streamable ? tmem_rows_per_expert(E, H, I) : 3) * E && aligned(x, 16) && aligned(out, 16));
     const int br = tmem && !tensor ? 16 : block_rows_for(R, E);
+    int st = EQ_OK;
     if (R <= kSmallPlanRows) {
-        moe_plan_small_kernel<<<1, 1024, 3 * E * sizeof(int32_t), stream>>>(eid, src_row, src_div, static_cast<int>(R), static_cast<int>(E), br, w.offsets,
-                                                                            w.blocks, w.n_blocks, w.max_blocks, w.src_of, w.dst_of, w.status);
-        EQ_LAUNCH_OK("moe_plan_small_kernel");
-    } else {
-        EQ_CUDA_OK(cudaMemsetAsync(w.counts, 0, E * 4, stream));
-        moe_count_kernel<<<static_cast<unsigned>(ceil_div(R, 256)), 256, 0, stream>>>(eid, static_cast<int>(R), static_cast<int>(E), w.counts, w.status);
-        EQ_LAUNCH_OK("moe_count_kernel");
-        moe_plan_kernel<<<1, 256, 2 * E * sizeof(int32_t), stream>>>(w.counts, static_cast<int>(E), br, w.offsets, w.cursor, w.blocks, w.n_blocks,
-                                                                     w.max_blocks);
-        EQ_LAUNCH_OK("moe_plan_kernel");
-        moe_scatter_kernel<<<static_cast<unsigned>(ceil_div(R, 256)), 256, 0, stream>>>(eid, src_row, static_cast<int>(R), static_cast<int>(E), w.offsets,
-                                                                                      w.cursor, w.src_of, w.dst_of, src_div);
-        EQ_LAUNCH_OK("moe_scatter_kernel");
+        st = launch_dependent(moe_plan_small_kernel, 1, 1024, 3 * E * sizeof(int32_t), stream, eid, src_row, src_div, R, E, br, w.offsets, w.blocks,
+                              w.n_blocks, w.max_blocks, w.src_of, w.dst_of, w.status);
+    } else {  // (w.counts has been cleared)
+        st = launch_dependent(moe_count_kernel, ceil_div(R, 256), 256, 0, stream, eid, R, E, w.counts, w.status);
+        if (st == EQ_OK)
+            st = launch_dependent(moe_plan_kernel, 1, 256, 2 * E * sizeof(int32_t), stream, w.counts, E, br, w.offsets, w.cursor, w.blocks, w.n_blocks, w.max_blocks);
+        if (st == EQ_OK)
+            st = launch_dependent(moe_scatter_kernel, ceil_div(R, 256), 256, 0, stream, eid, src_row, R, E, w.offsets, w.cursor, w.src_of, w.dst_of, src_div);
     }
+    if (st != EQ_OK) return st;
     if (tmem) {
         // rows into expert order (the region of the second GEMM's output in the workspace is free until then)
         const int act = sizeof(ActT) == 2 && std::is_same<ActT, __half>::value ? EQ_F16 : EQ_BF16;
         const int row_vec = static_cast<int>(H * 2 / 16);
         EQ_REQUIRE(aligned(x, 16) && aligned(out, 16), EQ_ERR_BAD_ALIGN, "grouped expert GEMM: activations and outputs must be 16-byte aligned");
         const int64_t gather_ctas = ceil_div(R * row_vec, 256);
-        moe_gather_rows_kernel<<<static_cast<unsigned>(gather_ctas < 32LL * sm_count() ? gather_ctas : 32LL * sm_count()), 256, 0, stream>>>(
-            static_cast<const uint4*>(x), w.src_of, w.offsets + E, row_vec, reinterpret_cast<uint4*>(w.out));
-        EQ_LAUNCH_OK("moe_gather_rows_kernel");
-        int st = w4_tmem_grouped_launch(static_cast<const unsigned char*>(wq_gate_up), static_cast<size_t>(2 * I / 16) * (H / 128) * kItemBytes, scale_dtype,
+        st = launch_dependent(moe_gather_rows_kernel, gather_ctas < 32LL * sm_count() ? gather_ctas : 32LL * sm_count(), 256, 0, stream,
+                              static_cast<const uint4*>(x), w.src_of, w.offsets + E, row_vec, reinterpret_cast<uint4*>(w.out));
+        if (st != EQ_OK) return st;
+        st = w4_tmem_grouped_launch(static_cast<const unsigned char*>(wq_gate_up), static_cast<size_t>(2 * I / 16) * (H / 128) * kItemBytes, scale_dtype,
                                         w.out, w.h, R, 2 * I, H, act, w.blocks, w.n_blocks, br, nullptr, true, w.status, stream);
         if (st != EQ_OK) return st;
         return w4_tmem_grouped_launch(static_cast<const unsigned char*>(wq_down), static_cast<size_t>(H / 16) * (I / 128) * kItemBytes, scale_dtype, w.h,
@@ -478,7 +518,7 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
     }
     if (streamable) {
         const int act = std::is_same<ActT, __half>::value ? EQ_F16 : EQ_BF16;
-        int st = moe_stream_launch(static_cast<const unsigned char*>(wq_gate_up), static_cast<size_t>(2 * I / 16) * (H / 128) * kItemBytes, scale_dtype,
+        st = moe_stream_launch(static_cast<const unsigned char*>(wq_gate_up), static_cast<size_t>(2 * I / 16) * (H / 128) * kItemBytes, scale_dtype,
                                    x, w.h1, w.src_of, nullptr, nullptr, w.blocks, w.n_blocks, w.max_blocks, H, 2 * I, act, stream);
         if (st != EQ_OK) return st;
         moe_swiglu_kernel<ActT><<<static_cast<unsigned>(ceil_div(R * I, 256)), 256, 0, stream>>>(reinterpret_cast<const ActT*>(w.h1), w.offsets + E,
@@ -499,7 +539,7 @@ static int experts_forward(const MoeWorkspace& w, const void* wq_gate_up, const 
     g1.K = static_cast<int>(H);
     g1.N = static_cast<int>(2 * I);
     g1.scale_dtype = scale_dtype;
-    int st = launch_grouped<ActT>(g1, w.max_blocks, stream);
+    st = launch_grouped<ActT>(g1, w.max_blocks, stream);
     if (st != EQ_OK) return st;
     moe_swiglu_kernel<ActT><<<static_cast<unsigned>(ceil_div(R * I, 256)), 256, 0, stream>>>(reinterpret_cast<const ActT*>(w.h1), w.offsets + E,
                                                                                           static_cast<int>(I), reinterpret_cast<ActT*>(w.h));
@@ -755,15 +795,18 @@ static int check_moe_shapes(const char* who, int64_t E, int64_t topk, int64_t H,
 
 using namespace eq;
 
-extern "C" int eq_moe_route(const float* logits, int64_t T, int64_t E, int64_t topk, int renorm, int32_t* ids, float* scores, void* stream) {
+static int moe_route(const float* logits, int64_t T, int64_t E, int64_t topk, int renorm, int32_t* ids, float* scores, int32_t* status, int32_t* counts,
+                     cudaStream_t stream) {
     EQ_REQUIRE(T >= 0 && E > 0 && E <= 1024 && topk > 0 && topk <= kMaxTopK && topk <= E, EQ_ERR_UNSUPPORTED,
                "eq_moe_route: needs 0 < top-k <= 16 and E <= 1024");
     if (T == 0) return EQ_OK;
     EQ_REQUIRE(logits && ids && scores, EQ_ERR_BAD_ARG, "eq_moe_route: null pointer");
-    moe_route_kernel<<<static_cast<unsigned>(ceil_div(T * 32, 256)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        logits, static_cast<int>(T), static_cast<int>(E), static_cast<int>(topk), renorm, ids, scores);
-    EQ_LAUNCH_OK("moe_route_kernel");
-    return EQ_OK;
+    auto run = [&](auto kernel) { return launch_dependent(kernel, ceil_div(T * 32, 256), 256, 0, stream, logits, T, E, topk, renorm, ids, scores, status, counts); };
+    return E <= 64 ? run(moe_route_kernel<2>) : E <= 128 ? run(moe_route_kernel<4>) : E <= 256 ? run(moe_route_kernel<8>) : run(moe_route_kernel<32>);
+}
+
+extern "C" int eq_moe_route(const float* logits, int64_t T, int64_t E, int64_t topk, int renorm, int32_t* ids, float* scores, void* stream) {
+    return moe_route(logits, T, E, topk, renorm, ids, scores, nullptr, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" size_t eq_moe_workspace_bytes(int64_t T, int64_t E, int64_t topk, int64_t H, int64_t I) {
@@ -784,6 +827,7 @@ extern "C" int eq_moe_experts_w4a16(const void* wq_gate_up, const void* wq_down,
                "eq_moe_experts_w4a16: workspace of %zu bytes (256-byte aligned) needed, %zu given", eq_moe_workspace_bytes(R, E, 1, H, I), workspace_bytes);
     MoeWorkspace w = carve(workspace, R, E, 1, H, I);
     EQ_CUDA_OK(cudaMemsetAsync(w.status, 0, 4, stream));
+    if (R > kSmallPlanRows) EQ_CUDA_OK(cudaMemsetAsync(w.counts, 0, E * 4, stream));
     if (act_dtype == EQ_F16)
         return experts_forward<__half>(w, wq_gate_up, wq_down, scale_dtype, E, H, I, x, src_row, 0, expert_ids, R, out, stream);
     return experts_forward<__nv_bfloat16>(w, wq_gate_up, wq_down, scale_dtype, E, H, I, x, src_row, 0, expert_ids, R, out, stream);
@@ -797,22 +841,17 @@ extern "C" int eq_moe_combine(const void* out_rows, const float* scores, int64_t
     EQ_REQUIRE(act_dtype == EQ_F16 || act_dtype == EQ_BF16, EQ_ERR_BAD_ARG, "eq_moe_combine: activations must be f16 or bf16");
     const int Ti = static_cast<int>(T), ki = static_cast<int>(topk), Hi = static_cast<int>(H);
     if (H % 8 == 0 && aligned(out_rows, 16) && aligned(y, 16)) {
-        const unsigned grid = static_cast<unsigned>(ceil_div(T * (H / 8), 256));
-        if (act_dtype == EQ_F16)
-            moe_combine_vec_kernel<__half><<<grid, 256, 0, stream>>>(static_cast<const uint4*>(out_rows), scores, Ti, ki, Hi / 8, static_cast<uint4*>(y));
-        else
-            moe_combine_vec_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(static_cast<const uint4*>(out_rows), scores, Ti, ki, Hi / 8,
-                                                                            static_cast<uint4*>(y));
-    } else {
-        const unsigned grid = static_cast<unsigned>(ceil_div(T * H, 256));
-        if (act_dtype == EQ_F16)
-            moe_combine_kernel<__half><<<grid, 256, 0, stream>>>(static_cast<const __half*>(out_rows), scores, Ti, ki, Hi, static_cast<__half*>(y));
-        else
-            moe_combine_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(out_rows), scores, Ti, ki, Hi,
-                                                                        static_cast<__nv_bfloat16*>(y));
+        const int64_t grid = ceil_div(T * (H / 8), 256);
+        const uint4* rows = static_cast<const uint4*>(out_rows);
+        uint4* out = static_cast<uint4*>(y);
+        return act_dtype == EQ_F16 ? launch_dependent(moe_combine_vec_kernel<__half>, grid, 256, 0, stream, rows, scores, Ti, ki, Hi / 8, out)
+                                   : launch_dependent(moe_combine_vec_kernel<__nv_bfloat16>, grid, 256, 0, stream, rows, scores, Ti, ki, Hi / 8, out);
     }
-    EQ_LAUNCH_OK("moe_combine_kernel");
-    return EQ_OK;
+    const int64_t grid = ceil_div(T * H, 256);
+    if (act_dtype == EQ_F16)
+        return launch_dependent(moe_combine_kernel<__half>, grid, 256, 0, stream, static_cast<const __half*>(out_rows), scores, Ti, ki, Hi, static_cast<__half*>(y));
+    return launch_dependent(moe_combine_kernel<__nv_bfloat16>, grid, 256, 0, stream, static_cast<const __nv_bfloat16*>(out_rows), scores, Ti, ki, Hi,
+                            static_cast<__nv_bfloat16*>(y));
 }
 
 extern "C" int eq_moe_w4a16(const void* wq_gate_up, const void* wq_down, int scale_dtype, int64_t E, int64_t topk, int64_t H, int64_t I, int64_t G,
@@ -832,8 +871,7 @@ extern "C" int eq_moe_w4a16(const void* wq_gate_up, const void* wq_down, int sca
         // a handful of tokens: router + [gate | up] in one launch, SwiGLU + down + combine in a second one
         return moe_decode_launch(wq_gate_up, wq_down, scale_dtype, E, topk, H, I, x, router_logits, T, act_dtype, y, w.ids, w.scores, w.h1, w.out,
                                  reinterpret_cast<int*>(w.h), w.status, stream);
-    EQ_CUDA_OK(cudaMemsetAsync(w.status, 0, 4, stream));
-    st = eq_moe_route(router_logits, T, E, topk, 1, w.ids, w.scores, stream_);
+    st = moe_route(router_logits, T, E, topk, 1, w.ids, w.scores, w.status, w.counts, stream);
     if (st != EQ_OK) return st;
     if (act_dtype == EQ_F16)
         st = experts_forward<__half>(w, wq_gate_up, wq_down, scale_dtype, E, H, I, x, nullptr, static_cast<int>(topk), w.ids, R, w.out, stream);

@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
     const int items = a.K / 128, n_tiles = a.N / 16;
     const int col_tiles = SWIGLU ? (a.N / 32 + 3) / 4 : (n_tiles + 7) / 8;  // SWIGLU: four gate and four up tiles per CTA
     int units = a.units;
+    if constexpr (GROUPED) asm volatile("griddepcontrol.wait;" ::: "memory");  // the block list and the rows are of the grids before
     if constexpr (GROUPED) units = *a.n_blocks * col_tiles;
     if (static_cast<int>(blockIdx.x) >= units) return;  // the whole CTA, before any barrier exists
 
@@ -453,7 +454,7 @@ int launch(W4TmemArgs a, const void* x, int64_t x_rows, int scale_dtype, cudaStr
     attr[1].val.clusterDim.x = static_cast<unsigned>(SPLIT ? a.splits : 1);
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = GROUPED ? 0 : SPLIT ? 2 : 1;  // the grouped form reads a block list the previous kernel wrote
+    cfg.numAttrs = SPLIT ? 2 : 1;
     EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, map_x, a));
     return EQ_OK;
 }

@@ -43,6 +43,29 @@ def test_router_matches_oracle_and_breaks_ties_low():
     np.testing.assert_allclose(scores.sum(dim=1).cpu().numpy(), 1.0, rtol=1e-5)
 
 
+@pytest.mark.parametrize("e,k", [(1, 1), (33, 3), (64, 6), (65, 8), (128, 8), (129, 16), (256, 4), (257, 5), (1000, 16)])
+def test_router_at_its_register_counts(e, k):
+    """Expert counts where a lane keeps two, four, eight or thirty-two logits, with ties across lanes, both zeros, infinities below
+    the rest and a NaN, which is never picked.  Probabilities: two exponentials (2 ulp each), a sum of at most 37 roundings, two divisions: 2^-24 x 43 < 2.6e-6."""
+    from emmy_b200 import ops_moe as om
+
+    logits = torch.randn(70, e, generator=torch.Generator().manual_seed(e)) * 3
+    logits[1] = torch.randint(-1, 2, (e,), generator=torch.Generator().manual_seed(k)).float()
+    logits[2] = 0.0
+    logits[2, ::2] = -0.0
+    if e > k + 1:
+        logits[3, : e - k] = float("-inf")
+    ids, scores = om.moe_route(logits.cuda(), k)
+    ref_s, ref_i = omoe.route_softmax_topk(logits, k)
+    ref_i, order = ref_i.sort(dim=1)
+    np.testing.assert_array_equal(ids.cpu().numpy(), ref_i.numpy())
+    np.testing.assert_allclose(scores.cpu().numpy(), ref_s.gather(1, order).numpy(), rtol=2.6e-6, atol=0)
+    if e > k:
+        logits[4, 0] = float("nan")
+        with_nan = om.moe_route(logits.cuda(), k)[0][4].tolist()
+        assert with_nan == sorted((torch.sort(logits[4, 1:], descending=True, stable=True).indices[:k] + 1).tolist())
+
+
 def test_experts_grouped_ffn_matches_per_expert_eager():
     from emmy_b200 import ops_moe as om
 

@@ -28,7 +28,7 @@ namespace eq {
 
 int w4_stream_launch(const W4Params& p, int act_dtype, cudaStream_t stream, bool* fits);  // w4_stream.cu
 int w4_gemv1_launch(const unsigned char* wq, int scale_dtype, const int32_t* perm, const void* x, void* y, int64_t N, int64_t K,
-                    int act_dtype, uint32_t* xchg, int* status, cudaStream_t stream, bool* fits);  // w4_gemv1.cu
+                    int act_dtype, bool swiglu, uint32_t* xchg, int* status, cudaStream_t stream, bool* fits);  // w4_gemv1.cu
 int w4_gemm_tc_launch(const unsigned char* wq, int scale_dtype, const int32_t* perm, const void* x, void* y, int64_t M, int64_t N,
                       int64_t K, int act_dtype, void* gathered, int* status, cudaStream_t stream);  // w4_gemm.cu
 
@@ -183,7 +183,7 @@ extern "C" int eq_w4a16_linear(const void* wq, int scale_dtype, const int32_t* p
     if (M == 1) {
         // the decode step's GEMV; the workspace carries its sixteen-word hand-overs between neighbouring CTAs
         bool fits = false;
-        const int st = w4_gemv1_launch(static_cast<const unsigned char*>(wq), scale_dtype, perm, x, y, N, K, act_dtype,
+        const int st = w4_gemv1_launch(static_cast<const unsigned char*>(wq), scale_dtype, perm, x, y, N, K, act_dtype, false,
                                        reinterpret_cast<uint32_t*>(partial), status, stream, &fits);
         if (st != EQ_OK || fits) return st;
     }
@@ -219,7 +219,8 @@ extern "C" const char* eq_w4a16_kernel(int64_t M, int64_t N, int64_t K, int has_
 // ---- gate / up + SwiGLU in one call ---------------------------------------------------------------------------
 // h[M, I] = act(silu(x W_gate)) * (x W_up) for a [gate | up] weight (the two projections concatenated along N, as the
 // reference stores them: emmy/compiler/trace/huggingface.py:1663-1669, 2110-2141), with the eager form's two roundings.
-// M > 16: the tensor path with gate and up tiles side by side in a CTA and the activation in the epilogue; fewer rows: the
+// M > 16: the tensor path with gate and up tiles side by side in a CTA and the activation in the epilogue; one row: the GEMV with
+// gate and up tiles side by side; between, the
 // [gate | up] linear into scratch, then an elementwise pass.
 namespace eq {
 namespace {
@@ -302,6 +303,13 @@ extern "C" int eq_w4a16_gate_up_swiglu(const void* wq, int scale_dtype, const in
     }
     // few rows, scattered act-order groups or an unaligned output: the [gate | up] linear, then the activation
     EQ_REQUIRE(M <= 16, EQ_ERR_UNSUPPORTED, "eq_w4a16_gate_up_swiglu: M > 16 needs a 16-byte aligned output and a weight without a row permutation");
+    if (M == 1) {
+        // the GEMV with gate and up tiles side by side and the activation where a pair of them is complete
+        bool fits = false;
+        st = w4_gemv1_launch(static_cast<const unsigned char*>(wq), scale_dtype, perm, x, h, 2 * I, K, act_dtype, true,
+                             reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(workspace) + kW4Header), static_cast<int*>(workspace), stream, &fits);
+        if (st != EQ_OK || fits) return st;
+    }
     void* gu = extra;  // [M][2 I] scratch
     st = eq_w4a16_linear(wq, scale_dtype, perm, K, 2 * I, G, x, M, act_dtype, gu, workspace, inner, stream_);
     if (st != EQ_OK) return st;

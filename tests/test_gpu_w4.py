@@ -616,3 +616,33 @@ def test_linear_behind_a_kernel_that_takes_a_second(m, n):
     ops.w4a16_status(ws, m, n)
     assert int(state[:4].view(torch.int32)) == 70  # it did run into its limit
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("inter,k,order,dtype", [
+    (2352, 256, "none", "bf16"),     # fewer pairs of tiles than SMs: two launches
+    (2368, 128, "none", "f16"),      # one pair per CTA, spans end with their tiles
+    (2384, 384, "none", "bf16"),     # spans cut inside gate tiles and up tiles
+    (4720, 128, "none", "bf16"), (4736, 384, "none", "f16"), (4752, 128, "none", "bf16"),  # from two pairs per SM on: two CTAs each
+    (9488, 256, "none", "f16"), (3008, 1024, "scattered", "bf16"),
+])
+def test_gate_up_of_one_row_with_the_activation_in_the_gemv(inter, k, order, dtype):
+    """One row: gate and up tiles side by side in the GEMV, the activation where a pair is complete; the sums cross CTAs in the middle
+    of a gate or an up tile.  Twice on one workspace, which stays zero behind its header; the output may start anywhere."""
+    from emmy_b200 import ops
+
+    qw, qz, sc, _ = synth.gptq_linear(k, 2 * inter, seed=inter)
+    gi = np.random.default_rng(k).permutation(np.arange(k) // 128).astype(np.int32) if order == "scattered" else None
+    w = ops.w4_repack(dev(qw), dev(qz), dev(sc), 128, "gptq", g_idx=None if gi is None else dev(gi))
+    x = synth.activations(1, k, dtype, seed=k + inter)
+    rnd = fm.round_bf16 if dtype == "bf16" else fm.round_f16
+    g, u = np.split(rnd(ol.w4a16_linear(x, qw, qz, sc, 128, "gptq", dtype, gi)), 2, axis=1)
+    ref = rnd(rnd(g / (np.float32(1) + np.exp(-g, dtype=np.float32))) * u)
+    lib = ops.L.load()
+    ws = torch.zeros(lib.eq_w4a16_gate_up_workspace_bytes(1, inter, k) + 256, dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        h = ops.w4a16_gate_up_swiglu(act(x, dtype), w, workspace=ws)
+        ops.w4a16_status(ws, 1, 2 * inter)
+        check_close(h, ref)
+    assert int(ws[256 : lib.eq_w4a16_workspace_bytes(1, 2 * inter, k)].count_nonzero()) == 0
+    odd = torch.empty(inter + 1, dtype=h.dtype, device="cuda")[1:].view(1, inter)
+    check_close(ops.w4a16_gate_up_swiglu(act(x, dtype), w, workspace=ws, out=odd), ref)

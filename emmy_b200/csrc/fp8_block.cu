@@ -10,12 +10,13 @@
 //                            rule of fp8_linear.cu applied per 128-element group; one warp per group.  Inside the linear
 //                            it also clears the status word and lets the kernel behind it start early.
 //   fp8_block_tc.cu          tcgen05 with a fresh accumulator per K block and promotion in registers: a swapped-operand
-//                            decode tile for M <= 16, 128 x 128 tiles up to 128 rows, 128 x 256 tiles above
+//                            decode tile for M <= 16, 128 x 128 tiles up to 128 rows or one wave, 128 x 256 tiles above
 //   fp8_block_gemm_kernel    the mma.sync form, kept for an output that is not 16-byte aligned: 128 x 128 output tile per
 //                            CTA, K in steps of one scale block, operand tiles by cp.async into XOR-swizzled shared
 //                            memory (two stages), fragments by ldmatrix, products by mma.sync m16n8k32 e4m3 into a
 //                            per-block accumulator that is folded into the running f32 sum with the block's two scales.
 #include "common.cuh"
+#include "quant.cuh"
 
 namespace eq {
 
@@ -56,6 +57,31 @@ __global__ void __launch_bounds__(256) quant_fp8_groups_kernel(const InT* __rest
     if (lane == 0) scale[gw] = s;
     const uint32_t lo = e4m3x2_sat(__fdiv_rn(v[0], s), __fdiv_rn(v[1], s)), hi = e4m3x2_sat(__fdiv_rn(v[2], s), __fdiv_rn(v[3], s));
     *reinterpret_cast<uint32_t*>(q + gw * 128 + lane * 4) = lo | (hi << 16);
+}
+
+// The same for large calls of 16-bit activations at a 16-byte aligned address: sixteen lanes per group, eight elements a lane, two vectors
+// in flight per thread.  `vecs` = M * K / 8, a multiple of 16.
+template <typename InT>
+__global__ void __launch_bounds__(256) quant_fp8_groups_vec_kernel(const uint4* __restrict__ x, int64_t vecs, uint2* __restrict__ q, float* __restrict__ scale,
+                                                                   int* __restrict__ status) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+    const int64_t first = blockIdx.x * int64_t(512) + threadIdx.x;
+    uint4 raw[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) raw[u] = first + 256 * u < vecs ? __ldg(x + first + 256 * u) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        float amax = quant::abs_max8<InT>(raw[u]);
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, off));
+        const int64_t at = first + 256 * u;
+        if (at >= vecs) continue;  // whole groups
+        const float s = __fdiv_rn(fmaxf(amax, 1e-12f), 448.0f);
+        if ((threadIdx.x & 15) == 0) scale[at >> 4] = s;
+        q[at] = quant::e4m3_codes8<InT>(raw[u], s);
+    }
 }
 
 constexpr int kBB = 128;             // tile edge = scale block edge
@@ -210,6 +236,17 @@ static int quant_fp8_groups(const void* x, int64_t M, int64_t K, int in_dtype, u
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = (status && M <= 128) ? 1 : 0;  // decode-sized calls inside the linear: resident when the kernel before it ends
+    // From 4 M elements on: below, the kernel of one warp per group has the shorter chain (us a linear, N=17408: 65 rows of 5120 22.2
+    // against 23.4, 300 rows 53.8 : 54.7, 2048 rows 237 : 233, 8192 rows 920 : 896).
+    if (M * K >= 4000000 && in_dtype != EQ_F32 && aligned(x, 16) && aligned(q, 8)) {
+        const int64_t vecs = M * K / 8;
+        cfg.gridDim = dim3(static_cast<unsigned>(ceil_div(vecs, 512)));
+        const uint4* xv = static_cast<const uint4*>(x);
+        uint2* qv = reinterpret_cast<uint2*>(q);
+        if (in_dtype == EQ_F16) EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_fp8_groups_vec_kernel<__half>, xv, vecs, qv, scale, status));
+        else EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_fp8_groups_vec_kernel<__nv_bfloat16>, xv, vecs, qv, scale, status));
+        return EQ_OK;
+    }
     switch (in_dtype) {
         case EQ_F16: EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_fp8_groups_kernel<__half>, static_cast<const __half*>(x), M, K, q, scale, status)); break;
         case EQ_BF16: EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_fp8_groups_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(x), M, K, q, scale, status)); break;
@@ -246,7 +283,7 @@ extern "C" int eq_fp8_block_linear(const uint8_t* weight, const float* weight_sc
     int* status = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(sx) + blk_align(static_cast<size_t>(M) * (K / 128) * sizeof(float)));
     int st = quant_fp8_groups(x, M, K, act_dtype, qx, sx, status, stream);
     if (st != EQ_OK) return st;
-    // the tensor cores (fp8_block_tc.cu: swapped-operand decode tile up to 16 rows, 128-column tiles up to 128 rows, 256-column
+    // the tensor cores (fp8_block_tc.cu: swapped-operand decode tile up to 16 rows, 128-column tiles up to 128 rows or one wave, 256-column
     // tiles above); the mma.sync tile kernel below serves an unaligned y
     if (M <= 16 || aligned(y, 16)) return fp8_block_tc_launch(qx, sx, weight, weight_scale, y, M, N, K, act_dtype, status, stream);
     const dim3 grid(static_cast<unsigned>(N / kBB), static_cast<unsigned>(ceil_div(M, kBB)));

@@ -3,8 +3,8 @@
 //   quant_fp8_rows_kernel   x[M,K] f16/bf16/f32 -> e4m3 bits + one f32 scale per row.  s = max(amax, 1e-12) / 448
 //                           and q = e4m3_rne_satfinite(x / s), both with round-to-nearest f32 division: bit-exact
 //                           against the numpy rule the reference spells (emmy/compiler/loader/quant.py:1655-1735).
-//   quant_fp8_rows_vec_kernel  the same for few rows (decode): one 1024-thread CTA per row, the row held in registers
-//                           between the maximum and the encode, 16-byte loads; also clears the status word.
+//   quant_fp8_rows_vec_kernel  the same for aligned rows: the row held in registers between the maximum and the encode,
+//                           16-byte loads; also clears the status word.
 //   fp8_decode_tc_kernel    M <= 16 (decode-shaped): tcgen05 with the operands' roles swapped -- 128-channel weight tiles
 //                           are the MMA's A operand, the rows its B operand with N = 16 -- so one TMA thread streams the
 //                           weight, 108 KB CTAs of two consecutive launches share an SM, and the weights are requested
@@ -19,6 +19,7 @@
 #include <type_traits>
 
 #include "gemm_pair.cuh"
+#include "quant.cuh"
 #include "tc_common.cuh"
 
 namespace eq {
@@ -380,17 +381,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
 }
 
-// Few rows (decode): one CTA of 1024 threads per row; the row stays in registers between the two passes.
-// kVecs 16-byte vectors per thread cover K <= 1024 * kVecs * (16 / sizeof(InT)) elements.
-template <typename InT, int kVecs>
-__global__ void __launch_bounds__(1024) quant_fp8_rows_vec_kernel(const InT* __restrict__ x, int64_t K, uint8_t* __restrict__ q,
+// One CTA per row, 16-byte loads; the row stays in registers between the two passes.  1024 threads for few rows (decode: latency),
+// 256 for many (K=5120 N=17408, us a linear, against two passes of 2-byte loads behind a memset: 100 rows 29.8 -> 23.9, 300 rows 52.6 ->
+// 41.3, 2048 rows 168 -> 153).  kVecs vectors per thread cover K <= kRowThreads * kVecs * (16 / sizeof(InT)) elements.
+template <typename InT, int kVecs, int kRowThreads>
+__global__ void __launch_bounds__(kRowThreads) quant_fp8_rows_vec_kernel(const InT* __restrict__ x, int64_t K, uint8_t* __restrict__ q,
                                                                   float* __restrict__ scale, int* __restrict__ status) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the linear behind this may start fetching weights
     // launched as a programmatic dependent itself: the kernel before it (usually the previous linear on this workspace)
     // may still read the codes, scales and status word this one rewrites
     asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int kPer = 16 / sizeof(InT);  // elements per 16-byte vector
-    __shared__ float warp_max[32];
+    __shared__ float warp_max[kRowThreads / 32];
     __shared__ float row_scale;
     const int64_t row = blockIdx.x;
     if (status && row == 0 && threadIdx.x == 0) *status = 0;
@@ -400,19 +402,23 @@ __global__ void __launch_bounds__(1024) quant_fp8_rows_vec_kernel(const InT* __r
     float amax = 0.f;
 #pragma unroll
     for (int u = 0; u < kVecs; ++u) {
-        const int idx = threadIdx.x + u * 1024;
+        const int idx = threadIdx.x + u * kRowThreads;
         v[u] = make_uint4(0, 0, 0, 0);
         if (idx < n_vec) v[u] = __ldg(xr + idx);
-        const InT* e = reinterpret_cast<const InT*>(&v[u]);
+        if constexpr (kPer == 8) {
+            amax = fmaxf(amax, quant::abs_max8<InT>(v[u]));
+        } else {
+            const InT* e = reinterpret_cast<const InT*>(&v[u]);
 #pragma unroll
-        for (int i = 0; i < kPer; ++i) amax = fmaxf(amax, fabsf(to_float(e[i])));
+            for (int i = 0; i < kPer; ++i) amax = fmaxf(amax, fabsf(to_float(e[i])));
+        }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, off));
     if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = amax;
     __syncthreads();
     if (threadIdx.x < 32) {
-        float m = warp_max[threadIdx.x];
+        float m = threadIdx.x < kRowThreads / 32 ? warp_max[threadIdx.x] : 0.f;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, off));
         if (threadIdx.x == 0) {
@@ -426,16 +432,22 @@ __global__ void __launch_bounds__(1024) quant_fp8_rows_vec_kernel(const InT* __r
     uint8_t* qr = q + row * K;
 #pragma unroll
     for (int u = 0; u < kVecs; ++u) {
-        const int idx = threadIdx.x + u * 1024;
+        const int idx = threadIdx.x + u * kRowThreads;
         if (idx < n_vec) {
-            const InT* e = reinterpret_cast<const InT*>(&v[u]);
-            uint16_t out[kPer / 2];
+            if constexpr (kPer == 8 && kRowThreads < 1024) {
+                *reinterpret_cast<uint2*>(qr + static_cast<size_t>(idx) * kPer) = quant::e4m3_codes8<InT>(v[u], s);
+            } else if constexpr (kPer == 8) {  // few rows: latency, where the divisions are the shorter chain (32 rows 20.5 against 20.7 us a linear)
+                const InT* e = reinterpret_cast<const InT*>(&v[u]);
+                uint16_t out[kPer / 2];
 #pragma unroll
-            for (int i = 0; i < kPer / 2; ++i) out[i] = e4m3x2_satfinite(__fdiv_rn(to_float(e[2 * i]), s), __fdiv_rn(to_float(e[2 * i + 1]), s));
-            if constexpr (kPer == 8)
+                for (int i = 0; i < kPer / 2; ++i) out[i] = e4m3x2_satfinite(__fdiv_rn(to_float(e[2 * i]), s), __fdiv_rn(to_float(e[2 * i + 1]), s));
                 *reinterpret_cast<uint2*>(qr + static_cast<size_t>(idx) * kPer) = *reinterpret_cast<const uint2*>(out);
-            else
-                *reinterpret_cast<uint32_t*>(qr + static_cast<size_t>(idx) * kPer) = *reinterpret_cast<const uint32_t*>(out);
+            } else {
+                const InT* e = reinterpret_cast<const InT*>(&v[u]);
+                const uint32_t a = e4m3x2_satfinite(__fdiv_rn(to_float(e[0]), s), __fdiv_rn(to_float(e[1]), s));
+                const uint32_t b = e4m3x2_satfinite(__fdiv_rn(to_float(e[2]), s), __fdiv_rn(to_float(e[3]), s));
+                *reinterpret_cast<uint32_t*>(qr + static_cast<size_t>(idx) * kPer) = a | (b << 16);
+            }
         }
     }
 }
@@ -462,21 +474,30 @@ using namespace eq;
 template <typename InT>
 static int quant_rows_launch(const InT* x, int64_t M, int64_t K, uint8_t* q, float* scale, int* status, cudaStream_t stream) {
     constexpr int kPer = 16 / sizeof(InT);
-    const bool vec = M <= 64 && K % kPer == 0 && aligned(x, 16) && aligned(q, 8) && K / kPer <= 4 * 1024;
+    const bool vec = K % kPer == 0 && aligned(x, 16) && aligned(q, 8) && K / kPer <= 4 * 1024;
     if (vec) {
+        const int64_t n_vec = K / kPer;
+        const bool few = M <= 64 || n_vec > 8 * 256;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(M));
-        cfg.blockDim = dim3(1024);
+        cfg.blockDim = dim3(few ? 1024 : 256);
         cfg.stream = stream;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // resident, past its launch latency, when the kernel before it ends
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if (K / kPer <= 1024) EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_fp8_rows_vec_kernel<InT, 1>, x, K, q, scale, status));
-        else if (K / kPer <= 2048) EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_fp8_rows_vec_kernel<InT, 2>, x, K, q, scale, status));
-        else EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_fp8_rows_vec_kernel<InT, 4>, x, K, q, scale, status));
-        return EQ_OK;
+        auto run = [&](auto kernel) -> int {
+            EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, x, K, q, scale, status));
+            return EQ_OK;
+        };
+        if (!few)
+            return n_vec <= 512    ? run(quant_fp8_rows_vec_kernel<InT, 2, 256>)
+                   : n_vec <= 1024 ? run(quant_fp8_rows_vec_kernel<InT, 4, 256>)
+                                   : run(quant_fp8_rows_vec_kernel<InT, 8, 256>);
+        return n_vec <= 1024   ? run(quant_fp8_rows_vec_kernel<InT, 1, 1024>)
+               : n_vec <= 2048 ? run(quant_fp8_rows_vec_kernel<InT, 2, 1024>)
+                               : run(quant_fp8_rows_vec_kernel<InT, 4, 1024>);
     }
     if (status) EQ_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), stream));
     quant_fp8_rows_kernel<InT><<<static_cast<unsigned>(M), 256, 0, stream>>>(x, K, q, scale);

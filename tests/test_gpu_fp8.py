@@ -178,6 +178,16 @@ def test_rmsnorm_inside_the_quantize(m):
 @pytest.mark.parametrize("m", [17, 128, 129, 256, 257, 300, 400])
 @pytest.mark.parametrize("n,k,dtype", [(128, 128, "bf16"), (384, 640, "f16"), (512, 1024, "bf16")])
 def test_block_scaled_at_tile_edges(m, n, k, dtype):
+    _check_block_scaled(m, n, k, dtype)
+
+
+@pytest.mark.parametrize("m,n,dtype", [(129, 9472, "bf16"), (129, 9600, "f16"), (500, 4736, "f16"), (500, 4864, "bf16")])
+def test_block_scaled_on_both_sides_of_one_wave(m, n, dtype):
+    """128 x 128 tiles fill at most one wave of 148 SMs, or one tile column more than that (256-column tiles)."""
+    _check_block_scaled(m, n, 384, dtype)
+
+
+def _check_block_scaled(m, n, k, dtype):
     """Block-scaled FP8 where the kernel changes form (128-column tiles up to 128 rows, 256-column tiles above) and where
     tiles are partial (a last row tile of one row, an odd number of row tiles, half a column tile, one K block).  Against the same codes
     and scales in 64 bits: the output's rounding (2^-8 bf16, 2^-11 f16, relative) and the f32 sums over K (2^-24 K)."""
@@ -196,3 +206,51 @@ def test_block_scaled_at_tile_edges(m, n, k, dtype):
     y = ops.fp8_block_linear(xd, dev(bits.reshape(n, k)), dev(s)).float().cpu().numpy()
     u = 2.0**-8 if dtype == "bf16" else 2.0**-11
     assert (np.abs(y - ref) <= u * np.abs(ref) + 2.0**-24 * k * np.abs(ref).max()).all()
+
+
+def _awkward(m, k, dtype):
+    """Rows whose quotients fall on rounding boundaries (amax = 1.75 x a power of two: x / scale = x times a power of two), zero
+    rows, denormals, infinities and NaNs among ordinary ones."""
+    t = torch.randn(m, k, generator=torch.Generator().manual_seed(m + k)) * 3
+    t[0] = (torch.randint(-224, 225, (k,), generator=torch.Generator().manual_seed(k)) / 128)
+    t[0, :2] = 1.75
+    t[1] = 0.0
+    t[2, 5], t[3, 7], t[4, 9 % k] = float("inf"), float("-inf"), float("nan")
+    t[5] *= 1e-6
+    t[6] *= 1e3
+    return t.to(torch.bfloat16 if dtype == "bf16" else torch.float16)
+
+
+def _unaligned(t):
+    """The same values at an address that only the element-wise kernels take."""
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")
+    buf[1:].copy_(t.flatten())
+    return buf[1:].view(t.shape)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("m,k", [(64, 256), (65, 8), (65, 4096), (70, 4104), (65, 8192), (65, 8200), (65, 16384), (65, 16392), (7, 32768)])
+def test_activation_quant_vector_kernel_equals_the_element_wise_one(m, k, dtype):
+    """Where the vector kernel changes its form (64 rows, 4096, 8192 and 16384 elements a row): the codes without a division per
+    element are those of the division, whatever the values."""
+    from emmy_b200 import ops
+
+    t = _awkward(m, k, dtype).cuda()
+    q, s = ops.quant_fp8_per_token(t)
+    rq, rs = ops.quant_fp8_per_token(_unaligned(t))
+    assert torch.equal(s, rs) and torch.equal(q, rq)
+    ordinary = torch.cat([t[:2], t[5:]]).float().cpu().numpy()
+    oq, os_ = oact.fp8_dynamic_per_token(ordinary)
+    np.testing.assert_array_equal(torch.cat([q[:2], q[5:]]).cpu().numpy(), oq)
+    np.testing.assert_array_equal(torch.cat([s[:2], s[5:]]).cpu().numpy(), os_)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("m,k", [(7, 128), (31251, 128), (6251, 640), (799, 5120), (1001, 4096)])
+def test_group_quant_vector_kernel_equals_the_element_wise_one(m, k, dtype):
+    from emmy_b200 import ops
+
+    t = _awkward(m, k, dtype).cuda()
+    q, s = ops.quant_fp8_per_group(t)
+    rq, rs = ops.quant_fp8_per_group(_unaligned(t))
+    assert torch.equal(s, rs) and torch.equal(q, rq)

@@ -199,3 +199,30 @@ def test_rmsnorm_inside_the_quantize(m):
     got = y.float().cpu().numpy()
     assert np.isfinite(got).all()
     assert np.abs(got - ref).max() <= 2e-2 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("m,k", [(7, 256), (33, 512), (127, 256), (128, 768), (129, 256), (300, 1280)])
+def test_activation_quant_inside_the_linear_equals_the_standalone_one(m, k, dtype):
+    """The linear quantizes into its workspace (codes, then scale atoms) one atom per CTA, without a division per element: the
+    same bytes as eq_quant_nvfp4_act's, on ordinary values and on ones that fall on rounding boundaries, zeros, infinities and NaNs."""
+    from emmy_b200 import ops_nvfp4 as o4
+
+    t = torch.randn(m, k, generator=torch.Generator().manual_seed(m)) * 2
+    t[0] = torch.randint(-24, 25, (k,), generator=torch.Generator().manual_seed(k)) / 4
+    t[1] = 0.0
+    t[2, 3], t[3, 4], t[4, 5] = float("inf"), float("-inf"), float("nan")
+    t[5] *= 1e-5
+    t = t.to(torch.bfloat16 if dtype == "bf16" else torch.float16).cuda()
+    packed, sbits, s2w = synth.nvfp4_weight(64, k, seed=1)
+    for s2 in (0.0025, 1.0 / 6, 1.0):
+        scale = torch.tensor([s2], device="cuda")
+        ws = o4.nvfp4_workspace(m, k, t.device)
+        o4.nvfp4_linear(t, dev(packed), o4.nvfp4_tile_weight_scales(dev(sbits), k), dev(s2w), scale, workspace=ws)
+        codes, sf = o4.quant_nvfp4_act(t, scale)
+        got = ws.cpu().numpy()
+        np.testing.assert_array_equal(got[: m * k // 2].reshape(m, k // 2), codes.cpu().numpy())
+        at = (m * k // 2 + 255) // 256 * 256
+        rows, blocks = np.meshgrid(np.arange(m), np.arange(k // 16), indexing="ij")
+        off = ((rows // 128) * (k // 64) + blocks // 4) * 512 + (rows % 32) * 16 + ((rows % 128) // 32) * 4 + blocks % 4
+        np.testing.assert_array_equal(got[at + off], sf.cpu().numpy())

@@ -25,10 +25,12 @@ constexpr int kBM = 128, kBK = 128;
 constexpr int kTileA = kBM * kBK;
 
 // BN = 256: two weight scale blocks per CTA, eight promotion warps, four 48 KB stages, all of TMEM.  BN = 128 (calls of
-// at most 128 rows, where the grid is one row of CTAs): twice as many CTAs stream the weight, six 32 KB stages.
+// at most 128 rows or one wave of such tiles): twice as many CTAs stream the weight, six 32 KB stages.
 //
 // The promotion bounds the kernel: a K block takes about 1050 cycles against 512 of MMA (128 x 256 x 128 products at 8192 a
-// clock), for 128 adds and 16 KB of TMEM reads per warp and block.  So a block's factor is loaded one block ahead, off the
+// clock), for 128 KB of accumulators read from TMEM.  That read is the limit, not the warps that wait for it: sixteen promotion warps of 64
+// columns took as long (2048 rows 249 us, 239 with packed f32 fma, against 234), and so did the same on CTA pairs, persistent
+// over tiles (242), which halves the shared-memory traffic.  So a block's factor is loaded one block ahead, off the
 // path behind the wait: K=5120 N=17408, 300 rows 62.8 -> 56.0 us, 2048 rows 237 -> 210, 8192 rows 878 -> 797.
 // Measured on top of that and dropped: reading the accumulator in pieces of 16 columns, one under way while the other is
 // added (it spills; 2048 rows 226), and CTA pairs (cta_group::2, half of the weight tile per CTA: 2048 rows 227 with those
@@ -384,7 +386,11 @@ template <typename OutT>
 int launch_any(const uint8_t* qx, const float* sx, const uint8_t* w, const float* sw, OutT* y, int64_t M, int64_t N, int64_t K, int* status,
                cudaStream_t stream) {
     if (M <= 16) return launch_decode<OutT>(qx, sx, w, sw, y, M, N, K, status, stream);
-    return M <= 128 ? launch<OutT, 128>(qx, sx, w, sw, y, M, N, K, status, stream) : launch<OutT, 256>(qx, sx, w, sw, y, M, N, K, status, stream);
+    // 128-column tiles for one row of tiles, and wherever they fit one wave: half as many columns to promote in a tile that nothing
+    // follows (K=5120, us: N=2048, 400 rows 26.5 -> 19.0; N=4096, 200 rows 26.3 -> 18.0; N=9472, 129 rows 28.5 -> 20.0).  From two
+    // waves of them on the 256-column tiles win (N=5120, 512 rows 31.2 against 37.4; N=17408, 2048 rows 226 against 270).
+    if (M <= 128 || ceil_div(M, 128) * ceil_div(N, 128) <= sm_count()) return launch<OutT, 128>(qx, sx, w, sw, y, M, N, K, status, stream);
+    return launch<OutT, 256>(qx, sx, w, sw, y, M, N, K, status, stream);
 }
 
 }  // namespace

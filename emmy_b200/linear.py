@@ -13,6 +13,7 @@ from __future__ import annotations
 import torch
 from torch import nn
 
+from . import lib as L
 from . import ops, ops_moe, ops_nvfp4
 
 # The custom ops take the repacked weights as TENSORS (plus plain ints), never as process-local handles: the packed
@@ -20,16 +21,12 @@ from . import ops, ops_moe, ops_nvfp4
 # but tensors and shapes.
 
 
-def _w4_weight(wq, perm, k, n, group, scale_bf16) -> ops.W4Weight:
-    w = ops.W4Weight()
-    w.wq, w.perm, w.k, w.n, w.group = wq, (perm if perm is not None and perm.numel() else None), k, n, group
-    w.scale_dtype, w.fmt = (torch.bfloat16 if scale_bf16 else torch.float16), "packed"
-    return w
+def _w4a16(x: torch.Tensor, wq: torch.Tensor, perm: torch.Tensor, k: int, n: int, group: int, scale_bf16: bool) -> torch.Tensor:
+    # (an empty perm has a null pointer)
+    return ops._w4a16(x.contiguous(), wq, perm, k, n, group, L.EQ_BF16 if scale_bf16 else L.EQ_F16)
 
 
-@torch.library.custom_op("emmyq::w4a16_linear", mutates_args=(), device_types="cuda")
-def _w4a16_op(x: torch.Tensor, wq: torch.Tensor, perm: torch.Tensor, k: int, n: int, group: int, scale_bf16: bool) -> torch.Tensor:
-    return ops.w4a16_linear(x.contiguous(), _w4_weight(wq, perm, k, n, group, scale_bf16))
+_w4a16_op = torch.library.custom_op("emmyq::w4a16_linear", mutates_args=(), device_types="cuda")(_w4a16)
 
 
 @_w4a16_op.register_fake
@@ -37,9 +34,11 @@ def _(x, wq, perm, k, n, group, scale_bf16):
     return x.new_empty((x.shape[0], n))
 
 
-@torch.library.custom_op("emmyq::fp8_linear", mutates_args=(), device_types="cuda")
-def _fp8_op(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor) -> torch.Tensor:
+def _fp8(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor) -> torch.Tensor:
     return ops.fp8_linear(x.contiguous(), weight, weight_scale)
+
+
+_fp8_op = torch.library.custom_op("emmyq::fp8_linear", mutates_args=(), device_types="cuda")(_fp8)
 
 
 @_fp8_op.register_fake
@@ -47,9 +46,11 @@ def _(x, weight, weight_scale):
     return x.new_empty((x.shape[0], weight.shape[0]))
 
 
-@torch.library.custom_op("emmyq::fp8_linear_static", mutates_args=(), device_types="cuda")
-def _fp8_static_op(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor, input_scale: torch.Tensor) -> torch.Tensor:
+def _fp8_static(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor, input_scale: torch.Tensor) -> torch.Tensor:
     return ops.fp8_linear(x.contiguous(), weight, weight_scale, input_scale=input_scale)
+
+
+_fp8_static_op = torch.library.custom_op("emmyq::fp8_linear_static", mutates_args=(), device_types="cuda")(_fp8_static)
 
 
 @_fp8_static_op.register_fake
@@ -79,9 +80,11 @@ def _(x, wq, k, n, group, scale_bf16):
     return x.new_empty((x.shape[0], n // 2))
 
 
-@torch.library.custom_op("emmyq::fp8_block_linear", mutates_args=(), device_types="cuda")
-def _fp8_block_op(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor) -> torch.Tensor:
+def _fp8_block(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor) -> torch.Tensor:
     return ops.fp8_block_linear(x.contiguous(), weight, weight_scale)
+
+
+_fp8_block_op = torch.library.custom_op("emmyq::fp8_block_linear", mutates_args=(), device_types="cuda")(_fp8_block)
 
 
 @_fp8_block_op.register_fake
@@ -89,9 +92,11 @@ def _(x, weight, weight_scale):
     return x.new_empty((x.shape[0], weight.shape[0]))
 
 
-@torch.library.custom_op("emmyq::nvfp4_linear", mutates_args=(), device_types="cuda")
-def _nvfp4_op(x: torch.Tensor, weight: torch.Tensor, scale_tiled: torch.Tensor, scale_2: torch.Tensor, input_scale: torch.Tensor) -> torch.Tensor:
+def _nvfp4(x: torch.Tensor, weight: torch.Tensor, scale_tiled: torch.Tensor, scale_2: torch.Tensor, input_scale: torch.Tensor) -> torch.Tensor:
     return ops_nvfp4.nvfp4_linear(x.contiguous(), weight, scale_tiled, scale_2, input_scale)
+
+
+_nvfp4_op = torch.library.custom_op("emmyq::nvfp4_linear", mutates_args=(), device_types="cuda")(_nvfp4)
 
 
 @_nvfp4_op.register_fake
@@ -99,8 +104,7 @@ def _(x, weight, scale_tiled, scale_2, input_scale):
     return x.new_empty((x.shape[0], weight.shape[0]))
 
 
-@torch.library.custom_op("emmyq::moe_w4a16", mutates_args=(), device_types="cuda")
-def _moe_op(x: torch.Tensor, router_logits: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, experts: int, hidden: int,
+def _moe(x: torch.Tensor, router_logits: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, experts: int, hidden: int,
             inter: int, group: int, scale_bf16: bool, topk: int) -> torch.Tensor:
     w = ops_moe.MoEWeights()
     w.gate_up, w.down, w.experts, w.hidden, w.inter, w.group = gate_up, down, experts, hidden, inter, group
@@ -108,13 +112,53 @@ def _moe_op(x: torch.Tensor, router_logits: torch.Tensor, gate_up: torch.Tensor,
     return ops_moe.moe_forward(x.contiguous(), router_logits.float().contiguous(), w, topk)
 
 
+_moe_op = torch.library.custom_op("emmyq::moe_w4a16", mutates_args=(), device_types="cuda")(_moe)
+
+
 @_moe_op.register_fake
 def _(x, router_logits, gate_up, down, experts, hidden, inter, group, scale_bf16, topk):
     return torch.empty_like(x)
 
 
+# An eager call on plain CUDA tensors needs nothing of the dispatcher: going through the custom op's Python layers costs about 20 us,
+# four times the kernel at one token (with the lighter calls of ops.py a 4096 x 4096 W4A16Linear of one row 49 -> 19 us a call, FP8Linear of 32 rows 43 -> 27, NVFP4Linear of 40 rows 47 -> 28, QuantMoE of one token 56 -> 35).  "Plain" is decided on each call, by what would make the dispatcher do anything else:
+# tracing or compilation, a tensor or function mode, vmap and the other function transforms (all visible in the thread's included
+# keys), a tensor subclass or wrapper (visible in the tensor's own keys), gradients and forward-mode levels, a profiler that wants
+# to see the operator.  Any of them takes the operator as before.
+_K = torch._C.DispatchKey
+_PLAIN_THREAD = {(torch._C.DispatchKeySet(_K.BackendSelect) | torch._C.DispatchKeySet(_K.ADInplaceOrView)).raw_repr(),
+                 torch._C.DispatchKeySet(_K.BackendSelect).raw_repr()}
+_PLAIN_TENSOR = (_K.CUDA, _K.ADInplaceOrView, _K.AutogradCUDA, _K.AutocastCUDA)
+
+
+def _keys(*names):
+    s = torch._C.DispatchKeySet(names[0])
+    for n in names[1:]:
+        s = s | torch._C.DispatchKeySet(n)
+    return s.raw_repr()
+
+
+_PLAIN_KEYS = {_keys(*_PLAIN_TENSOR), _keys(_K.CUDA, _K.AutocastCUDA)}
+
+
+def _direct(x, *weights):
+    if torch.compiler.is_compiling() or torch._C._dispatch_tls_local_include_set().raw_repr() not in _PLAIN_THREAD:
+        return False
+    if torch._C._len_torch_function_stack() or torch.autograd.forward_ad._current_level >= 0 or torch.autograd._profiler_enabled():
+        return False
+    if type(x) is not torch.Tensor or torch._C._dispatch_keys(x).raw_repr() not in _PLAIN_KEYS:
+        return False
+    grad = torch.is_grad_enabled()
+    if grad and x.requires_grad:
+        return False
+    for w in weights:
+        if type(w) is not torch.Tensor or not w.is_cuda or (grad and w.requires_grad):
+            return False
+    return True
+
+
 def _flat(x):
-    return x.reshape(-1, x.shape[-1]), x.shape[:-1]
+    return (x, x.shape[:-1]) if x.dim() == 2 else (x.reshape(-1, x.shape[-1]), x.shape[:-1])
 
 
 class W4A16Linear(nn.Module):
@@ -168,8 +212,9 @@ class W4A16Linear(nn.Module):
             self.finalize(keep_checkpoint=True)
         x2, lead = _flat(x)
         g = self.in_features if self.group_size == -1 else self.group_size
-        y = _w4a16_op(x2, self.packed_wq, self.packed_perm, self.in_features, self.out_features, g, self._scale_bf16)
-        return y.reshape(*lead, self.out_features)
+        op = _w4a16 if _direct(x2, self.packed_wq) else _w4a16_op
+        y = op(x2, self.packed_wq, self.packed_perm, self.in_features, self.out_features, g, self._scale_bf16)
+        return y if x.dim() == 2 else y.reshape(*lead, self.out_features)
 
 
 class FP8Linear(nn.Module):
@@ -197,7 +242,8 @@ class FP8Linear(nn.Module):
         x2, lead = _flat(x)
         if getattr(self, "input_scale", None) is not None:
             return _fp8_static_op(x2, self.weight, self.weight_scale, self.input_scale).reshape(*lead, self.out_features)
-        return _fp8_op(x2, self.weight, self.weight_scale).reshape(*lead, self.out_features)
+        op = _fp8 if _direct(x2, self.weight, self.weight_scale) else _fp8_op
+        return op(x2, self.weight, self.weight_scale).reshape(*lead, self.out_features)
 
 
 class FP8BlockLinear(nn.Module):
@@ -220,7 +266,8 @@ class FP8BlockLinear(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         x2, lead = _flat(x)
-        return _fp8_block_op(x2, self.weight, self.weight_scale_inv).reshape(*lead, self.out_features)
+        op = _fp8_block if _direct(x2, self.weight, self.weight_scale_inv) else _fp8_block_op
+        return op(x2, self.weight, self.weight_scale_inv).reshape(*lead, self.out_features)
 
 
 class NVFP4Linear(nn.Module):
@@ -246,7 +293,8 @@ class NVFP4Linear(nn.Module):
         if self.scale_tiled is None:
             self.finalize()
         x2, lead = _flat(x)
-        y = _nvfp4_op(x2, self.weight, self.scale_tiled, self.weight_scale_2.reshape(1), self.input_scale.reshape(1))
+        op = _nvfp4 if _direct(x2, self.weight, self.scale_tiled, self.weight_scale_2, self.input_scale) else _nvfp4_op
+        y = op(x2, self.weight, self.scale_tiled, self.weight_scale_2.reshape(1), self.input_scale.reshape(1))
         return y.reshape(*lead, self.out_features)
 
 
@@ -272,5 +320,6 @@ class QuantMoE(nn.Module):
         if self._geometry is None:
             raise RuntimeError("QuantMoE.forward: load_experts() has not been called")
         x2, lead = _flat(x)
-        y = _moe_op(x2, router_logits.reshape(-1, router_logits.shape[-1]), self.packed_gate_up, self.packed_down, *self._geometry, self.top_k)
+        op = _moe if _direct(x2, router_logits, self.packed_gate_up, self.packed_down) else _moe_op
+        y = op(x2, router_logits.reshape(-1, router_logits.shape[-1]), self.packed_gate_up, self.packed_down, *self._geometry, self.top_k)
         return y.reshape(*lead, x.shape[-1])

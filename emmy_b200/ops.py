@@ -18,20 +18,23 @@ _DTYPE = {torch.float16: L.EQ_F16, torch.bfloat16: L.EQ_BF16, torch.float32: L.E
 _FMT = {"awq": L.EQ_W4_AWQ, "gptq": L.EQ_W4_GPTQ, "ct": L.EQ_W4_CT}
 
 
+# Eager calls of a few microseconds of device time are bound by what happens here: plain integers for the pointer arguments
+# (the signatures of lib.py convert them), the raw stream handle instead of a Stream object.
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else C.c_void_p(0)
+    return t.data_ptr() if t is not None else None
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _need_cuda(*tensors):
     for t in tensors:
-        if t is not None and not t.is_cuda:
-            raise RuntimeError("emmy_b200 operators take CUDA tensors only; there is no CPU path")
-        if t is not None and not t.is_contiguous():
-            raise ValueError("emmy_b200 operators take contiguous tensors")
+        if t is not None:
+            if not t.is_cuda:
+                raise RuntimeError("emmy_b200 operators take CUDA tensors only; there is no CPU path")
+            if not t.is_contiguous():
+                raise ValueError("emmy_b200 operators take contiguous tensors")
 
 
 def unpack_int4(words: torch.Tensor, fmt: str, along_rows: bool = False) -> torch.Tensor:
@@ -156,8 +159,12 @@ _workspaces: dict = {}
 
 def w4a16_workspace(m: int, n: int, device, k: int = 1) -> torch.Tensor:
     """A zeroed scratch buffer per (device, stream); grown on demand, reused by calls on that stream."""
+    return _kept_workspace(m, n, k, device, device.index if device.index is not None else torch.cuda.current_device())
+
+
+def _kept_workspace(m, n, k, device, index):
     need = L.load().eq_w4a16_workspace_bytes(m, n, k)
-    key = (device.index if device.index is not None else torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream)
+    key = (index, _stream())
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < need:
         buf = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
@@ -167,16 +174,19 @@ def w4a16_workspace(m: int, n: int, device, k: int = 1) -> torch.Tensor:
 
 def w4a16_linear(x: torch.Tensor, w: W4Weight, workspace: torch.Tensor | None = None, out: torch.Tensor | None = None):
     """y[M, N] = x[M, K] @ W, x and y in f16 or bf16."""
+    return _w4a16(x, w.wq, w.perm, w.k, w.n, w.group, _DTYPE[w.scale_dtype], workspace, out)
+
+
+def _w4a16(x, wq, perm, wk, n, group, scale_code, workspace=None, out=None):
     _need_cuda(x)
     m, k = x.shape
-    if k != w.k:
-        raise ValueError(f"x has {k} features, the weight takes {w.k}")
-    y = out if out is not None else torch.empty((m, w.n), dtype=x.dtype, device=x.device)
-    ws = workspace if workspace is not None else w4a16_workspace(m, w.n, x.device, w.k)
+    if k != wk:
+        raise ValueError(f"x has {k} features, the weight takes {wk}")
+    y = out if out is not None else x.new_empty((m, n))
+    ws = workspace if workspace is not None else _kept_workspace(m, n, k, x.device, x.get_device())
     L.check(
         L.load().eq_w4a16_linear(
-            _ptr(w.wq), _DTYPE[w.scale_dtype], _ptr(w.perm), w.k, w.n, w.group, _ptr(x), m, _DTYPE[x.dtype],
-            _ptr(y), _ptr(ws), ws.numel(), _stream(),
+            wq.data_ptr(), scale_code, _ptr(perm), k, n, group, x.data_ptr(), m, _DTYPE[x.dtype], y.data_ptr(), ws.data_ptr(), ws.numel(), _stream(),
         )
     )
     return y

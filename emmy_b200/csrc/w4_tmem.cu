@@ -362,11 +362,11 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                         break;
                     }
                     tc::fence_after_sync();
-                    const uint32_t b_addr = tc::smem_u32(tiles_b) + stage * Cfg::kStageBytes;
+                    const uint64_t b_desc = tc::smem_desc_k_sw128(tc::smem_u32(tiles_b) + stage * Cfg::kStageBytes);  // further steps: + bytes / 16
 #pragma unroll
                     for (int ks = 0; ks < 8; ++ks)
-                        mma_f16_ts(tmem_base + b * Cfg::kAccCols, tmem_a + 64 * stage + 8 * ks, tc::smem_desc_k_sw128(b_addr + (ks >> 2) * (NB * 128) + (ks & 3) * 32),
-                                   idesc, ks > 0 || (!PROMOTE && it > 0));
+                        mma_f16_ts(tmem_base + b * Cfg::kAccCols, tmem_a + 64 * stage + 8 * ks, b_desc + ((ks >> 2) * (NB * 128) + (ks & 3) * 32) / 16, idesc,
+                                   ks > 0 || (!PROMOTE && it > 0));
                     tc::mma_commit(empty + 8 * stage);
                     if (PROMOTE) tc::mma_commit(acc_full + 8 * b);
                 }

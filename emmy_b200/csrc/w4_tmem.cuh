@@ -82,17 +82,21 @@ namespace tm {
 // DEPENDENT: in a programmatic dependent the warps wait for each other while the grid before it may still run, for as long as
 // it likes: a wait that runs out is taken once more from the end of that grid.  (griddepcontrol.wait ahead of the first wait
 // does that too, but costs 0.3 to 0.6 us of a 16 us launch where launches follow each other.)
+__device__ __forceinline__ bool try_asleep(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(parity), "r"(1000000u)
+                 : "memory");
+    return ok != 0;
+}
 template <bool DEPENDENT = false>
 __device__ __forceinline__ bool wait_asleep(uint32_t bar, uint32_t parity) {
+    if (try_asleep(bar, parity)) return true;  // the usual case, without a look at the clock
     bool again = DEPENDENT;
     long long start = clock64();
-    for (;;) {
-        uint32_t ok;
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
-                     : "=r"(ok)
-                     : "r"(bar), "r"(parity), "r"(1000000u)
-                     : "memory");
-        if (ok) return true;
+#pragma unroll 1
+    while (!try_asleep(bar, parity)) {
         if (clock64() - start > tc::kWaitCycles) {
             if (!again) return false;
             again = false;
@@ -100,6 +104,7 @@ __device__ __forceinline__ bool wait_asleep(uint32_t bar, uint32_t parity) {
             start = clock64();
         }
     }
+    return true;
 }
 
 // ---- distributed shared memory

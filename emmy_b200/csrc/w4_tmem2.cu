@@ -250,11 +250,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         break;
                     }
                     tc::fence_after_sync();
-                    const uint32_t b_addr = tiles_b + sb * kTileB;
+                    const uint64_t b_desc = tc::smem_desc_k_sw128(tiles_b + sb * kTileB);  // further steps: + bytes / 16
 #pragma unroll
                     for (int ks = 0; ks < 8; ++ks)
-                        mma_f16_ts_pair(tmem_base, tmem_a + 64 * sa + 8 * ks, tc::smem_desc_k_sw128(b_addr + (ks >> 2) * (kHalfRows * 128) + (ks & 3) * 32), idesc,
-                                        ks > 0 || it > 0);
+                        mma_f16_ts_pair(tmem_base, tmem_a + 64 * sa + 8 * ks, b_desc + ((ks >> 2) * (kHalfRows * 128) + (ks & 3) * 32) / 16, idesc, ks > 0 || it > 0);
                     tc::commit_pair(empty_a + 8 * sa);
                     tc::commit_pair(empty_b + 8 * sb);
                 }

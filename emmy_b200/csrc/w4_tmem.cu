@@ -155,8 +155,7 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
             } while (pf_unit < units && pf_item >= pf_items);
         }
         if (pf_unit < units) {
-            fetch_item(pf_slot, lo, pf0);
-            fetch_item(pf_slot + kItemBytes, lo, pf1);
+            fetch_items(pf_slot, lo, pf0, pf1);
             pf0 += 2 * kItemBytes;
             pf1 += 2 * kItemBytes;
             pf_item += 2;
@@ -196,7 +195,6 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
         // this warp's items: every second one of the CTA's sequence over all units
         int next = wg;       // its next item, counted from the start of the current unit
         int stage = wg, phase = 1, ring_at = wg;  // stage and (inverted) use parity of that item; its scales' slot
-        uint32_t slot = my_ring;
         bool first = true, broken = false;
         bool waited = false;  // behind griddepcontrol.wait
         int n_unit = 0;
@@ -209,11 +207,9 @@ __global__ void __launch_bounds__(TmemCfg<NB, PROMOTE>::kThreads, 2)
                 cp_wait<D - 1>();
                 __syncwarp();
                 ItemWords w;
-                load_item(slot, lo, w);
+                load_item(pf_slot, lo, w);  // the oldest of the ring, and the next to be refilled
                 __syncwarp();
-                prefetch();  // refills the slot just read
-                slot += 2 * kItemBytes;
-                if (slot == my_ring + D * 2 * kItemBytes) slot = my_ring;
+                prefetch();  // refills it
                 if (!first && !__all_sync(0xFFFFFFFFu, wait_asleep<!GROUPED>(empty + 8 * stage, phase))) {
                     if (lane == 0) atomicExch(a.status, 4);
                     broken = true;

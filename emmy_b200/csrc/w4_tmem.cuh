@@ -145,25 +145,11 @@ struct Mul<__nv_bfloat16> {
     }
 };
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-    uint32_t r;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(a) : "memory");
-    return r;
-}
-__device__ __forceinline__ uint2 lds64(uint32_t a) {
-    uint2 r;
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(a) : "memory");
-    return r;
-}
-
 // 16 lanes x 32 columns: lane 4 g + j of the warp gives rows g and g + 8 of column 4 i + j in registers 2 i, 2 i + 1.
 __device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
@@ -271,24 +257,41 @@ struct LaneOffsets {
         get_meta = 1024 + 8 * g;
     }
 };
+// (Offsets as immediates: with an address computed for each of them the reads and copies cost thirty more instructions an item.)
+template <int OFF>
+__device__ __forceinline__ uint32_t lds32_at(uint32_t a) {
+    uint32_t r;
+    asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(r) : "r"(a), "n"(OFF) : "memory");
+    return r;
+}
 __device__ __forceinline__ void load_item(uint32_t slot_addr, const LaneOffsets& o, ItemWords& w) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const uint32_t at = slot_addr + o.get[r];
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            w.wd[t][2 * r] = lds32(at + t * kItemBytes);
-            w.wd[t][2 * r + 1] = lds32(at + t * kItemBytes + 512);
-        }
+        w.wd[0][2 * r] = lds32_at<0>(at);
+        w.wd[0][2 * r + 1] = lds32_at<512>(at);
+        w.wd[1][2 * r] = lds32_at<kItemBytes>(at);
+        w.wd[1][2 * r + 1] = lds32_at<kItemBytes + 512>(at);
     }
-    w.mt[0] = lds64(slot_addr + o.get_meta);
-    w.mt[1] = lds64(slot_addr + o.get_meta + kItemBytes);
+    const uint32_t meta = slot_addr + o.get_meta;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w.mt[0].x), "=r"(w.mt[0].y) : "r"(meta) : "memory");
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2+%3];" : "=r"(w.mt[1].x), "=r"(w.mt[1].y) : "r"(meta), "n"(kItemBytes) : "memory");
 }
-// One tile's record (1088 bytes) into a ring slot; src: the record + 16 * lane.
-__device__ __forceinline__ void fetch_item(uint32_t slot_addr, const LaneOffsets& o, const unsigned char* src) {
-    cp_async16(slot_addr + o.put, src);
-    cp_async16(slot_addr + o.put + 512, src + 512);
-    if ((threadIdx.x & 31) < 4) cp_async16(slot_addr + o.put_meta, src + 1024);
+// The records (1088 bytes) of a warp's two tiles into its ring slot; src0, src1: the records + 16 * lane.
+__device__ __forceinline__ void fetch_items(uint32_t slot_addr, const LaneOffsets& o, const unsigned char* src0, const unsigned char* src1) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.lt.u32 p, %4, 4;\n"
+        "cp.async.cg.shared.global [%0], [%2], 16;\n"
+        "cp.async.cg.shared.global [%0+512], [%2+512], 16;\n"
+        "@p cp.async.cg.shared.global [%1], [%2+1024], 16;\n"
+        "cp.async.cg.shared.global [%0+%5], [%3], 16;\n"
+        "cp.async.cg.shared.global [%0+%6], [%3+512], 16;\n"
+        "@p cp.async.cg.shared.global [%1+%5], [%3+1024], 16;\n"
+        "}\n" ::"r"(slot_addr + o.put),
+        "r"(slot_addr + o.put_meta), "l"(src0), "l"(src1), "r"(threadIdx.x & 31), "n"(kItemBytes), "n"(kItemBytes + 512)
+        : "memory");
 }
 // Zero point pair -> constants of the exact dequant (Frag<ActT>::expand), fewer instructions than Frag<ActT>::zero: the
 // zero points are the integers 0..16.

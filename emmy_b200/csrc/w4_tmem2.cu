@@ -128,8 +128,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 if (pf_unit < units) pf_locate();
             }
             if (pf_unit < units) {
-                fetch_item(pf_slot, lo, pf0);
-                fetch_item(pf_slot + kItemBytes, lo, pf1);
+                fetch_items(pf_slot, lo, pf0, pf1);
                 pf0 += kGroups * kItemBytes;
                 pf1 += kGroups * kItemBytes;
                 pf_item += kGroups;
@@ -143,7 +142,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         for (int d = 0; d < kDepth; ++d) prefetch();
 
         int next = wg;  // this warp's next item (every fourth of the pair's sequence), from the start of the current unit
-        uint32_t slot = my_ring, phase = 1;
+        uint32_t phase = 1;
         bool first = true, broken = false, waited = false;
         int n_unit = 0;
         const uint32_t a_dst = tmem_a + (static_cast<uint32_t>(32 * q) << 16) + 64 * wg;
@@ -154,11 +153,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 cp_wait<kDepth - 1>();
                 __syncwarp();
                 ItemWords w;
-                load_item(slot, lo, w);
+                load_item(pf_slot, lo, w);  // the oldest of the ring, and the next to be refilled
                 __syncwarp();
-                prefetch();  // refills the slot just read
-                slot += 2 * kItemBytes;
-                if (slot == my_ring + kDepth * 2 * kItemBytes) slot = my_ring;
+                prefetch();  // refills it
                 if (!first && !__all_sync(0xFFFFFFFFu, wait_asleep<true>(my_empty, phase))) {
                     if (lane == 0) atomicExch(a.status, 4);
                     broken = true;

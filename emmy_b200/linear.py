@@ -121,10 +121,11 @@ def _(x, router_logits, gate_up, down, experts, hidden, inter, group, scale_bf16
 
 
 # An eager call on plain CUDA tensors needs nothing of the dispatcher: going through the custom op's Python layers costs about 20 us,
-# four times the kernel at one token (with the lighter calls of ops.py a 4096 x 4096 W4A16Linear of one row 49 -> 19 us a call, FP8Linear of 32 rows 43 -> 27, NVFP4Linear of 40 rows 47 -> 28, QuantMoE of one token 56 -> 35).  "Plain" is decided on each call, by what would make the dispatcher do anything else:
-# tracing or compilation, a tensor or function mode, vmap and the other function transforms (all visible in the thread's included
-# keys), a tensor subclass or wrapper (visible in the tensor's own keys), gradients and forward-mode levels, a profiler that wants
-# to see the operator.  Any of them takes the operator as before.
+# four times the kernel at one token (with the lighter calls of ops.py a 4096 x 4096 W4A16Linear of one row 49 -> 19 us a call,
+# FP8Linear of 32 rows 43 -> 27, NVFP4Linear of 40 rows 47 -> 28, QuantMoE of one token 56 -> 35).  "Plain" is decided on each call,
+# by what would make the dispatcher do anything else: tracing or compilation, a tensor or function mode, vmap and the other function
+# transforms (all visible in the thread's included keys), a tensor subclass or wrapper (visible in the tensor's own keys), gradients
+# and forward-mode levels, a profiler that wants to see the operator.  Any of them takes the operator as before.
 _K = torch._C.DispatchKey
 _PLAIN_THREAD = {(torch._C.DispatchKeySet(_K.BackendSelect) | torch._C.DispatchKeySet(_K.ADInplaceOrView)).raw_repr(),
                  torch._C.DispatchKeySet(_K.BackendSelect).raw_repr()}

@@ -34,7 +34,7 @@ __device__ __forceinline__ uint16_t e4m3x2_sat(float lo, float hi) {
 template <typename InT>
 __global__ void __launch_bounds__(256) quant_fp8_groups_kernel(const InT* __restrict__ x, int64_t M, int64_t K, uint8_t* __restrict__ q,
                                                                float* __restrict__ scale, int* __restrict__ status) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the linear behind this may start fetching weights
+    if (status) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // inside a linear, which may start fetching its weights
     // inside the linear this kernel is a programmatic dependent itself: the kernel before it (usually the previous
     // linear on this workspace) may still read the codes, scales and status word it rewrites
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) quant_fp8_groups_kernel(const InT* __rest
 template <typename InT>
 __global__ void __launch_bounds__(256) quant_fp8_groups_vec_kernel(const uint4* __restrict__ x, int64_t vecs, uint2* __restrict__ q, float* __restrict__ scale,
                                                                    int* __restrict__ status) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (status) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
     const int64_t first = blockIdx.x * int64_t(512) + threadIdx.x;

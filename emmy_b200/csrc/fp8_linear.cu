@@ -387,7 +387,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 template <typename InT, int kVecs, int kRowThreads>
 __global__ void __launch_bounds__(kRowThreads) quant_fp8_rows_vec_kernel(const InT* __restrict__ x, int64_t K, uint8_t* __restrict__ q,
                                                                   float* __restrict__ scale, int* __restrict__ status) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the linear behind this may start fetching weights
+    // Inside a linear the kernel behind this one may start fetching its weights.  On its own this may BE the quantizer of a weight,
+    // which nothing may fetch before it is complete.
+    if (status) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // launched as a programmatic dependent itself: the kernel before it (usually the previous linear on this workspace)
     // may still read the codes, scales and status word this one rewrites
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -72,7 +72,7 @@ template <typename InT>
 __global__ void quant_nvfp4_act_kernel(const InT* __restrict__ x, int64_t M, int64_t K, const float* __restrict__ scale2,
                                        uint8_t* __restrict__ codes, uint8_t* __restrict__ sf_plain, uint8_t* __restrict__ sf_tiled,
                                        int* __restrict__ status) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (status) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // inside a linear, which may start fetching its weights
     // launched as a programmatic dependent itself when it runs inside the linear: the kernel before it (usually the
     // previous linear on this workspace) still reads the codes and the status word this one rewrites
     asm volatile("griddepcontrol.wait;" ::: "memory");

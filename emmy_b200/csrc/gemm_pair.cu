@@ -215,6 +215,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         OutT* const y = static_cast<OutT*>(p.y);
         const float g = FP4 ? p.sx[0] * p.sw[0] : 0.f;
         int t = 0;
+        bool broken = false;
         for (int u = cluster; u < p.units; u += clusters, ++t) {
             const int b = t & 1, n0 = col_of(u), m = row_of(u) + rank * 128 + quarter * 32 + lane;
             float row_scale = 0.f;
@@ -224,10 +225,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 sw_tile[b * 256 + i] = n0 + i < p.N ? p.sw[n0 + i] : 0.f;
                 asm volatile("bar.sync 1, 256;" ::: "memory");  // the epilogue warps; the other half of sw_tile is free again too
             }
-            if (!__all_sync(0xFFFFFFFFu, tc::mbar_wait(acc_full + 8 * b, (t >> 1) & 1))) {
+            // A warp that gives up meets the others at the barrier above until its tiles end, and does nothing else: their waits, each with
+            // its own clock, may have been met a moment later.
+            if (!broken && !__all_sync(0xFFFFFFFFu, tc::mbar_wait(acc_full + 8 * b, (t >> 1) & 1))) {
                 if (lane == 0) atomicExch(p.status, 3);
-                break;
+                broken = true;
             }
+            if (broken) continue;
             tc::fence_after_sync();
 #pragma unroll 1
             for (int i = 0; i < 4; ++i) {

@@ -118,7 +118,8 @@ __global__ void quant_nvfp4_act_kernel(const InT* __restrict__ x, int64_t M, int
 template <typename InT>
 __global__ void __launch_bounds__(512) quant_nvfp4_act_atoms_kernel(const uint4* __restrict__ x, int64_t M, int k64_blocks, const float* __restrict__ scale2,
                                                                     uint8_t* __restrict__ codes, uint8_t* __restrict__ sf_tiled, int* __restrict__ status) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // Only inside a linear: on its own this may write the operands of a weight, which a linear behind it would fetch ahead of its wait.
+    if (status) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int r = threadIdx.x >> 2, i = threadIdx.x & 3, kb = blockIdx.x;
     if (status && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) *status = 0;

@@ -226,3 +226,30 @@ def test_activation_quant_inside_the_linear_equals_the_standalone_one(m, k, dtyp
         rows, blocks = np.meshgrid(np.arange(m), np.arange(k // 16), indexing="ij")
         off = ((rows // 128) * (k // 64) + blocks // 4) * 512 + (rows % 32) * 16 + ((rows % 128) // 32) * 4 + blocks % 4
         np.testing.assert_array_equal(got[at + off], sf.cpu().numpy())
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("rows,k", [(72, 256), (128, 512), (200, 768), (264, 1280), (1000, 512)])
+def test_tiled_only_quantize_on_its_own_as_a_weight(rows, k, dtype):
+    """eq_quant_nvfp4_act with tiled scales and no plain ones, above 64 rows: the bytes of the plain form, zeros in the atoms' padding
+    rows; and a linear right behind it that takes those operands as its weight reads finished ones."""
+    from emmy_b200 import lib as L
+    from emmy_b200 import ops_nvfp4 as o4
+    from emmy_b200.ops import _DTYPE, _ptr, _stream
+
+    gen = torch.Generator().manual_seed(rows)
+    values = torch.randn(rows, k, generator=gen).to(torch.bfloat16 if dtype == "bf16" else torch.float16).cuda()
+    s2 = o4.nvfp4_global_scale(values)
+    plain_codes, plain_sf, plain_tiled = o4.quant_nvfp4_act(values, s2, tiled=True)
+    x = torch.randn(33, k, generator=gen).to(values.dtype).cuda()
+    s2x = o4.nvfp4_global_scale(x)
+    codes, tiled = torch.full_like(plain_codes, 0xEE), torch.full((o4.nvfp4_tile_weight_scales(plain_sf, k).numel(),), 0xEE, dtype=torch.uint8, device="cuda")
+    ws, y = o4.nvfp4_workspace(33, k, x.device), torch.empty(33, rows, dtype=x.dtype, device="cuda")
+    torch.cuda.synchronize()
+    L.check(L.load().eq_quant_nvfp4_act(_ptr(values), rows, k, _DTYPE[values.dtype], _ptr(s2), _ptr(codes), None, _ptr(tiled), _stream()))
+    o4.nvfp4_linear(x, codes, tiled, s2, s2x, workspace=ws, out=y)
+    torch.cuda.synchronize()
+    assert torch.equal(codes, plain_codes)
+    assert torch.equal(tiled[: plain_tiled.numel()], plain_tiled)
+    want = o4.nvfp4_linear(x, plain_codes, o4.nvfp4_tile_weight_scales(plain_sf, k), s2, s2x)
+    assert torch.equal(y, want)

@@ -1,4 +1,4 @@
-"""Every wait of a kernel ends, also when another one has run out: read off the sources, nothing is launched.
+"""Order between threads and between launches, read off the kernel sources; nothing is launched.
 
 A barrier that is crossed once per turn of a loop is met by all of its threads only if none of them leaves the loop, or skips to its
 next turn ahead of the barrier, on its own account (a bounded wait that ran out in one warp and was met in the next)."""
@@ -90,3 +90,24 @@ def test_the_reading_finds_what_it_looks_for():
     assert read("continue;", "") == [(4, "continue")]
     assert read("a();", "broken = true; continue;") == []
     assert read("for (int i = 0; i < 4; ++i) { if (i) break; }", "auto g = [&](int i) { return i; };") == []
+
+
+@pytest.mark.parametrize(
+    "source,kernel",
+    [
+        ("fp8_linear.cu", "quant_fp8_rows_vec_kernel"),
+        ("fp8_block.cu", "quant_fp8_groups_kernel"),
+        ("fp8_block.cu", "quant_fp8_groups_vec_kernel"),
+        ("nvfp4_linear.cu", "quant_nvfp4_act_kernel"),
+        ("nvfp4_linear.cu", "quant_nvfp4_act_atoms_kernel"),
+    ],
+)
+def test_a_quantizer_on_its_own_releases_nothing(source, kernel):
+    """A quantizer that is also an entry of its own (no status word) may be writing a weight, and a linear fetches its weights ahead of
+    its wait: only inside a linear does it let the kernel behind it start."""
+    code = _code((CSRC / source).read_text())
+    body = code[code.index(kernel + "(") :]
+    body = body[: body.index("\n}\n")]
+    release = [line.strip() for line in body.splitlines() if "griddepcontrol.launch_dependents" in line]
+    assert release and all(line.startswith("if (status) asm volatile") for line in release)
+    assert "griddepcontrol.wait" in body

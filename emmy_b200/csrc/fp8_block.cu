@@ -226,6 +226,7 @@ static int quant_fp8_groups(const void* x, int64_t M, int64_t K, int in_dtype, u
     EQ_REQUIRE(x && q && scale, EQ_ERR_BAD_ARG, "eq_quant_fp8_per_group: null pointer");
     EQ_REQUIRE(K % 128 == 0, EQ_ERR_UNSUPPORTED, "eq_quant_fp8_per_group: K must be a multiple of 128");
     EQ_REQUIRE(aligned(q, 4), EQ_ERR_BAD_ALIGN, "eq_quant_fp8_per_group: q must be 4-byte aligned");
+    EQ_REQUIRE(in_dtype == EQ_F16 || in_dtype == EQ_BF16 || in_dtype == EQ_F32, EQ_ERR_BAD_ARG, "eq_quant_fp8_per_group: unknown dtype %d", in_dtype);
     const int64_t warps = M * (K / 128);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(ceil_div(warps * 32, 256)));
@@ -250,8 +251,7 @@ static int quant_fp8_groups(const void* x, int64_t M, int64_t K, int in_dtype, u
     switch (in_dtype) {
         case EQ_F16: EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_fp8_groups_kernel<__half>, static_cast<const __half*>(x), M, K, q, scale, status)); break;
         case EQ_BF16: EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_fp8_groups_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(x), M, K, q, scale, status)); break;
-        case EQ_F32: EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_fp8_groups_kernel<float>, static_cast<const float*>(x), M, K, q, scale, status)); break;
-        default: return fail(EQ_ERR_BAD_ARG, "eq_quant_fp8_per_group: unknown dtype %d", in_dtype);
+        default: EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_fp8_groups_kernel<float>, static_cast<const float*>(x), M, K, q, scale, status)); break;
     }
     return EQ_OK;
 }

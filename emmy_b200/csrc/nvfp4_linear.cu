@@ -629,6 +629,7 @@ static int quant_nvfp4_act(const void* x, int64_t M, int64_t K, int in_dtype, co
     EQ_REQUIRE(x && input_scale && codes, EQ_ERR_BAD_ARG, "eq_quant_nvfp4_act: null pointer");
     EQ_REQUIRE(K % 16 == 0 && (!scale_tiled || K % 64 == 0), EQ_ERR_UNSUPPORTED, "eq_quant_nvfp4_act: K must be a multiple of 16 (64 with tiled scales)");
     EQ_REQUIRE(aligned(codes, 8), EQ_ERR_BAD_ALIGN, "eq_quant_nvfp4_act: codes must be 8-byte aligned");
+    EQ_REQUIRE(in_dtype == EQ_F16 || in_dtype == EQ_BF16 || in_dtype == EQ_F32, EQ_ERR_BAD_ARG, "eq_quant_nvfp4_act: unknown dtype %d", in_dtype);
     if (scale_tiled && pad_rows) EQ_CUDA_OK(cudaMemsetAsync(scale_tiled, 0, sf_tiled_bytes(M, K), stream));
     const int64_t total = M * (K / 16);
     cudaLaunchConfig_t cfg = {};
@@ -654,8 +655,7 @@ static int quant_nvfp4_act(const void* x, int64_t M, int64_t K, int in_dtype, co
     switch (in_dtype) {
         case EQ_F16: EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_nvfp4_act_kernel<__half>, static_cast<const __half*>(x), M, K, input_scale, codes, scale_bits, scale_tiled, status)); break;
         case EQ_BF16: EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_nvfp4_act_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(x), M, K, input_scale, codes, scale_bits, scale_tiled, status)); break;
-        case EQ_F32: EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_nvfp4_act_kernel<float>, static_cast<const float*>(x), M, K, input_scale, codes, scale_bits, scale_tiled, status)); break;
-        default: return fail(EQ_ERR_BAD_ARG, "eq_quant_nvfp4_act: unknown dtype %d", in_dtype);
+        default: EQ_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_nvfp4_act_kernel<float>, static_cast<const float*>(x), M, K, input_scale, codes, scale_bits, scale_tiled, status)); break;
     }
     return EQ_OK;
 }

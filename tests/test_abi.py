@@ -105,3 +105,14 @@ def test_kernel_names_by_extent(eq):
                             (20, 256, 14336, "stream"), (20, 512, 5120, "tmem"), (25, 4096, 512, "tmem")]:
         assert name(m, n, k) == f"w4a16_{kernel}_kernel", (m, n, k)
     assert name(4096, 16) == "w4a16_tmem_kernel"  # too narrow to occupy the pairs
+
+
+@pytest.mark.parametrize("m", [4, 65, 4096])
+def test_quantizers_refuse_unknown_dtypes(eq, m):
+    """Whatever the size: small and large calls run on different kernels.  The pointers are never dereferenced."""
+    null, one = C.c_void_p(0), C.c_void_p(4096)
+    for dtype in (3, 7, -1):
+        assert eq.eq_quant_fp8_per_token(one, m, 1024, dtype, one, one, null) == L.EQ_ERR_BAD_ARG
+        assert eq.eq_quant_fp8_per_group(one, m, 1024, dtype, one, one, null) == L.EQ_ERR_BAD_ARG
+        assert eq.eq_quant_nvfp4_act(one, m, 1024, dtype, one, one, null, one, null) == L.EQ_ERR_BAD_ARG
+        assert eq.eq_quant_nvfp4_act(one, m, 1024, dtype, one, one, one, null, null) == L.EQ_ERR_BAD_ARG

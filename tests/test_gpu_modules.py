@@ -107,3 +107,64 @@ def test_nvfp4_module():
     y = mod.cuda()(torch.from_numpy(x).bfloat16().cuda()).float().cpu().numpy()
     ref = ol.nvfp4_linear(x, packed, sbits, s2, s2x)
     assert np.abs(y - ref).max() <= 2e-2 * np.abs(ref).max()
+
+
+def _modules():
+    """Each module that has a direct form, an input of its own, and the registered operator on the same tensors."""
+    from emmy_b200 import linear
+    from emmy_b200.ops_nvfp4 import nvfp4_global_scale
+
+    k, n, dev = 512, 256, lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    gen = torch.Generator().manual_seed(21)
+    x16, xb = torch.randn(33, k, generator=gen).half().cuda(), torch.randn(33, k, generator=gen).bfloat16().cuda()
+    qw, qz, sc, gi = synth.gptq_linear(k, n, seed=22)
+    w4 = linear.W4A16Linear(k, n, 128, fmt="gptq", act_order=True)
+    w4.load_state_dict({"qweight": torch.from_numpy(qw), "qzeros": torch.from_numpy(qz), "scales": torch.from_numpy(sc), "g_idx": torch.from_numpy(gi)})
+    w4 = w4.cuda().finalize()
+    yield "w4a16", lambda x: w4(x), lambda x: linear._w4a16_op(x, w4.packed_wq, w4.packed_perm, k, n, 128, w4._scale_bf16), x16, (w4.packed_wq,)
+    bits, sw = synth.fp8_weight(n, k, seed=23)
+    fp8 = linear.FP8Linear(k, n).cuda()
+    fp8.load_float8(dev(bits).view(torch.float8_e4m3fn), dev(sw))
+    yield "fp8", lambda x: fp8(x), lambda x: linear._fp8_op(x, fp8.weight, fp8.weight_scale), xb, (fp8.weight, fp8.weight_scale)
+    blk = linear.FP8BlockLinear(k, n).cuda()
+    blk.weight, blk.weight_scale_inv = dev(bits), torch.rand(n // 128, k // 128, generator=gen).cuda() + 0.5
+    yield "fp8_block", lambda x: blk(x), lambda x: linear._fp8_block_op(x, blk.weight, blk.weight_scale_inv), xb, (blk.weight, blk.weight_scale_inv)
+    packed, sbits, s2 = synth.nvfp4_weight(n, k, seed=24)
+    fp4 = linear.NVFP4Linear(k, n)
+    fp4.load_state_dict({"weight": torch.from_numpy(packed), "weight_scale": torch.from_numpy(sbits), "weight_scale_2": torch.from_numpy(s2),
+                         "input_scale": nvfp4_global_scale(xb).cpu()})
+    fp4 = fp4.cuda()
+    fp4.finalize()
+    yield ("nvfp4", lambda x: fp4(x), lambda x: linear._nvfp4_op(x, fp4.weight, fp4.scale_tiled, fp4.weight_scale_2.reshape(1), fp4.input_scale.reshape(1)), xb,
+           (fp4.weight, fp4.scale_tiled, fp4.weight_scale_2, fp4.input_scale))
+    e, h, inter = 4, 256, 128
+    awq = lambda k_, n_: (torch.randint(-(2**31), 2**31 - 1, (e, k_, n_ // 8), dtype=torch.int32, generator=gen).cuda(),
+                          torch.randint(-(2**31), 2**31 - 1, (e, k_ // 128, n_ // 8), dtype=torch.int32, generator=gen).cuda(),
+                          (torch.rand(e, k_ // 128, n_, generator=gen) * 0.02).half().cuda())
+    moe = linear.QuantMoE(2).load_experts(awq(h, 2 * inter), awq(inter, h), 128, "awq")
+    xm, logits = torch.randn(33, h, generator=gen).bfloat16().cuda(), torch.randn(33, e, generator=gen).cuda()
+    yield ("moe", lambda x: moe(x, logits), lambda x: linear._moe_op(x, logits, moe.packed_gate_up, moe.packed_down, *moe._geometry, moe.top_k), xm,
+           (logits, moe.packed_gate_up, moe.packed_down))
+
+
+def test_plain_cuda_calls_are_direct_and_equal_the_operators(monkeypatch):
+    """What an eager program passes on a GPU counts as plain (its dispatch keys are those that linear.py spells), the modules then leave
+    the operators out, and the outputs are the same bits (33 rows: every sum has a fixed order there)."""
+    from emmy_b200 import linear
+
+    taken = []
+    real = linear._direct
+    monkeypatch.setattr(linear, "_direct", lambda *a: taken.append(real(*a)) or taken[-1])
+    for name, module, operator, x, weights in _modules():
+        for mode in (torch.enable_grad, torch.no_grad, torch.inference_mode):
+            with mode():
+                t = x.clone()  # an inference tensor inside inference mode
+                assert real(t, *weights), (name, mode)
+                taken.clear()
+                got = module(t)
+                assert taken == [True], (name, mode)
+                assert torch.equal(got, operator(t)), (name, mode)
+                assert torch.equal(module(t.reshape(3, 11, -1)), got.reshape(3, 11, -1)), (name, mode)
+        with torch.enable_grad():
+            assert not real(x.clone().requires_grad_(), *weights), name
+        assert not real(x.cpu(), *weights), name

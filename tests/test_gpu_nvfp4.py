@@ -253,3 +253,25 @@ def test_tiled_only_quantize_on_its_own_as_a_weight(rows, k, dtype):
     assert torch.equal(tiled[: plain_tiled.numel()], plain_tiled)
     want = o4.nvfp4_linear(x, plain_codes, o4.nvfp4_tile_weight_scales(plain_sf, k), s2, s2x)
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize(
+    "m,n,k,pairs",
+    [
+        (300, 12288, 512, False),  # 3 row tiles x 48 column tiles: one wave of 148, where the pairs, 2 x 48, take two
+        (257, 9736, 256, False),   # one row in the third row tile; a last column tile of 8
+        (384, 12536, 1536, False),  # whole row tiles; 49 column tiles, the last of 248
+        (300, 9472, 512, True),    # 37 column tiles: the pairs fit one wave too
+        (300, 12552, 512, True),   # 50 column tiles: 150 one-CTA tiles are more than a wave
+        (385, 12288, 512, True),   # four row tiles
+    ],
+)
+def test_one_cta_tiles_between_the_pairs(m, n, k, pairs, dtype):
+    """Above 128 rows the 128 x 256 tiles of one CTA serve the calls that they fit in one wave and the pairs do not; these and their
+    neighbours on either side of the rule (`pairs`: the form that a B200's 148 SMs give), with partial tiles and a ring that wraps."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    fits = lambda height, places: -(-m // height) * -(-n // 256) <= places  # a tile is `height` rows by 256 columns
+    if sms == 148:
+        assert pairs == (not (fits(128, sms) and not fits(256, sms // 2)))
+    _check(m, n, k, seed=m + n, dtype=dtype)

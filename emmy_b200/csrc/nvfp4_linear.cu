@@ -758,12 +758,16 @@ static int nvfp4_linear_any(const uint8_t* weight, const uint8_t* weight_scale_t
     // codes are bytes holding two e2m1 values: the maps move bytes; 128 bytes = 256 elements of K per tile row
     st = make_tensor_map_2d(&map_a, codes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K / 2, K / 2, kBM, kBKBytes, CU_TENSOR_MAP_SWIZZLE_128B);
     if (st != EQ_OK) return st;
-    // More than 128 rows: 256 x 256 tiles on CTA pairs (K=5120 N=17408: 300 rows 32.3 -> 25.9 us, 1024 rows 69.6 -> 49.4, 4096 rows
-    // 248 -> 167 with the quantize, against 128 x 256 tiles up to a few waves and 256 x 224 tiles of one CTA above).  128 x 256
-    // tiles of one CTA stay for an odd number of 128-row tiles that fits one wave where the pairs, half of the last row of
-    // tiles empty, take two (N=12288, 300 rows: 19.9 against 24.9).
+    // More than 128 rows: 256 x 256 tiles on CTA pairs (figures in gemm_pair.cu).  128 x 256 tiles of one CTA, where they fit one wave, stay
+    // - for an odd number of 128-row tiles where the pairs, half of the last row of tiles empty, take two waves (N=12288, 300 rows: K=5120
+    //   19.9 us against 24.9, K=1024 10.4 against 14.9);
+    // - for a short K, where the pairs' cluster barriers and second operand hand-over are not hidden (one-CTA : pairs, us; K=512 N=2048,
+    //   256 rows 7.7 : 8.2; K=1024 N=4096, 129 rows 8.2 : 8.7, 1000 rows 9.2 : 10.2; K=2048 N=6144, 257 rows 11.3 : 12.3; K=2560 2.6 % and
+    //   K=3072 1.5 % on the mean of 50 shapes; K=4096 even, K=8192 N=4096, 200 rows 19.8 : 17.9).
+    // Linears with the quantize, graph replays over four weights, both forms forced.
     const int64_t col_tiles = ceil_div(N, 256);
-    const bool pairs = M > 128 && !(ceil_div(M, 128) * col_tiles <= sm_count() && ceil_div(M, 256) * col_tiles > sm_count() / 2);
+    const bool one_wave = ceil_div(M, 128) * col_tiles <= sm_count();
+    const bool pairs = M > 128 && !(one_wave && (K < 4096 || ceil_div(M, 256) * col_tiles > sm_count() / 2));
     if (pairs) return nvfp4_pair_launch(codes, sfa, input_scale, weight, weight_scale_tiled, weight_scale_2, y, M, N, K, act_dtype, status, stream);
     // the 128-row-block scale layout at the front of the blob
     const int bn = M <= 128 ? 128 : 256;

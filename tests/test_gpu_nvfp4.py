@@ -259,19 +259,21 @@ def test_tiled_only_quantize_on_its_own_as_a_weight(rows, k, dtype):
 @pytest.mark.parametrize(
     "m,n,k,pairs",
     [
-        (300, 12288, 512, False),  # 3 row tiles x 48 column tiles: one wave of 148, where the pairs, 2 x 48, take two
-        (257, 9736, 256, False),   # one row in the third row tile; a last column tile of 8
-        (384, 12536, 1536, False),  # whole row tiles; 49 column tiles, the last of 248
-        (300, 9472, 512, True),    # 37 column tiles: the pairs fit one wave too
-        (300, 12552, 512, True),   # 50 column tiles: 150 one-CTA tiles are more than a wave
-        (385, 12288, 512, True),   # four row tiles
+        (300, 12288, 4096, False),  # 3 row tiles x 48 column tiles: one wave of 148, where the pairs, 2 x 48, take two
+        (384, 12536, 4352, False),  # whole row tiles; 49 column tiles, the last of 248
+        (300, 9472, 4096, True),    # 37 column tiles: the pairs fit one wave too
+        (300, 12552, 512, True),    # 50 column tiles: 150 one-CTA tiles are more than a wave
+        (385, 12288, 512, True),    # four row tiles
+        (129, 8, 4096, True), (257, 264, 4096, True), (700, 1000, 4352, True),   # small calls on either side of the line on K
+        (129, 8, 3840, False), (257, 264, 3840, False), (700, 1000, 3840, False),
+        (257, 9736, 256, False),    # the shortest K; a last column tile of 8
     ],
 )
-def test_one_cta_tiles_between_the_pairs(m, n, k, pairs, dtype):
-    """Above 128 rows the 128 x 256 tiles of one CTA serve the calls that they fit in one wave and the pairs do not; these and their
-    neighbours on either side of the rule (`pairs`: the form that a B200's 148 SMs give), with partial tiles and a ring that wraps."""
+def test_one_cta_tiles_beside_the_pairs(m, n, k, pairs, dtype):
+    """Above 128 rows the 128 x 256 tiles of one CTA serve the calls that they fit in one wave and the pairs do not, and those of a short
+    K; these and their neighbours on either side of the rule (`pairs`: the form that a B200's 148 SMs give), with partial tiles."""
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     fits = lambda height, places: -(-m // height) * -(-n // 256) <= places  # a tile is `height` rows by 256 columns
     if sms == 148:
-        assert pairs == (not (fits(128, sms) and not fits(256, sms // 2)))
+        assert pairs == (not (fits(128, sms) and (k < 4096 or not fits(256, sms // 2))))
     _check(m, n, k, seed=m + n, dtype=dtype)

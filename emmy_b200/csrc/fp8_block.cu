@@ -237,8 +237,9 @@ static int quant_fp8_groups(const void* x, int64_t M, int64_t K, int in_dtype, u
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = (status && M <= 128) ? 1 : 0;  // decode-sized calls inside the linear: resident when the kernel before it ends
-    // From 4 M elements on: below, the kernel of one warp per group has the shorter chain (us a linear, N=17408: 65 rows of 5120 22.2
-    // against 23.4, 300 rows 53.8 : 54.7, 2048 rows 237 : 233, 8192 rows 920 : 896).
+    // From 4 M elements on the vector kernel; below, the kernel of one warp per group has the shorter chain.  Both forced, one warp per
+    // group : vectors, us a linear in graph replays, K=5120 N=17408: 65 rows 21.3 : 21.9, 300 rows (1.5 M elements) 54.1 : 54.0, 800 rows
+    // 102.9 : 101.8, 1024 rows 107.2 : 105.6, 2048 rows 207 : 203, 8192 rows 901 : 881.
     if (M * K >= 4000000 && in_dtype != EQ_F32 && aligned(x, 16) && aligned(q, 8)) {
         const int64_t vecs = M * K / 8;
         cfg.gridDim = dim3(static_cast<unsigned>(ceil_div(vecs, 512)));

@@ -27,14 +27,15 @@ constexpr int kTileA = kBM * kBK;
 // BN = 256: two weight scale blocks per CTA, eight promotion warps, four 48 KB stages, all of TMEM.  BN = 128 (calls of
 // at most 128 rows or one wave of such tiles): twice as many CTAs stream the weight, six 32 KB stages.
 //
-// The promotion bounds the kernel: a K block takes about 1050 cycles against 512 of MMA (128 x 256 x 128 products at 8192 a
-// clock), for 128 KB of accumulators read from TMEM.  That read is the limit, not the warps that wait for it: sixteen promotion warps of 64
-// columns took as long (2048 rows 249 us, 239 with packed f32 fma, against 234), and so did the same on CTA pairs, persistent
-// over tiles (242), which halves the shared-memory traffic.  So a block's factor is loaded one block ahead, off the
-// path behind the wait: K=5120 N=17408, 300 rows 62.8 -> 56.0 us, 2048 rows 237 -> 210, 8192 rows 878 -> 797.
-// Measured on top of that and dropped: reading the accumulator in pieces of 16 columns, one under way while the other is
-// added (it spills; 2048 rows 226), and CTA pairs (cta_group::2, half of the weight tile per CTA: 2048 rows 227 with those
-// pieces, and an odd number of row tiles leaves half a pair idle: K=5120 N=12288, 300 rows, one wave 37.0, two waves 57.9).
+// The promotion bounds the kernel, not the MMA: a K block takes about 1050 cycles against 512 of MMA (128 x 256 x 128 products at 8192
+// a clock).  Which part of it (the wait for the MMA, the read of 128 KB of accumulators from TMEM, the f32 adds) has not been timed apart.
+// More warps or less shared-memory traffic do not help: sixteen promotion warps of 64 columns (249 us, 239 with packed f32 fma, against
+// 234), and the same on CTA pairs, persistent over tiles (242; an odd number of row tiles leaves half a pair idle: N=12288, 300 rows, one
+// wave 37.0, two waves 57.9).  A block's factor is loaded one block ahead, off the path behind the wait: 300 rows 62.8 -> 56.0, 2048 rows
+// 237 -> 210, 8192 rows 878 -> 797.  On top of that and dropped: reading the accumulator in pieces of 16 columns, one under way while the
+// other is added (it spills: 226), and those pieces on CTA pairs (227).
+// Figures: us a linear of 2048 rows, K=5120 N=17408, where nothing else is said; each group of them is one session's, with the quantize of
+// that time in eager calls or replays.  As it is now, in graph replays: 300 rows 53.5, 2048 rows 203, 8192 rows 770 to 880 (power cap).
 template <int BN>
 struct BlkCfg {
     static constexpr int kTileB = BN * kBK;

@@ -5,8 +5,8 @@
 //                           against the numpy rule the reference spells (emmy/compiler/loader/quant.py:1655-1735).
 //   quant_fp8_rows_vec_kernel  the same for aligned rows: the row held in registers between the maximum and the encode,
 //                           16-byte loads; also clears the status word.
-//   fp8_decode_tc_kernel    M <= 16 (decode-shaped): tcgen05 with the operands' roles swapped -- 128-channel weight tiles
-//                           are the MMA's A operand, the rows its B operand with N = 16 -- so one TMA thread streams the
+//   fp8_decode_tc_kernel    M <= 64 (decode-shaped): tcgen05 with the operands' roles swapped -- 128-channel weight tiles
+//                           are the MMA's A operand, the rows its B operand, N = 16, 32 or 64 -- so one TMA thread streams the
 //                           weight, 108 KB CTAs of two consecutive launches share an SM, and the weights are requested
 //                           before griddepcontrol.wait (the quantize and the linear are both programmatic dependents).
 //   fp8_gemm_tc_kernel      64 < M <= 128: tcgen05.mma kind::f8f6f4, 128 x 128 output tile per CTA, K-major operands brought

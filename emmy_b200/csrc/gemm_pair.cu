@@ -13,9 +13,11 @@
 //
 // Why pairs: a lone CTA's tile is bound by shared memory (fills and operand reads of a 256 x 256 FP8 tile, 160 KB a K step, are 1250
 // cycles at 128 B/clock beside 1024 of MMA; of a 256 x 224 NVFP4 tile 164 KB, 1280 beside 950); here an SM moves 64 KB for
-// 128 x 256 x 128 bytes, 512 cycles beside 512.  Measured with the activation quantize (us, one-CTA tiles -> here; K=5120 N=17408):
-// NVFP4 512 rows 36.7 -> 29.3, 1024 rows 70 -> 50, 4096 rows 235 -> 162 (the GEMM alone 135: 5.4 PFLOP/s); FP8 200 rows 47 -> 35,
-// 1024 rows 103 -> 87, 2048 rows 198 -> 158, 8192 rows 761 -> 559 (2.6 PFLOP/s, under the power cap).
+// 128 x 256 x 128 bytes, 512 cycles beside 512.
+// Measured (us a linear, quantize included; K=5120 N=17408; graph replays over several weights).  One-CTA tiles -> here, both with the
+// two-pass quantizers of that time: NVFP4 512 rows 36.7 -> 29.3, 1024 rows 70 -> 50, 4096 rows 235 -> 162; FP8 200 rows 47 -> 35, 1024
+// rows 103 -> 87, 2048 rows 198 -> 158, 8192 rows 761 -> 559.  With the quantizers of quant.cuh: NVFP4 512 rows 27.5, 1024 rows 47,
+// 4096 rows 158 to 168 (the GEMM alone 135: 5.4 PFLOP/s); FP8 200 rows 27.3, 1024 rows 76, 2048 rows 141, 8192 rows 550 to 626 (power cap).
 #include "gemm_pair.cuh"
 #include "tc_common.cuh"
 

@@ -112,9 +112,11 @@ __global__ void quant_nvfp4_act_kernel(const InT* __restrict__ x, int64_t M, int
 }
 
 // The same rule for 16-bit activations at 16-byte aligned addresses, K a multiple of 64, tiled scales only: a CTA takes up to 128
-// rows x 64 elements, i.e. one scale atom; four neighbouring threads a row, whose four scale bytes are one word of the atom.  (No
-// division per thread to find its place, no scattered bytes: a linear of 1024 rows 54.3 -> 52.9 us, 4096 rows 175 -> 172, then 2048 x 2048 22.0 -> 20.5 by dividing single
-// elements.  Bound by its instructions: before the latter 336 a warp, 2.8 a cycle and SM, at 24% of the memory rate.  Fewer CTAs that walk over the pieces with the next one's loads under way are slower: 4096 rows 177.)
+// rows x 64 elements, i.e. one scale atom; four neighbouring threads a row, whose four scale bytes are one word of the atom: no
+// division per thread to find its place, no scattered bytes.  Bound by its instructions (336 a warp, 2.8 a cycle and SM, at 24 % of the
+// memory rate, before single elements were divided).
+// Measured, us a linear, K=5120, N=17408: 1024 rows 54.3 -> 52.9, 4096 rows 175 -> 172 (fewer CTAs that walk over the pieces with the
+// next one's loads under way: 177); then, by dividing single elements, 2048 rows of 2048 columns 22.0 -> 20.5.
 template <typename InT>
 __global__ void __launch_bounds__(512) quant_nvfp4_act_atoms_kernel(const uint4* __restrict__ x, int64_t M, int k64_blocks, const float* __restrict__ scale2,
                                                                     uint8_t* __restrict__ codes, uint8_t* __restrict__ sf_tiled, int* __restrict__ status) {

@@ -3,12 +3,14 @@
 // The rule divides every element by the scale in f32, rounds to nearest, and encodes the quotient (round to nearest even, saturating).
 // Encoding is monotonic, so a division per element is not needed: with lo <= 1 / s <= hi a hair apart (one division per
 // scale), fl(v lo) and fl(v hi) enclose fl(v / s) on either side of zero, and where both encode to the same code that is the code
-// of the quotient.  Where an element's two codes differ the quotient lies
-// within 2^-20, relatively, of a rounding boundary, and is divided.  With a scale that comes from a maximum of 16-bit values that is not rare:
-// quotients of short significands often fall on a boundary (e2m1, 1024 x 5120 normal bf16 values with a maximum of 5.0625: 0.4% of the elements, so 3% of
-// the groups of eight and 85% of the warps).  e2m1 divides only the elements concerned (NVFP4 linears, against dividing the group of eight: bf16 300 rows x
-// 5120 columns 17.9 -> 17.1 us, 2048 x 2048 22.0 -> 20.5, f16 2048 x 2048 20.0 -> 19.8; sixteen elements in one loop: f16 21.0).  e4m3 divides the group:
-// looking for the element gave nothing (FP8 linear of 128 rows 25.6 and 26.0 us).
+// of the quotient.  Where an element's two codes differ the quotient lies within 2^-20, relatively, of a rounding boundary, and is
+// divided.  With a scale that comes from a maximum of 16-bit values that is not rare: quotients of short significands often fall on a
+// boundary (e2m1, 1024 x 5120 normal bf16 values with a maximum of 5.0625: 0.4 % of the elements, so 3 % of the groups of eight and 85 %
+// of the warps).
+//
+// So e2m1 divides only the elements concerned.  Measured against dividing the group of eight, us an NVFP4 linear of K=5120, rows x columns: bf16
+// 300 x 5120 17.9 -> 17.1, 2048 x 2048 22.0 -> 20.5, f16 2048 x 2048 20.0 -> 19.8 (sixteen elements in one loop: f16 21.0).
+// e4m3 divides the group: looking for the element gave nothing (FP8 linear of 128 rows 25.6 and 26.0 us).
 #pragma once
 #include "common.cuh"
 

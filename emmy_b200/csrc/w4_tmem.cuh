@@ -5,12 +5,15 @@
 
 namespace eq {
 
-// Row counts at which the weights-in-TMEM kernels take over (us, K=4096 N=14336 | K=14336 N=4096 | K=N=4096 | the
-// [gate | up] + down MLP of hidden 4096, intermediate 14336; the other side first).
-// From 17 rows: below, w4_stream.cu stages all rows in shared memory and is the faster one (16 rows: 15.1 against 21.1, MLP
-// 42.8 against 44.5; 20 rows: 25.3 | 12.3 (K=N=4096) | MLP 73.2 against 17.1 | 9.6 | 49.4).  17 to 24 rows keep that
-// kernel's arithmetic, integers in the MMA and scales applied to f32 sums (PROMOTE); above, the weights are scaled before
-// the MMA, which at 28 rows costs 15.8 against 20.0 promoted.
+// Row counts at which the weights-in-TMEM kernels take over (us in graph replays, both kernels forced, streamed : in TMEM).
+// From 17 rows: 17 rows K=4096 N=14336 23.6 : 15.8, K=14336 N=4096 21.2 : 15.8, K=N=4096 11.5 : 9.0.  At 16 rows w4_stream.cu, which
+// then stages all rows in shared memory at once, is the faster one for K=4096 (14.4 : 15.4, K=N=4096 8.6 : 8.9), and for the
+// [gate | up] + down MLP of hidden 4096, intermediate 14336 (f16 42.2 : 45.5, bf16 43.4 : 47.8; 12 rows 40.4 : 45.1, 8 rows 33.2 : 44.5),
+// but not for every shape: from 12 rows on a K that has to be cut to fit is the slower one streamed (K=14336 N=4096, 8 rows 13.9 :
+// 15.4, 12 rows 17.2 : 15.5, 16 rows 18.3 : 15.8; MLP of hidden 5120, intermediate 17408, 8 rows 43.1 : 51.6, 12 rows 64.8 : 51.3, 16 rows
+// 70.5 : 50.6).  The rule does not look at that yet.
+// 17 to 24 rows keep the stream's arithmetic, integers in the MMA and scales applied to f32 sums (PROMOTE); above, the weights are
+// scaled before the MMA (28 rows, K=4096 N=14336: 15.8 against 20.0 promoted, measured when the kernel was new).
 constexpr int64_t kTmemPromoteRows = 24;
 
 // 17 to 24 rows of a small matrix stay with w4_stream.cu: with little of K per slice the tensor path's prologue, hand-overs

@@ -35,7 +35,11 @@ constexpr int kBoxRows = 32;
 constexpr int kWarps = kDW + 2, kThreads = kWarps * 32;
 constexpr size_t kSmem = 1024 + static_cast<size_t>(kStagesB) * kTileB + kRing + 256;
 constexpr uint32_t kTmemCols = 512;
-constexpr int64_t kExpandCycles = 480, kUnitCycles = 3500;  // of an SM: one item of 128 channels; a unit's prologue and epilogue
+// Of the choice of row tiles: cycles of an SM for one item of 128 channels, for a unit's prologue and epilogue.  Weights of a model, not
+// measured cycles: at 1965 MHz an item takes 0.32 us (620 cycles) with 32 or 48 rows, 0.40 with 80, 0.42 with 112, 0.51 with 128, 0.60
+// with 144, 0.81 with 256 (K=4096 against 12288, N=18944), a unit 2.5 to 5 us.  900 cycles an item in their place: 300 rows equal, K=4096
+// I=3584 at 600 rows 59.7 -> 69.9 us.
+constexpr int64_t kExpandCycles = 480, kUnitCycles = 3500;
 static_assert(kNB + 64 * kStagesA <= 512, "accumulator and A stages fill TMEM");
 static_assert(kSmem <= 227 * 1024, "one CTA per SM");
 

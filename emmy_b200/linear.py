@@ -46,11 +46,9 @@ def _(x, weight, weight_scale):
     return x.new_empty((x.shape[0], weight.shape[0]))
 
 
-def _fp8_static(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor, input_scale: torch.Tensor) -> torch.Tensor:
+@torch.library.custom_op("emmyq::fp8_linear_static", mutates_args=(), device_types="cuda")
+def _fp8_static_op(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor, input_scale: torch.Tensor) -> torch.Tensor:
     return ops.fp8_linear(x.contiguous(), weight, weight_scale, input_scale=input_scale)
-
-
-_fp8_static_op = torch.library.custom_op("emmyq::fp8_linear_static", mutates_args=(), device_types="cuda")(_fp8_static)
 
 
 @_fp8_static_op.register_fake
@@ -126,6 +124,8 @@ def _(x, router_logits, gate_up, down, experts, hidden, inter, group, scale_bf16
 # by what would make the dispatcher do anything else: tracing or compilation, a tensor or function mode, vmap and the other function
 # transforms (all visible in the thread's included keys), a tensor subclass or wrapper (visible in the tensor's own keys), gradients
 # and forward-mode levels, a profiler that wants to see the operator.  Any of them takes the operator as before.
+# W4A16Linear, FP8Linear with per-token scales, FP8BlockLinear, NVFP4Linear and QuantMoE ask; FP8Linear with a static input_scale and
+# the fused operators always go through the dispatcher.
 _K = torch._C.DispatchKey
 _PLAIN_THREAD = {(torch._C.DispatchKeySet(_K.BackendSelect) | torch._C.DispatchKeySet(_K.ADInplaceOrView)).raw_repr(),
                  torch._C.DispatchKeySet(_K.BackendSelect).raw_repr()}
